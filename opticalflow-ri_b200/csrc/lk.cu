@@ -62,22 +62,10 @@ __device__ __forceinline__ void lk_weights(int id, int ws, int lo, int hi, float
   }
 }
 
-__device__ __forceinline__ float lk_bilinear(const float* __restrict__ J, int H, int W, int pitch, float x, float y) {
-  float xs = __fsub_rn(x, 0.5f), ys = __fsub_rn(y, 0.5f);
-  float fx0 = floorf(xs), fy0 = floorf(ys);
-  float a = __fsub_rn(xs, fx0), b = __fsub_rn(ys, fy0);
-  int i0 = (int)fx0, j0 = (int)fy0;
-  int xa = clampi(i0, 0, W - 1), xb = clampi(i0 + 1, 0, W - 1);
-  int ya = clampi(j0, 0, H - 1), yb = clampi(j0 + 1, 0, H - 1);
-  float t00 = __ldg(J + (size_t)ya * pitch + xa), t10 = __ldg(J + (size_t)ya * pitch + xb);
-  float t01 = __ldg(J + (size_t)yb * pitch + xa), t11 = __ldg(J + (size_t)yb * pitch + xb);
-  float oa = __fsub_rn(1.f, a), ob = __fsub_rn(1.f, b);
-  float r = __fmul_rn(__fmul_rn(oa, ob), t00);
-  r = __fmaf_rn(__fmul_rn(a, ob), t10, r);
-  r = __fmaf_rn(__fmul_rn(oa, b), t01, r);
-  r = __fmaf_rn(__fmul_rn(a, b), t11, r);
-  return r;
-}
+// A texel index from a floored position.  The error of a pixel whose flow is infinite (or
+// merely huge) is evaluated there too; its index is held within 2^22 of the origin, beyond
+// every image (H, W < 2^21), so that the index arithmetic that follows cannot overflow.
+__device__ __forceinline__ int lk_texel(float f) { return (int)fminf(fmaxf(f, -4194304.f), 4194304.f); }
 
 // The same bilinear sample from the staged region when its 2 x 2 footprint lies inside it
 // (rx, ry: footprint origin relative to the region), else from global memory.
@@ -86,7 +74,7 @@ __device__ __forceinline__ float lk_bilinear_s(const float2* __restrict__ sJ, co
   float xs = __fsub_rn(x, 0.5f), ys = __fsub_rn(y, 0.5f);
   float fx0 = floorf(xs), fy0 = floorf(ys);
   float a = __fsub_rn(xs, fx0), b = __fsub_rn(ys, fy0);
-  int i0 = (int)fx0, j0 = (int)fy0;
+  const int i0 = lk_texel(fx0), j0 = lk_texel(fy0);
   const int rx = i0 - ox, ry = j0 - oy;
   float t00, t10, t01, t11;
   if ((unsigned)rx <= (unsigned)(LK_JR - 2) && (unsigned)ry <= (unsigned)(LK_JR - 2)) {

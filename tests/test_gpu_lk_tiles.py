@@ -1,0 +1,40 @@
+"""Dense Lucas-Kanade from initial flows that are infinite, not a number or huge at some
+pixels, against the CPU oracle bit for bit."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def frames(h, w, seed):
+    from ofb200 import synthetic as S
+    a, b, _, _ = S.piv_pair(h, w, "lamb_oseen", seed=seed, core_radius=10, density=0.08)
+    return a.astype(np.float32), b.astype(np.float32)
+
+
+@pytest.mark.parametrize("hw", [5, 9, 13])
+def test_lk_infinite_flow(cuda_ok, hw):
+    """Such pixels end untracked, with a status and an error, and leave the others alone (the
+    pixels are independent, so the oracle runs with those at rest)."""
+    import torch
+    from ofb200 import ops
+    h, w = 19, 23
+    a, b = frames(h, w, hw)
+    rng = np.random.default_rng(hw)
+    U0, V0 = (rng.uniform(-1, 1, (h, w)).astype(np.float32) for _ in range(2))
+    odd = np.zeros((h, w), bool)
+    U1, V1 = U0.copy(), V0.copy()
+    for k, x in enumerate((np.inf, -np.inf, 1e30, -1e30, 2.0 ** 31, -2.0 ** 31)):
+        odd[3 * k, 2 * k] = odd[3 * k, 20 - k] = odd[3 * k + 1, 9] = True
+        U1[3 * k, 2 * k] = V1[3 * k, 20 - k] = U1[3 * k + 1, 9] = V1[3 * k + 1, 9] = x
+    U, V = (torch.from_numpy(t).cuda() for t in (U1, V1))
+    st = torch.empty((h, w), dtype=torch.uint8, device="cuda")
+    er = torch.empty((h, w), dtype=torch.float32, device="cuda")
+    ops.lk_dense(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), U, V, hw, 5, (0, 0, 0, 0), st, er)
+    got = [t.cpu().numpy() for t in (U, V, st, er)]
+    want = O.lk_dense(a, b, U0, V0, hw, 5, want_status=True)
+    for x, y in zip(got, want):
+        assert np.array_equal(x[~odd], y[~odd])
+    assert not got[2][odd].any()
