@@ -10,14 +10,21 @@
 // the same pairing: A, b and the error are reduced in exactly the reference's order.
 // J is sampled with exact float32 bilinear weights (pixel-centre convention, clamp to
 // edge) from a 64x64 region staged per CTA around the tile's mean displaced window, stored
-// as (J[y][x], J[y][x+1]) pairs so a bilinear footprint is two 64-bit loads; the gradients
-// are stored as (dx, dy) pairs.  A warp whose every footprint of a Newton step lies in the
-// region runs the samples without per-sample region tests; others fall back per sample to
-// clamped global reads.  Issue bound: ~7e4 FP32 flops per pixel at a 27x27 window and
-// 5 Newton steps, about 7 shared-memory reads per sample.
+// as (J[y][x], J[y+4][x]) pairs: the two work items of a lane lie 4 rows apart, so the four
+// 64-bit loads of a footprint feed both of them and the blend, the difference and the sums
+// run as packed f32x2 operations (each half rounds as the scalar operation does).
+//
+// What bounds it: shared-memory reads and issue slots.  A sample needs 16 bytes of J on every
+// Newton step, and the 27 x 27 window's intensities and gradients another 12; those do not
+// change between the steps of a pixel, so each lane keeps its samples' 84 values in
+// registers (the reason for 128-thread CTAs at 168 registers, 3 per SM).  The footprints of
+// a lane's samples lie at fixed steps of 8 texels unless a position rounds across a texel,
+// which the step's fractions show; so all addresses are one base plus constants.  A
+// warp with such a position, or one outside the region, takes the per-sample path.
+// One 512x512 level from a smooth field (4.5 steps per pixel): 1.14 -> 0.92 ms (shared-memory
+// pipe 72 %, FMA pipe 60 %, issue 67 % busy); a 301x413 level with a 19 x 19 window, status
+// and error: 1.16 -> 0.52 ms.
 #include <float.h>
-
-#include <type_traits>
 
 #include "common.cuh"
 
@@ -38,6 +45,11 @@ constexpr int LK_JR = 64, LK_JP = 72;  // LK_JP counts float2 texel pairs
 static_assert(LK_JP % 16 == 8, "J pair stride");
 // dynamic shared memory of the kernel: sJ2 pairs, sD2 pairs, sI
 constexpr size_t LK_SMEM = (size_t)LK_JR * LK_JP * 8 + (size_t)LK_G * LK_GP * 8 + (size_t)LK_I * LK_IP * 4;
+
+// Threads and CTAs per SM of the kernel for NT window tiles per axis: 3 values per sample are
+// held in registers, 2 NT^2 samples per lane (the default window: 28).
+constexpr int lk_threads(int nt) { return nt == 4 ? 128 : 256; }
+constexpr int lk_ctas(int nt, bool def) { return nt == 4 && def ? 3 : 2; }
 
 struct LkParams {
   int ws, hw, aL, aR, aT, aB, niter;
@@ -67,7 +79,7 @@ __device__ __forceinline__ void lk_weights(int id, int ws, int lo, int hi, float
 // every image (H, W < 2^21), so that the index arithmetic that follows cannot overflow.
 __device__ __forceinline__ int lk_texel(float f) { return (int)fminf(fmaxf(f, -4194304.f), 4194304.f); }
 
-// The same bilinear sample from the staged region when its 2 x 2 footprint lies inside it
+// A bilinear sample (clamp to edge) from the staged region when its 2 x 2 footprint lies inside it
 // (rx, ry: footprint origin relative to the region), else from global memory.
 __device__ __forceinline__ float lk_bilinear_s(const float2* __restrict__ sJ, const float* __restrict__ J, int H, int W,
                                                int pitch, float x, float y, int ox, int oy) {
@@ -78,11 +90,11 @@ __device__ __forceinline__ float lk_bilinear_s(const float2* __restrict__ sJ, co
   const int rx = i0 - ox, ry = j0 - oy;
   float t00, t10, t01, t11;
   if ((unsigned)rx <= (unsigned)(LK_JR - 2) && (unsigned)ry <= (unsigned)(LK_JR - 2)) {
-    const float2 top = sJ[ry * LK_JP + rx], bot = sJ[(ry + 1) * LK_JP + rx];
-    t00 = top.x;
-    t10 = top.y;
-    t01 = bot.x;
-    t11 = bot.y;
+    const float2* q = sJ + ry * LK_JP + rx;
+    t00 = q[0].x;
+    t10 = q[1].x;
+    t01 = q[LK_JP].x;
+    t11 = q[LK_JP + 1].x;
   } else {
     int xa = clampi(i0, 0, W - 1), xb = clampi(i0 + 1, 0, W - 1);
     int ya = clampi(j0, 0, H - 1), yb = clampi(j0 + 1, 0, H - 1);
@@ -119,6 +131,21 @@ __device__ __forceinline__ float lk_tree(float lo, float hi) {
   return __shfl_sync(0xffffffffu, t, 0);
 }
 
+// Two sums by the same tree in half the shuffles: after the first exchange lanes 0-15 carry
+// the first and lanes 16-31 the second (float32 addition commutes, so the pairing is all
+// that matters).  Both results reach every lane.
+__device__ __forceinline__ void lk_tree2(float2 a, float2 b, float& sa, float& sb) {
+  const float qa = __fadd_rn(a.x, a.y), qb = __fadd_rn(b.x, b.y);
+  const bool hi = (threadIdx.x & 16) != 0;
+  float q = __fadd_rn(hi ? qb : qa, __shfl_xor_sync(0xffffffffu, hi ? qa : qb, 16));
+  q = __fadd_rn(q, __shfl_down_sync(0xffffffffu, q, 8));
+  q = __fadd_rn(q, __shfl_down_sync(0xffffffffu, q, 4));
+  q = __fadd_rn(q, __shfl_down_sync(0xffffffffu, q, 1));
+  q = __fadd_rn(q, __shfl_down_sync(0xffffffffu, q, 2));
+  sa = __shfl_sync(0xffffffffu, q, 0);
+  sb = __shfl_sync(0xffffffffu, q, 16);
+}
+
 // Whether sample (v, ty, tx) of lane (xid, yid) has a non-zero tile weight.
 template <bool DEF>
 __device__ __forceinline__ bool lk_on(unsigned act, int v, int ty, int tx, int xid, int yid) {
@@ -126,48 +153,32 @@ __device__ __forceinline__ bool lk_on(unsigned act, int v, int ty, int tx, int x
   return (act >> (16 * v + 4 * ty + tx)) & 1u;
 }
 
-// DEF: the default window (27 x 27, no asymmetric mask), whose tile-weight pattern is known
-// at compile time (and whose registers fit 3 CTAs per SM, 80 per thread): lane (xid, yid)'s 4th column tile is used when xid < 3, its 4th row tile
-// of the first half when yid < 3, the 4th row tile of the second half never.
-template <bool DEF>
-__global__ void __launch_bounds__(256, DEF ? 3 : 2) lk_dense_kernel(const float* __restrict__ I, const float* __restrict__ J,
-                                                       float* __restrict__ U, float* __restrict__ V, int H, int W,
-                                                       int pitch, LkParams p, uint8_t* __restrict__ status,
-                                                       float* __restrict__ err) {
+// NT: the window's tiles of 8 per axis (ceil(ws / 8)); tiles past it have no weight.  DEF: the
+// default window (27 x 27, no asymmetric mask), whose tile-weight pattern is known at compile
+// time: lane (xid, yid)'s 4th column tile is used when xid < 3, its 4th row tile of the first
+// half when yid < 3, the 4th row tile of the second half never.
+template <int NT, bool DEF>
+__global__ void __launch_bounds__(lk_threads(NT), lk_ctas(NT, DEF)) lk_dense_kernel(
+    const float* __restrict__ I, const float* __restrict__ J, float* __restrict__ U, float* __restrict__ V, int H, int W,
+    int pitch, LkParams p, uint8_t* __restrict__ status, float* __restrict__ err) {
+  constexpr int LK_THREADS = lk_threads(NT);
   extern __shared__ float4 lk_dyn[];
-  float2* const sJ = reinterpret_cast<float2*>(lk_dyn);  // (J[y][x], J[y][x + 1]) pairs
+  float2* const sJ = reinterpret_cast<float2*>(lk_dyn);  // (J[y][x], J[y + 4][x]) pairs
   float2* const sD = sJ + LK_JR * LK_JP;                 // (dx, dy) pairs
   float* const sI = reinterpret_cast<float*>(sD + LK_G * LK_GP);
   const int i0 = blockIdx.y * LK_PT, j0 = blockIdx.x * LK_PT;
   const int oy = i0 - p.hw - 1, ox = j0 - p.hw - 1;  // image position of sI[0][0]
-  for (int t = threadIdx.x; t < LK_I * LK_I; t += blockDim.x) {
+  for (int t = threadIdx.x; t < LK_I * LK_I; t += LK_THREADS) {
     int ly = t / LK_I, lx = t - ly * LK_I;
     sI[ly * LK_IP + lx] = I[(size_t)clampi(oy + ly, 0, H - 1) * pitch + clampi(ox + lx, 0, W - 1)];
   }
-  __syncthreads();
-  for (int t = threadIdx.x; t < LK_G * LK_G; t += blockDim.x) {
-    int gy = t / LK_G, gx = t - gy * LK_G;
-    const float* c = sI + (gy + 1) * LK_IP + gx + 1;
-#define P(dy, dx) c[(dy) * LK_IP + (dx)]
-    float ddx, ddy;
-    ddx = __fmaf_rn(__fsub_rn(__fsub_rn(__fadd_rn(P(-1, 1), P(1, 1)), P(-1, -1)), P(1, -1)), 3.0f,
-                       __fmul_rn(__fsub_rn(P(0, 1), P(0, -1)), 10.0f));
-    ddy = __fmaf_rn(__fsub_rn(__fsub_rn(__fadd_rn(P(1, -1), P(1, 1)), P(-1, -1)), P(-1, 1)), 3.0f,
-                       __fmul_rn(__fsub_rn(P(1, 0), P(-1, 0)), 10.0f));
-#undef P
-    sD[gy * LK_GP + gx] = make_float2(ddx, ddy);
-  }
   // J region: centred on the tile centre displaced by the mean initial flow of the tile
-  __shared__ float red_u[8], red_v[8];
-  {
-    float su = 0.f, sv = 0.f;
-    if (threadIdx.x < LK_PT * LK_PT) {
-      const int yy = min(i0 + (int)(threadIdx.x >> 3), H - 1), xx = min(j0 + (int)(threadIdx.x & 7), W - 1);
-      su = U[(size_t)yy * pitch + xx];
-      sv = V[(size_t)yy * pitch + xx];
-      su = isfinite(su) ? fminf(fmaxf(su, -1e6f), 1e6f) : 0.f;
-      sv = isfinite(sv) ? fminf(fmaxf(sv, -1e6f), 1e6f) : 0.f;
-    }
+  __shared__ float red_u[2], red_v[2];
+  if (threadIdx.x < LK_PT * LK_PT) {
+    const int yy = min(i0 + (int)(threadIdx.x >> 3), H - 1), xx = min(j0 + (int)(threadIdx.x & 7), W - 1);
+    float su = U[(size_t)yy * pitch + xx], sv = V[(size_t)yy * pitch + xx];
+    su = isfinite(su) ? fminf(fmaxf(su, -1e6f), 1e6f) : 0.f;
+    sv = isfinite(sv) ? fminf(fmaxf(sv, -1e6f), 1e6f) : 0.f;
     for (int o = 16; o > 0; o >>= 1) {
       su += __shfl_down_sync(0xffffffffu, su, o);
       sv += __shfl_down_sync(0xffffffffu, sv, o);
@@ -180,16 +191,31 @@ __global__ void __launch_bounds__(256, DEF ? 3 : 2) lk_dense_kernel(const float*
   __syncthreads();
   const float mu = (red_u[0] + red_u[1]) * (1.f / 64.f), mv = (red_v[0] + red_v[1]) * (1.f / 64.f);
   const int jox = j0 + LK_PT / 2 + (int)floorf(mu) - LK_JR / 2, joy = i0 + LK_PT / 2 + (int)floorf(mv) - LK_JR / 2;
-  for (int t = threadIdx.x; t < LK_JR * LK_JR; t += blockDim.x) {
+#pragma unroll 4
+  for (int t = threadIdx.x; t < LK_JR * LK_JR; t += LK_THREADS) {
     const int ly = t / LK_JR, lx = t - ly * LK_JR;
-    const float* row = J + (size_t)clampi(joy + ly, 0, H - 1) * pitch;
-    sJ[ly * LK_JP + lx] = make_float2(__ldg(row + clampi(jox + lx, 0, W - 1)), __ldg(row + clampi(jox + lx + 1, 0, W - 1)));
+    const float* col = J + clampi(jox + lx, 0, W - 1);
+    sJ[ly * LK_JP + lx] = make_float2(__ldg(col + (size_t)clampi(joy + ly, 0, H - 1) * pitch),
+                                      __ldg(col + (size_t)clampi(joy + ly + 4, 0, H - 1) * pitch));
+  }
+  for (int t = threadIdx.x; t < LK_G * LK_G; t += LK_THREADS) {
+    int gy = t / LK_G, gx = t - gy * LK_G;
+    const float* c = sI + (gy + 1) * LK_IP + gx + 1;
+#define P(dy, dx) c[(dy) * LK_IP + (dx)]
+    float ddx, ddy;
+    ddx = __fmaf_rn(__fsub_rn(__fsub_rn(__fadd_rn(P(-1, 1), P(1, 1)), P(-1, -1)), P(1, -1)), 3.0f,
+                       __fmul_rn(__fsub_rn(P(0, 1), P(0, -1)), 10.0f));
+    ddy = __fmaf_rn(__fsub_rn(__fsub_rn(__fadd_rn(P(1, -1), P(1, 1)), P(-1, -1)), P(-1, 1)), 3.0f,
+                       __fmul_rn(__fsub_rn(P(1, 0), P(-1, 0)), 10.0f));
+#undef P
+    sD[gy * LK_GP + gx] = make_float2(ddx, ddy);
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int xid = lane & 7, yid = lane >> 3;
   unsigned act = 0;  // bit 16 v + 4 ty + tx: the sample's tile weight is not 0
-  {
+  unsigned any = 0;  // the same bit set when it is for some lane of the warp
+  if (!DEF) {
     float wx[4], wy0[4], wy1[4];
     int bx[2], by0[2], by1[2];
     lk_weights(xid, p.ws, p.aL, p.aR, wx, bx);
@@ -202,187 +228,221 @@ __global__ void __launch_bounds__(256, DEF ? 3 : 2) lk_dense_kernel(const float*
 #pragma unroll
         for (int tx = 0; tx < 4; tx++)
           act |= (unsigned)(__fmul_rn(wx[tx], (v ? wy1 : wy0)[ty]) != 0.f) << (16 * v + 4 * ty + tx);
+    any = __reduce_or_sync(0xffffffffu, act);
   }
+  // samples no lane has (row tile ty of half v, column tile tx): warp-uniform
+#define LK_SKIP(v, ty, tx) (DEF ? ((v) == 1 && (ty) == 3) : !((any >> (16 * (v) + 4 * (ty) + (tx))) & 1u))
+#define LK_SKIP2(ty, tx) (LK_SKIP(0, ty, tx) && LK_SKIP(1, ty, tx))
   const float hw = (float)p.hw;
-  const int i = i0 + warp;
-  if (i >= H) return;
-  for (int c = 0; c < LK_PT; c++) {
-    const int j = j0 + c;
-    if (j >= W) break;
-    const int gyb = warp, gxb = c;  // gradient-tile origin of this pixel's window
-    float a11[2] = {0.f, 0.f}, a12[2] = {0.f, 0.f}, a22[2] = {0.f, 0.f};
+  const float2 m1 = make_float2(-1.f, -1.f);  // a - b as one fused multiply-add
+#pragma unroll 1
+  for (int i = i0 + warp; i < min(i0 + LK_PT, H); i += LK_THREADS / 32) {
+    const int gyb = i - i0;
+    // the row's initial flow, one pixel per lane
+    const int jl = min(j0 + (lane & (LK_PT - 1)), W - 1);
+    const float row_u = U[(size_t)i * pitch + jl], row_v = V[(size_t)i * pitch + jl];
+#pragma unroll 1
+    for (int c = 0; c < LK_PT; c++) {
+      const int j = j0 + c;
+      if (j >= W) break;
+      const int gxb = c;  // (gyb, gxb): gradient-tile origin of this pixel's window
+      const float* const pI = sI + (gyb + yid + 1) * LK_IP + gxb + xid + 1;
+      const float2* const pD = sD + (gyb + yid) * LK_GP + gxb + xid;
+      // The window's intensities (negated) and gradients, as pairs over the two row halves:
+      // they stay in registers for every Newton step.  Samples without weight hold 0.
+      float2 nI[NT][NT], Dx[NT][NT], Dy[NT][NT];
+      float a11[2] = {0.f, 0.f}, a12[2] = {0.f, 0.f}, a22[2] = {0.f, 0.f};
 #pragma unroll
-    for (int v = 0; v < 2; v++) {
-      const int yy = yid + 4 * v;
+      for (int ty = 0; ty < NT; ty++)
 #pragma unroll
-      for (int ty = 0; ty < 4; ty++)
+        for (int tx = 0; tx < NT; tx++) {
+          float iv[2], dx[2], dy[2];
 #pragma unroll
-        for (int tx = 0; tx < 4; tx++) {
-          if (!lk_on<DEF>(act, v, ty, tx, xid, yid)) continue;  // tile weight 0
-          int g = (gyb + ty * 8 + yy) * LK_GP + gxb + tx * 8 + xid;
-          // w is 1 here (the tile weights are products of 0 / 1 values and w == 0 is
-          // skipped), so the reference's multiplications by w are exact identities
-          const float2 d = sD[g];
-          const float dx = d.x, dy = d.y;
-          a11[v] = __fmaf_rn(dx, dx, a11[v]);
-          a12[v] = __fmaf_rn(dx, dy, a12[v]);
-          a22[v] = __fmaf_rn(dy, dy, a22[v]);
+          for (int v = 0; v < 2; v++) {
+            iv[v] = dx[v] = dy[v] = 0.f;
+            if (LK_SKIP(v, ty, tx)) continue;
+            iv[v] = -pI[(ty * 8 + 4 * v) * LK_IP + tx * 8];
+            const float2 d = pD[(ty * 8 + 4 * v) * LK_GP + tx * 8];
+            const bool on = lk_on<DEF>(act, v, ty, tx, xid, yid);
+            dx[v] = on ? d.x : 0.f;
+            dy[v] = on ? d.y : 0.f;
+            // w is 1 here (the tile weights are products of 0 / 1 values), so the reference's
+            // multiplications by w are exact identities; + 0 * 0 changes no sum
+            a11[v] = __fmaf_rn(dx[v], dx[v], a11[v]);
+            a12[v] = __fmaf_rn(dx[v], dy[v], a12[v]);
+            a22[v] = __fmaf_rn(dy[v], dy[v], a22[v]);
+          }
+          nI[ty][tx] = make_float2(iv[0], iv[1]);
+          Dx[ty][tx] = make_float2(dx[0], dx[1]);
+          Dy[ty][tx] = make_float2(dy[0], dy[1]);
         }
-    }
-    float A11 = lk_tree(a11[0], a11[1]), A12 = lk_tree(a12[0], a12[1]), A22 = lk_tree(a22[0], a22[1]);
-    const size_t gid = (size_t)i * pitch + j;
-    float D = __fmaf_rn(A11, A22, -__fmul_rn(A12, A12));
-    if (D < 1.192092896e-07f) {
-      if (lane == 0) {
-        if (status) status[gid] = 0;
-        if (err) err[gid] = 0.f;
+      float A11, A12, A22;
+      lk_tree2(make_float2(a11[0], a11[1]), make_float2(a12[0], a12[1]), A11, A12);
+      A22 = lk_tree(a22[0], a22[1]);
+      const size_t gid = (size_t)i * pitch + j;
+      float D = __fmaf_rn(A11, A22, -__fmul_rn(A12, A12));
+      if (D < 1.192092896e-07f) {
+        if (lane == 0) {
+          if (status) status[gid] = 0;
+          if (err) err[gid] = 0.f;
+        }
+        continue;
       }
-      continue;
-    }
-    A11 = __fdiv_rn(A11, D);
-    A12 = __fdiv_rn(A12, D);
-    A22 = __fdiv_rn(A22, D);
-    float ptx = __fsub_rn(__fadd_rn((float)j, U[gid]), hw), pty = __fsub_rn(__fadd_rn((float)i, V[gid]), hw);
-    float lx[4], ly[2][4];
-    lx[0] = __fadd_rn(ptx, __fadd_rn((float)xid, 0.5f));
-    ly[0][0] = __fadd_rn(pty, __fadd_rn((float)yid, 0.5f));
-    ly[1][0] = __fadd_rn(pty, __fadd_rn((float)(yid + 4), 0.5f));
+      A11 = __fdiv_rn(A11, D);
+      A12 = __fdiv_rn(A12, D);
+      A22 = __fdiv_rn(A22, D);
+      float ptx = __fsub_rn(__fadd_rn((float)j, __shfl_sync(0xffffffffu, row_u, c)), hw);
+      float pty = __fsub_rn(__fadd_rn((float)i, __shfl_sync(0xffffffffu, row_v, c)), hw);
+      // sample positions: x per column tile, y per row tile as pairs over the two row halves
+      float lx[NT];
+      float2 ly[NT];
+      lx[0] = __fadd_rn(ptx, __fadd_rn((float)xid, 0.5f));
+      ly[0].x = __fadd_rn(pty, __fadd_rn((float)yid, 0.5f));
+      ly[0].y = __fadd_rn(pty, __fadd_rn((float)(yid + 4), 0.5f));
 #pragma unroll
-    for (int t = 1; t < 4; t++) {
-      lx[t] = __fadd_rn(lx[t - 1], 8.0f);
-      ly[0][t] = __fadd_rn(ly[0][t - 1], 8.0f);
-      ly[1][t] = __fadd_rn(ly[1][t - 1], 8.0f);
-    }
-    uint8_t st = 1;
-    for (int k = 0; k < p.niter; k++) {
-      if (ptx < -hw || ptx >= (float)W || pty < -hw || pty >= (float)H) {
-        st = 0;
-        break;
+      for (int t = 1; t < NT; t++) {
+        lx[t] = __fadd_rn(lx[t - 1], 8.0f);
+        ly[t].x = __fadd_rn(ly[t - 1].x, 8.0f);
+        ly[t].y = __fadd_rn(ly[t - 1].y, 8.0f);
       }
-      // The bilinear sample positions of a Newton step: x parts per column tile, y parts per
-      // row tile (the same float32 operations as lk_bilinear_s, computed once per step)
-      float xa[4], xoa[4], yb[2][4], yob[2][4];
-      int xr[4], yr[2][4];
-      unsigned inx = 0, iny = 0;
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
+      uint8_t st = 1;
+#pragma unroll 1
+      for (int k = 0; k < p.niter; k++) {
+        if (ptx < -hw || ptx >= (float)W || pty < -hw || pty >= (float)H) {
+          st = 0;
+          break;
+        }
         // positions here are within a window of the image (the step's range test), so
         // |xs|, |ys| < 2^22 (the ABI caps H, W) and lk_floor is floorf
-        int ix;
-        const float xs = __fsub_rn(lx[t], 0.5f), fx0 = lk_floor(xs, ix);
-        xa[t] = __fsub_rn(xs, fx0);
-        xoa[t] = __fsub_rn(1.f, xa[t]);
-        xr[t] = ix - jox;
-        inx |= ((unsigned)xr[t] <= (unsigned)(LK_JR - 2)) << t;
+        int rx, ry;
+        const float fx = lk_floor(__fsub_rn(lx[0], 0.5f), rx), fy = lk_floor(__fsub_rn(ly[0].x, 0.5f), ry);
+        // The fractions of every position against the first one's floor plus the tile step: a
+        // fraction in [0, 1) is the position's own (the float32 difference is exact), so a
+        // lane whose fractions all are has its footprints at fixed steps from the first.
+        float2 xa[NT], xo[NT], yb[NT], yo[NT];
+        unsigned worst = 0;
 #pragma unroll
-        for (int v = 0; v < 2; v++) {
-          int iy;
-          const float ys = __fsub_rn(ly[v][t], 0.5f), fy0 = lk_floor(ys, iy);
-          yb[v][t] = __fsub_rn(ys, fy0);
-          yob[v][t] = __fsub_rn(1.f, yb[v][t]);
-          yr[v][t] = iy - joy;
-          iny |= ((unsigned)yr[v][t] <= (unsigned)(LK_JR - 2)) << (4 * v + t);
+        for (int t = 0; t < NT; t++) {
+          const float a = __fsub_rn(__fsub_rn(lx[t], 0.5f), __fadd_rn(fx, 8.f * t)), oa = __fsub_rn(1.f, a);
+          xa[t] = make_float2(a, a);
+          xo[t] = make_float2(oa, oa);
+          const float2 f = __fadd2_rn(make_float2(fy, fy), make_float2(8.f * t, 8.f * t + 4.f));
+          yb[t] = __ffma2_rn(f, m1, __fadd2_rn(ly[t], make_float2(-0.5f, -0.5f)));
+          yo[t] = __ffma2_rn(yb[t], m1, make_float2(1.f, 1.f));
+          worst = max(max(worst, __float_as_uint(a)), max(__float_as_uint(yb[t].x), __float_as_uint(yb[t].y)));
         }
-      }
-      float b1[2] = {0.f, 0.f}, b2[2] = {0.f, 0.f};
-      // The samples of the step; a warp whose every footprint lies inside the staged J
-      // region (the common case) runs the variant without the per-sample region test.
-      auto samples = [&](auto all_in) {
+        rx -= jox;
+        ry -= joy;
+        const bool regular = worst < 0x3f800000u && (unsigned)rx <= (unsigned)(LK_JR - 2 - 8 * (NT - 1)) &&
+                             (unsigned)ry <= (unsigned)(LK_JR - 2 - 8 * (NT - 1) - 4);
+        float2 b1 = make_float2(0.f, 0.f), b2 = b1;
+        if (__all_sync(0xffffffffu, regular)) {
+          const float2* const q = sJ + ry * LK_JP + rx;
 #pragma unroll
-        for (int v = 0; v < 2; v++) {
-          const int yy = yid + 4 * v;
+          for (int ty = 0; ty < NT; ty++)
 #pragma unroll
-          for (int ty = 0; ty < 4; ty++)
-#pragma unroll
-            for (int tx = 0; tx < 4; tx++) {
-              if (!lk_on<DEF>(act, v, ty, tx, xid, yid)) continue;  // tile weight 0
-              int g = (gyb + ty * 8 + yy) * LK_GP + gxb + tx * 8 + xid;
-              float Iv = sI[(gyb + ty * 8 + yy + 1) * LK_IP + gxb + tx * 8 + xid + 1];
-              float t00, t10, t01, t11;
-              if (decltype(all_in)::value || (((inx >> tx) & (iny >> (4 * v + ty))) & 1u)) {
-                const float2* q = sJ + yr[v][ty] * LK_JP + xr[tx];
-                const float2 top = q[0], bot = q[LK_JP];
-                t00 = top.x;
-                t10 = top.y;
-                t01 = bot.x;
-                t11 = bot.y;
-              } else {  // outside the staged region: clamped global reads
-                const int i0 = xr[tx] + jox, j0 = yr[v][ty] + joy;
-                const int xa0 = clampi(i0, 0, W - 1), xb0 = clampi(i0 + 1, 0, W - 1);
-                const int ya0 = clampi(j0, 0, H - 1), yb0 = clampi(j0 + 1, 0, H - 1);
-                t00 = __ldg(J + (size_t)ya0 * pitch + xa0);
-                t10 = __ldg(J + (size_t)ya0 * pitch + xb0);
-                t01 = __ldg(J + (size_t)yb0 * pitch + xa0);
-                t11 = __ldg(J + (size_t)yb0 * pitch + xb0);
+            for (int tx = 0; tx < NT; tx++) {
+              if (LK_SKIP2(ty, tx)) continue;
+              const float2* const s = q + (8 * ty) * LK_JP + 8 * tx;
+              if (DEF && ty == NT - 1) {  // the first half alone: 32-bit reads, scalar arithmetic
+                float Jv = __fmul_rn(__fmul_rn(xo[tx].x, yo[ty].x), s[0].x);
+                Jv = __fmaf_rn(__fmul_rn(xa[tx].x, yo[ty].x), s[1].x, Jv);
+                Jv = __fmaf_rn(__fmul_rn(xo[tx].x, yb[ty].x), s[LK_JP].x, Jv);
+                Jv = __fmaf_rn(__fmul_rn(xa[tx].x, yb[ty].x), s[LK_JP + 1].x, Jv);
+                float d = __fadd_rn(Jv, nI[ty][tx].x);
+                if (!lk_on<DEF>(act, 0, ty, tx, xid, yid)) d = 0.f;
+                b1.x = __fmaf_rn(d, Dx[ty][tx].x, b1.x);
+                b2.x = __fmaf_rn(d, Dy[ty][tx].x, b2.x);
+                continue;
               }
-              float Jv = __fmul_rn(__fmul_rn(xoa[tx], yob[v][ty]), t00);
-              Jv = __fmaf_rn(__fmul_rn(xa[tx], yob[v][ty]), t10, Jv);
-              Jv = __fmaf_rn(__fmul_rn(xoa[tx], yb[v][ty]), t01, Jv);
-              Jv = __fmaf_rn(__fmul_rn(xa[tx], yb[v][ty]), t11, Jv);
-              float diff = __fsub_rn(Jv, Iv);  // (Jv - Iv) * w with w == 1
-              const float2 d = sD[g];
-              b1[v] = __fmaf_rn(diff, d.x, b1[v]);
-              b2[v] = __fmaf_rn(diff, d.y, b2[v]);
+              const float2 w00 = __fmul2_rn(xo[tx], yo[ty]), w10 = __fmul2_rn(xa[tx], yo[ty]);
+              const float2 w01 = __fmul2_rn(xo[tx], yb[ty]), w11 = __fmul2_rn(xa[tx], yb[ty]);
+              float2 Jv = __fmul2_rn(w00, s[0]);
+              Jv = __ffma2_rn(w10, s[1], Jv);
+              Jv = __ffma2_rn(w01, s[LK_JP], Jv);
+              Jv = __ffma2_rn(w11, s[LK_JP + 1], Jv);
+              float2 d = __fadd2_rn(Jv, nI[ty][tx]);  // (Jv - Iv) * w with w == 1
+              if (!DEF || tx == NT - 1) {
+                if (!lk_on<DEF>(act, 0, ty, tx, xid, yid)) d.x = 0.f;
+                if (!lk_on<DEF>(act, 1, ty, tx, xid, yid)) d.y = 0.f;
+              }
+              b1 = __ffma2_rn(d, Dx[ty][tx], b1);
+              b2 = __ffma2_rn(d, Dy[ty][tx], b2);
             }
+        } else {  // some footprint leaves the staged region or rounds to another texel
+          auto half = [&](int v, float& s1, float& s2) {
+#pragma unroll
+            for (int ty = 0; ty < NT; ty++)
+#pragma unroll
+              for (int tx = 0; tx < NT; tx++) {
+                if (LK_SKIP(v, ty, tx) || !lk_on<DEF>(act, v, ty, tx, xid, yid)) continue;
+                const float Jv = lk_bilinear_s(sJ, J, H, W, pitch, lx[tx], v ? ly[ty].y : ly[ty].x, jox, joy);
+                const float d = __fadd_rn(Jv, v ? nI[ty][tx].y : nI[ty][tx].x);
+                s1 = __fmaf_rn(d, v ? Dx[ty][tx].y : Dx[ty][tx].x, s1);
+                s2 = __fmaf_rn(d, v ? Dy[ty][tx].y : Dy[ty][tx].x, s2);
+              }
+          };
+          half(0, b1.x, b2.x);
+          half(1, b1.y, b2.y);
         }
-      };
-      if (__all_sync(0xffffffffu, inx == 0xFu && iny == 0xFFu))
-        samples(std::true_type());
-      else
-        samples(std::false_type());
-      float B1 = lk_tree(b1[0], b1[1]), B2 = lk_tree(b2[0], b2[1]);
-      float dx = __fmul_rn(__fmaf_rn(A12, B2, -__fmul_rn(A22, B1)), 32.0f);
-      float dy = __fmul_rn(__fmaf_rn(A12, B1, -__fmul_rn(A11, B2)), 32.0f);
-      ptx = __fadd_rn(ptx, dx);
-      pty = __fadd_rn(pty, dy);
+        float B1, B2;
+        lk_tree2(b1, b2, B1, B2);
+        float dx = __fmul_rn(__fmaf_rn(A12, B2, -__fmul_rn(A22, B1)), 32.0f);
+        float dy = __fmul_rn(__fmaf_rn(A12, B1, -__fmul_rn(A11, B2)), 32.0f);
+        ptx = __fadd_rn(ptx, dx);
+        pty = __fadd_rn(pty, dy);
 #pragma unroll
-      for (int t = 0; t < 4; t++) {
-        lx[t] = __fadd_rn(lx[t], dx);
-        ly[0][t] = __fadd_rn(ly[0][t], dy);
-        ly[1][t] = __fadd_rn(ly[1][t], dy);
-      }
-      if (fabsf(dx) < 0.01f && fabsf(dy) < 0.01f) break;
-    }
-    if (err) {
-      // GetError visiting order and guards (:620-653); bits: 1 xBase, 2 yBase, 4 xBase2, 8 yBase2
-      const int ord[16] = {0x000, 0x010, 0x100, 0x110, 0x021, 0x121, 0x202, 0x212,
-                           0x223, 0x034, 0x134, 0x234, 0x308, 0x318, 0x328, 0x33c};
-      float wx[4], wy0[4], wy1[4];  // recomputed here rather than kept live through the steps
-      int bx[2], by0[2], by1[2];
-      lk_weights(xid, p.ws, p.aL, p.aR, wx, bx);
-      lk_weights(yid, p.ws, p.aT, p.aB, wy0, by0);
-      lk_weights(yid + 4, p.ws, p.aT, p.aB, wy1, by1);
-      float e[2] = {0.f, 0.f};
-#pragma unroll
-      for (int v = 0; v < 2; v++) {
-        const float* wy = v ? wy1 : wy0;
-        const int* by = v ? by1 : by0;
-        const int yy = yid + 4 * v;
-#pragma unroll
-        for (int o = 0; o < 16; o++) {
-          int ty = ord[o] >> 8, tx = (ord[o] >> 4) & 15, gb = ord[o] & 15;
-          if ((gb & 1) && !(bx[0] < p.ws)) continue;
-          if ((gb & 2) && !(by[0] < p.ws)) continue;
-          if ((gb & 4) && !(bx[1] < p.ws)) continue;
-          if ((gb & 8) && !(by[1] < p.ws)) continue;
-          float w = __fmul_rn(wx[tx], wy[ty]);
-          float Iv = sI[(gyb + ty * 8 + yy + 1) * LK_IP + gxb + tx * 8 + xid + 1];
-          float Jv = lk_bilinear_s(sJ, J, H, W, pitch, lx[tx], ly[v][ty], jox, joy);
-          float d = __fmul_rn(__fsub_rn(__fdiv_rn(__fmaf_rn(Jv, 16384.f, 256.f), 512.f),
-                                        __fdiv_rn(__fmaf_rn(Iv, 16384.f, 256.f), 512.f)),
-                              w);
-          e[v] = __fadd_rn(e[v], fabsf(d));
+        for (int t = 0; t < NT; t++) {
+          lx[t] = __fadd_rn(lx[t], dx);
+          ly[t] = __fadd2_rn(ly[t], make_float2(dy, dy));
         }
+        if (fabsf(dx) < 0.01f && fabsf(dy) < 0.01f) break;
       }
-      float E = lk_tree(e[0], e[1]);
-      if (lane == 0) err[gid] = __fdiv_rn(E, (float)(32 * p.ws * p.ws));
-    }
-    if (lane == 0) {
-      U[gid] = __fsub_rn(__fadd_rn(ptx, hw), (float)j);
-      V[gid] = __fsub_rn(__fadd_rn(pty, hw), (float)i);
-      if (status) status[gid] = st;
+      if (err) {
+        // GetError visiting order and guards (:620-653); bits: 1 xBase, 2 yBase, 4 xBase2, 8 yBase2
+        const int ord[16] = {0x000, 0x010, 0x100, 0x110, 0x021, 0x121, 0x202, 0x212,
+                             0x223, 0x034, 0x134, 0x234, 0x308, 0x318, 0x328, 0x33c};
+        float wx[4], wy0[4], wy1[4];  // recomputed here rather than kept live through the steps
+        int bx[2], by0[2], by1[2];
+        lk_weights(xid, p.ws, p.aL, p.aR, wx, bx);
+        lk_weights(yid, p.ws, p.aT, p.aB, wy0, by0);
+        lk_weights(yid + 4, p.ws, p.aT, p.aB, wy1, by1);
+        float e[2] = {0.f, 0.f};
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+          const float* wy = v ? wy1 : wy0;
+          const int* by = v ? by1 : by0;
+#pragma unroll
+          for (int o = 0; o < 16; o++) {
+            int ty = ord[o] >> 8, tx = (ord[o] >> 4) & 15, gb = ord[o] & 15;
+            if ((gb & 1) && !(bx[0] < p.ws)) continue;
+            if ((gb & 2) && !(by[0] < p.ws)) continue;
+            if ((gb & 4) && !(bx[1] < p.ws)) continue;
+            if ((gb & 8) && !(by[1] < p.ws)) continue;
+            float w = __fmul_rn(wx[tx], wy[ty]);
+            float Iv = pI[(ty * 8 + 4 * v) * LK_IP + tx * 8];
+            // positions past the window's last tile continue the same additions of 8
+            float x = lx[tx < NT ? tx : NT - 1], y = v ? ly[ty < NT ? ty : NT - 1].y : ly[ty < NT ? ty : NT - 1].x;
+            float Jv = lk_bilinear_s(sJ, J, H, W, pitch, x, y, jox, joy);
+            // the reference's divisions by 512 are exact scalings
+            float d = __fmul_rn(__fsub_rn(__fmul_rn(__fmaf_rn(Jv, 16384.f, 256.f), 1.f / 512.f),
+                                          __fmul_rn(__fmaf_rn(Iv, 16384.f, 256.f), 1.f / 512.f)),
+                                w);
+            e[v] = __fadd_rn(e[v], fabsf(d));
+          }
+        }
+        float E = lk_tree(e[0], e[1]);
+        if (lane == 0) err[gid] = __fdiv_rn(E, (float)(32 * p.ws * p.ws));
+      }
+      if (lane == 0) {
+        U[gid] = __fsub_rn(__fadd_rn(ptx, hw), (float)j);
+        V[gid] = __fsub_rn(__fadd_rn(pty, hw), (float)i);
+        if (status) status[gid] = st;
+      }
     }
   }
+#undef LK_SKIP2
+#undef LK_SKIP
 }
 
 }  // namespace ofb
@@ -408,11 +468,17 @@ extern "C" int of_lk_dense(const float* I, const float* J, float* U, float* V, i
   p.niter = niter;
   dim3 grid((W + LK_PT - 1) / LK_PT, (H + LK_PT - 1) / LK_PT);
   const bool def = p.ws == 27 && !(p.aL | p.aR | p.aT | p.aB);
-  cudaError_t e = def ? OF_SMEM_OPT_IN(lk_dense_kernel<true>, LK_SMEM) : OF_SMEM_OPT_IN(lk_dense_kernel<false>, LK_SMEM);
-  if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_lk_dense: %s", cudaGetErrorString(e));
-  if (def)
-    lk_dense_kernel<true><<<grid, 256, LK_SMEM, as_stream(stream)>>>(I, J, U, V, H, W, pitch, p, status, err);
-  else
-    lk_dense_kernel<false><<<grid, 256, LK_SMEM, as_stream(stream)>>>(I, J, U, V, H, W, pitch, p, status, err);
-  return check_launch("of_lk_dense");
+  // tiles with weight per axis; the error visits one more (of weight 0) when ws < 16
+  const int nt = p.ws > 24 ? 4 : (p.ws > 16 || err) ? 3 : 2;
+  auto run = [&](auto kernel, int threads, cudaError_t e) {
+    if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_lk_dense: %s", cudaGetErrorString(e));
+    kernel<<<grid, threads, LK_SMEM, as_stream(stream)>>>(I, J, U, V, H, W, pitch, p, status, err);
+    return check_launch("of_lk_dense");
+  };
+#define LK_RUN(NT, DEF) \
+  run(lk_dense_kernel<NT, DEF>, lk_threads(NT), OF_SMEM_OPT_IN((lk_dense_kernel<NT, DEF>), LK_SMEM))
+  if (def) return LK_RUN(4, true);
+  if (nt == 4) return LK_RUN(4, false);
+  return nt == 3 ? LK_RUN(3, false) : LK_RUN(2, false);
+#undef LK_RUN
 }

@@ -1,5 +1,6 @@
-"""Dense Lucas-Kanade from initial flows that are infinite, not a number or huge at some
-pixels, against the CPU oracle bit for bit."""
+"""Dense Lucas-Kanade at the edges of its kernel's window tiles, against the CPU oracle bit
+for bit: windows on both sides of a multiple of 8, asymmetric masks, footprints that leave
+the staged region of J or whose positions round across a texel, infinite initial flows."""
 import numpy as np
 import pytest
 
@@ -12,6 +13,37 @@ def frames(h, w, seed):
     from ofb200 import synthetic as S
     a, b, _, _ = S.piv_pair(h, w, "lamb_oseen", seed=seed, core_radius=10, density=0.08)
     return a.astype(np.float32), b.astype(np.float32)
+
+
+def flow(kind, h, w, rng):
+    if kind == "spread":  # neighbouring pixels tens of pixels apart: outside the staged region
+        return (rng.uniform(-30, 30, (h, w)).astype(np.float32) for _ in range(2))
+    # positions on texels and one float32 step to either side of them
+    base = rng.integers(-2, 3, (2, h, w)).astype(np.float32)
+    step = rng.integers(-1, 2, (2, h, w))
+    out = np.where(step == 0, base, np.nextafter(base, base + step.astype(np.float32)))
+    return out[0].astype(np.float32), out[1].astype(np.float32)
+
+
+@pytest.mark.parametrize("err", [False, True])
+@pytest.mark.parametrize("kind", ["texel", "spread"])
+@pytest.mark.parametrize("hw,asym", [(1, (0, 0, 0, 0)), (3, (1, 0, 0, 1)), (7, (0, 0, 0, 0)), (8, (0, 1, 0, 1)),
+                                     (11, (0, 0, 0, 0)), (12, (0, 0, 0, 0)), (13, (0, 0, 0, 0)), (13, (1, 0, 0, 1)),
+                                     (15, (0, 1, 1, 0))])
+def test_lk_window_tiles(cuda_ok, hw, asym, kind, err):
+    import torch
+    from ofb200 import ops
+    h, w = 21, 27
+    a, b = frames(h, w, hw)
+    U0, V0 = flow(kind, h, w, np.random.default_rng(hw))
+    U, V = (torch.from_numpy(t.copy()).cuda() for t in (U0, V0))
+    st = torch.empty((h, w), dtype=torch.uint8, device="cuda") if err else None
+    er = torch.empty((h, w), dtype=torch.float32, device="cuda") if err else None
+    ops.lk_dense(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), U, V, hw, 5, asym, st, er)
+    Uo, Vo, sto, ero = O.lk_dense(a, b, U0, V0, hw, 5, asym, want_status=True)
+    assert np.array_equal(U.cpu().numpy(), Uo) and np.array_equal(V.cpu().numpy(), Vo)
+    if err:
+        assert np.array_equal(st.cpu().numpy(), sto) and np.array_equal(er.cpu().numpy(), ero)
 
 
 @pytest.mark.parametrize("hw", [5, 9, 13])
