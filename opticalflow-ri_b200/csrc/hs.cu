@@ -68,72 +68,141 @@ __global__ void hs_sweep_kernel(const float* __restrict__ fx, const float* __res
   Vn[i] = __fsub_rn(va, __fmul_rn(gy, der));
 }
 
-// Temporally blocked sweeps: one pass runs up to HB_T sweeps on a tile held in shared
-// memory, so the three derivative planes and (U, V) cross HBM/L2 once per HB_T sweeps
-// instead of once per sweep.  A CTA owns 56 x 32 pixels and stages a 64 x 40 region (halo
-// HB_T): sweep s computes the cells at least s + 1 from the region's edge, which after
-// HB_T sweeps leaves exactly the owned pixels exact; they are written back.  On image
-// borders every neighbour index goes through the same 'mirror' map as hs_sweep_kernel
-// (mapped neighbours stay within one row / column of their cell, so inside the region),
-// and out-of-image cells are neither computed nor read.  Each cell's arithmetic is
-// hs_sweep_kernel's: the averaging weights are float32 values (24-bit mantissas), so every
-// product with a float32 sample is exact in double and fma(v, w, acc) rounds exactly as
-// the separate multiply and add.  U and V sit in shared memory as float64 copies of their
-// float32 values, so the float64 sums read their operands without a conversion each.
-constexpr int HB_T = 4, HB_TW = 56, HB_TH = 32, HB_RW = HB_TW + 2 * HB_T, HB_RH = HB_TH + 2 * HB_T;  // 64 x 40
-constexpr int HB_PL = HB_RW * HB_RH;
-constexpr size_t HB_SMEM = 3 * (size_t)HB_PL * sizeof(float) + 4 * (size_t)HB_PL * sizeof(double);  // 110 KB
+// Temporally blocked sweeps: one pass runs up to HB_T sweeps on a region of the image whose
+// cells the CTA's threads hold in registers in 2 x 4 blocks (hr_sweep, hsweep.cuh), so the
+// three derivative planes and (U, V) cross HBM/L2 once per HB_T sweeps.  A CTA owns
+// 56 x 24 pixels and sweeps a 64 x 32 region (halo HB_T): after sweep s the cells at least
+// s + 1 from the region's edge are exact, after HB_T sweeps the owned ones, which are written
+// back.  A warp is one row of blocks.
+//
+// What bounds it: the issue slots (65 instructions per cell update, 16 of them float64
+// multiply-adds) at 50 % busy, and the latency of the pass's loads and barriers behind two
+// CTAs per SM (128 registers a thread).  600 sweeps, one pair alone: 256 x 256 2.75 -> 1.46 ms,
+// 512 x 512 3.3 -> 1.55 ms; 100 sweeps of 2048 x 2048 3.96 -> 2.3 ms (106 -> 180 G cell updates
+// per second) against the column walk with one cell per thread and row it replaces.  4 x 4
+// blocks spill at 12 warps per SM (113 G/s), a 64 x 64 region in one CTA of 512 threads does
+// less halo work but leaves its loads exposed (164 G/s).
+constexpr int HB_T = 4, HB_RW = 64, HB_RH = 32, HB_TW = HB_RW - 2 * HB_T, HB_TH = HB_RH - 2 * HB_T;
+constexpr int HB_BX = 2, HB_BY = 4;  // block of a thread
+using HbGeom = HrGeom<HB_RW, HB_RH, HB_BX, HB_BY>;
+constexpr size_t HB_SMEM = 2 * HbGeom::BUF;  // ping-pong: one barrier per sweep
 
-__global__ void __launch_bounds__(HQ_THREADS, 2) hs_pass_kernel(const float* __restrict__ fx, const float* __restrict__ fy,
-                                                      const float* __restrict__ ft, const float* __restrict__ U,
-                                                      const float* __restrict__ V, float* __restrict__ Un,
-                                                      float* __restrict__ Vn, int H, int W, int pitch, float a2,
-                                                      int nsw) {
-  extern __shared__ float hb_sm[];
-  float* sfx = hb_sm;
-  float* sfy = sfx + HB_PL;
-  float* sft = sfy + HB_PL;
-  // ping-pong buffer q (float64): u at plane 2q after the float planes, v right after it
-  double* const hb_uv = reinterpret_cast<double*>(sft + HB_PL);
-#define HB_U(q) (hb_uv + (2 * (q)) * HB_PL)
-#define HB_V(q) (hb_uv + (1 + 2 * (q)) * HB_PL)
-  const int x0 = blockIdx.x * HB_TW, y0 = blockIdx.y * HB_TH;
-  for (int k = threadIdx.x; k < HB_PL; k += HQ_THREADS) {
-    const int r = k / HB_RW, c = k - r * HB_RW;
-    const int gy = y0 - HB_T + r, gx = x0 - HB_T + c;
-    if (gy < 0 || gy >= H || gx < 0 || gx >= W) continue;  // never read
-    const size_t i = (size_t)gy * pitch + gx;
-    sfx[k] = fx[i];
-    sfy[k] = fy[i];
-    sft[k] = ft[i];
-    HB_U(0)[k] = U[i];
-    HB_V(0)[k] = V[i];
+// A block's cells of a plane, 0 outside the image.  `inside`: the whole region is, and the
+// rows are 8-byte aligned: no branch between the loads, which are then all in flight at once.
+__device__ __forceinline__ void hb_load(float2 out[HB_BY], const float* __restrict__ p, int gy0, int gx0, int H, int W,
+                                        int pitch, bool inside) {
+  const float* r = p + (ptrdiff_t)gy0 * pitch + gx0;
+  if (inside) {
+#pragma unroll
+    for (int j = 0; j < HB_BY; j++) out[j] = *reinterpret_cast<const float2*>(r + (size_t)j * pitch);
+  } else {
+#pragma unroll
+    for (int j = 0; j < HB_BY; j++) {
+      const bool y = gy0 + j >= 0 && gy0 + j < H;
+      const float* q = r + (ptrdiff_t)j * pitch;
+      out[j] = make_float2(y && gx0 >= 0 && gx0 < W ? q[0] : 0.f, y && gx0 + 1 >= 0 && gx0 + 1 < W ? q[1] : 0.f);
+    }
   }
+}
+
+__device__ __forceinline__ void hb_store2(float* __restrict__ p, const double v[2], int gy, int gx, int H, int W,
+                                          int pitch, bool vec) {
+  if (gy >= H || gx >= W) return;
+  float* r = p + (size_t)gy * pitch + gx;
+  if (vec && gx + 2 <= W) {
+    *reinterpret_cast<float2*>(r) = make_float2((float)v[0], (float)v[1]);
+  } else {
+    r[0] = (float)v[0];
+    if (gx + 1 < W) r[1] = (float)v[1];
+  }
+}
+
+struct HbPass {
+  const float *fx, *fy, *ft, *U, *V;
+  float *Un, *Vn;
+  int H, W, pitch, nsw, vec;
+  float a2;
+  float one;  // 1.0f (hr_row)
+};
+
+using HbBlock = HrBlock<HB_BX, HB_BY>;
+
+__device__ __forceinline__ void hb_load_uv(HbBlock& K, const HbPass& P, int gy0, int gx0, bool inside) {
+  float2 u[HB_BY], v[HB_BY];
+  hb_load(u, P.U, gy0, gx0, P.H, P.W, P.pitch, inside);
+  hb_load(v, P.V, gy0, gx0, P.H, P.W, P.pitch, inside);
+#pragma unroll
+  for (int j = 0; j < HB_BY; j++) {
+    K.u[j][0] = u[j].x; K.u[j][1] = u[j].y;
+    K.v[j][0] = v[j].x; K.v[j][1] = v[j].y;
+  }
+}
+
+// The sweeps of a pass; on return the CTA's last sweep is in the blocks only.
+template <bool EDGE, bool DIV>
+__device__ __forceinline__ void hb_sweeps(HbBlock& K, const HbPass& P, double2* sm, bool in, int r0, int c0, int gy0,
+                                          int gx0) {
+  if (in) hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, sm, r0, c0);
   __syncthreads();
-  const bool edge = x0 < HB_T || y0 < HB_T || x0 + HB_TW + HB_T > W || y0 + HB_TH + HB_T > H;
+  // a warp whose rows no later sweep reads (the outermost, in the last sweep) sits out
+  auto needed = [&](int k) { return in && r0 + HB_BY > 1 + k && r0 < HB_RH - 1 - k; };
 #pragma unroll 1
-  for (int s = 0; s < nsw; s++) {
-    const int q = s & 1;
-    if (edge)
-      hq_sweep2<HB_RW, HB_RH, HB_T, true, false, HQ_THREADS, false>(sfx, sfy, sft, nullptr, HB_U(q), HB_V(q),
-                                                                   HB_U(q ^ 1), HB_V(q ^ 1), s, x0, y0, H, W, a2);
-    else
-      hq_sweep2<HB_RW, HB_RH, HB_T, false, false, HQ_THREADS, false>(sfx, sfy, sft, nullptr, HB_U(q), HB_V(q),
-                                                                    HB_U(q ^ 1), HB_V(q ^ 1), s, x0, y0, H, W, a2);
+  for (int s = 0; s < P.nsw; s += 2) {
+    double2* const b0 = sm;
+    double2* const b1 = sm + HB_RW * HB_RH;
+    if (needed(s)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, EDGE, DIV>(K, b0, r0, c0, gy0, gx0, P.H, P.W);
+    if (s + 1 >= P.nsw) break;
+    if (needed(s)) hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, b1, r0, c0);
+    __syncthreads();
+    if (needed(s + 1)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, EDGE, DIV>(K, b1, r0, c0, gy0, gx0, P.H, P.W);
+    if (s + 2 >= P.nsw) break;
+    if (needed(s + 1)) hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, b0, r0, c0);
     __syncthreads();
   }
-  const double* fu = HB_U(nsw & 1);
-  const double* fv = HB_V(nsw & 1);
-  for (int k = threadIdx.x; k < HB_TW * HB_TH; k += HQ_THREADS) {
-    const int r = k / HB_TW, c = k - r * HB_TW;
-    const int y = y0 + r, x = x0 + c;
-    if (y >= H || x >= W) continue;
-    const int o = (r + HB_T) * HB_RW + c + HB_T;
-    Un[(size_t)y * pitch + x] = (float)fu[o];
-    Vn[(size_t)y * pitch + x] = (float)fv[o];
+}
+
+__global__ void __launch_bounds__(HbGeom::NT, 2) hs_pass_kernel(const HbPass P) {
+  // passes after the first are programmatic dependents of the pass before them: they take the
+  // SM slots its tail frees and load the derivatives, which do not change during a solve
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  extern __shared__ __align__(16) double2 hb_sm[];
+  const int x0 = blockIdx.x * HB_TW - HB_T, y0 = blockIdx.y * HB_TH - HB_T;  // image position of region cell (0, 0)
+  const int c0 = ((int)threadIdx.x % HbGeom::NX) * HB_BX, r0 = ((int)threadIdx.x / HbGeom::NX) * HB_BY;
+  const int gx0 = x0 + c0, gy0 = y0 + r0;
+  const bool in = gx0 + HB_BX > 0 && gy0 + HB_BY > 0 && gx0 < P.W && gy0 < P.H;  // the block has cells in the image
+  HbBlock K;
+  const bool edge = x0 < 0 || y0 < 0 || x0 + HB_RW > P.W || y0 + HB_RH > P.H, inside = !edge && P.vec;
+  bool ok = true;
+  if (in) {
+    float2 a[HB_BY], b[HB_BY], c[HB_BY];
+    hb_load(a, P.fx, gy0, gx0, P.H, P.W, P.pitch, inside);
+    hb_load(b, P.fy, gy0, gx0, P.H, P.W, P.pitch, inside);
+    hb_load(c, P.ft, gy0, gx0, P.H, P.W, P.pitch, inside);
+#pragma unroll
+    for (int j = 0; j < HB_BY; j++) {
+      K.g[j][0] = make_float2(a[j].x, b[j].x);
+      K.g[j][1] = make_float2(a[j].y, b[j].y);
+      K.gt[j][0] = c[j].x; K.gt[j][1] = c[j].y;
+    }
+    ok = hr_init_den(K, P.a2, P.one);
   }
-#undef HB_U
-#undef HB_V
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (in) hb_load_uv(K, P, gy0, gx0, inside);
+  if (edge)
+    hb_sweeps<true, false>(K, P, hb_sm, in, r0, c0, gy0, gx0);
+  else
+    hb_sweeps<false, false>(K, P, hb_sm, in, r0, c0, gy0, gx0);
+  if (__syncthreads_or(in && !(ok && hr_in_range(K)))) {  // rare: see hr_row
+    if (in) hb_load_uv(K, P, gy0, gx0, inside);
+    hb_sweeps<true, true>(K, P, hb_sm, in, r0, c0, gy0, gx0);
+  }
+  if (in && c0 >= HB_T && c0 < HB_T + HB_TW && r0 >= HB_T && r0 < HB_T + HB_TH) {
+#pragma unroll
+    for (int j = 0; j < HB_BY; j++) {
+      hb_store2(P.Un, K.u[j], gy0 + j, gx0, P.H, P.W, P.pitch, P.vec);
+      hb_store2(P.Vn, K.v[j], gy0 + j, gx0, P.H, P.W, P.pitch, P.vec);
+    }
+  }
 }
 
 __global__ void copy2_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ ao,
@@ -239,14 +308,27 @@ extern "C" int of_hs_solve(const float* I0, const float* I1, float* U, float* V,
     if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_hs_solve: %s", cudaGetErrorString(e));
     const int np = (niter + HB_T - 1) / HB_T;
     dim3 pg((W + HB_TW - 1) / HB_TW, (H + HB_TH - 1) / HB_TH);
+    // the workspace planes start 256-byte aligned: the callers' U, V decide
+    const int vec = (pitch % 2) == 0 && ((reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(V)) & 7) == 0;
     for (int p = 0; p < np; p++) {
       // the last pass writes U, V; earlier ones alternate with Ub, Vb; the first reads U0, V0
       const bool to_uv = ((np - 1 - p) & 1) == 0;
       const float* su = p == 0 ? U0 : (to_uv ? Ub : U);
       const float* sv = p == 0 ? V0 : (to_uv ? Vb : V);
       const int nsw = niter - p * HB_T < HB_T ? niter - p * HB_T : HB_T;
-      hs_pass_kernel<<<pg, HQ_THREADS, HB_SMEM, st>>>(fx, fy, ft, su, sv, to_uv ? U : Ub, to_uv ? V : Vb, H, W, pitch, a2,
-                                              nsw);
+      HbPass P{fx, fy, ft, su, sv, to_uv ? U : Ub, to_uv ? V : Vb, H, W, pitch, nsw, vec, a2, 1.0f};
+      cudaLaunchAttribute pdl[1];
+      pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      pdl[0].val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = pg;
+      cfg.blockDim = dim3(HbGeom::NT);
+      cfg.dynamicSmemBytes = HB_SMEM;
+      cfg.stream = st;
+      cfg.attrs = pdl;
+      cfg.numAttrs = p > 0 ? 1 : 0;
+      e = cudaLaunchKernelEx(&cfg, hs_pass_kernel, P);
+      if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_hs_solve: pass launch: %s", cudaGetErrorString(e));
     }
     long long n = 2 + np;
     if (err_out) {

@@ -221,4 +221,210 @@ __device__ __forceinline__ void hq_sweep2(const float* __restrict__ sfx, const f
   }
 }
 
+// ---- Register-blocked sweep (bit-exact arithmetic) ---------------------------------------
+// A thread owns a BX x BY block of region cells and keeps their (u, v), as float64 copies of
+// the float32 values, and their derivatives in registers through all sweeps of a pass; a sweep
+// exchanges only the blocks' boundary cells through shared memory.  A cell update then costs
+// 20 bytes of reads and 12 of writes at 4 x 4 where a column walk reads 72 and writes 16.
+// The exchange buffer holds region cell (r, c) as a double2 (u, v) at [r][c % BX][c / BX], so
+// that the threads of a row, BX cells apart, access consecutive 16-byte words.
+template <int RW, int RH, int BX, int BY>
+struct HrGeom {
+  static_assert(RW % BX == 0 && RH % BY == 0, "whole blocks");
+  static constexpr int NX = RW / BX, NY = RH / BY, NT = NX * NY;
+  static constexpr size_t BUF = (size_t)RW * RH * sizeof(double2);
+  static __device__ __forceinline__ int at(int r, int c) { return r * RW + (c % BX) * NX + c / BX; }
+};
+
+// One window row of a block: its BX cells and the cell to either side.
+template <int BX>
+struct HrRow {
+  double u[BX + 2], v[BX + 2];
+};
+
+template <int BX, int BY>
+struct HrBlock {
+  double u[BY][BX], v[BY][BX];
+  float2 g[BY][BX];    // spatial derivatives (fx, fy)
+  float gt[BY][BX];    // temporal derivative
+  float y[BY][BX];     // 1 / den, correctly rounded
+  float a2;            // alpha^2
+  float one;           // 1.0f, unknown to the assembler (see hr_row)
+  unsigned lo;         // range of the numerators seen: smallest 2 |num| (bits) - 1
+  float hi;            // and largest |num|
+};
+
+// Where the quotient by refinement (hr_row) is the correctly rounded one: for den in [2^-40,
+// 2^40] and |num| in [2^-60, 2^60] no intermediate leaves the normal range and the residuals
+// are exact (multiples of 2^-46 |num|; the quotients are at least 2^-100); and for num = +0,
+// which is what a zero numerator is unless gt is -0.
+constexpr float HR_DEN = 1.0995116e12f, HR_NUM = 1.1529215e18f;
+constexpr unsigned HR_LO = 2u * 0x21800000u - 1u;  // 2^-60
+
+__device__ __forceinline__ float hr_max_nan(float a, float b) {  // NaN if either is
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+__device__ __forceinline__ float hr_den(float2 g, float a2) {
+  const float2 q = __fmul2_rn(g, g);
+  return __fadd_rn(__fadd_rn(a2, q.x), q.y);
+}
+
+// The block's reciprocals; false when a denominator or gt is outside the ranges above.
+template <int BX, int BY>
+__device__ __forceinline__ bool hr_init_den(HrBlock<BX, BY>& K, float a2, float one) {
+  K.a2 = a2;
+  K.one = one;
+  K.lo = 0xffffffffu;
+  K.hi = 0.f;
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < BY; j++)
+#pragma unroll
+    for (int i = 0; i < BX; i++) {
+      const float den = hr_den(K.g[j][i], a2);
+      ok = ok && den >= 1.f / HR_DEN && den <= HR_DEN && __float_as_uint(K.gt[j][i]) != 0x80000000u;
+      K.y[j][i] = __frcp_rn(den);
+    }
+  return ok;
+}
+
+// Whether every quotient since hr_init_den was in range.
+template <int BX, int BY>
+__device__ __forceinline__ bool hr_in_range(const HrBlock<BX, BY>& K) {
+  return K.lo >= HR_LO && K.hi <= HR_NUM;
+}
+
+// The update of a block's row j from the old window rows U (above), C, D (below):
+// hs_sweep_kernel's arithmetic, the 8 neighbours summed in its order; the results replace the
+// block's cells.  DIV: the quotient by __fdiv_rn; else by two residual corrections of num * y,
+// y the correctly rounded reciprocal, the last of which is correctly rounded (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Develop. 34(1), 1990) for numerators in range.  The range is only recorded here: one
+// check per pass, and a CTA that fails it repeats the pass with DIV.
+template <int BX, int BY, bool DIV>
+__device__ __forceinline__ void hr_row(HrBlock<BX, BY>& K, int j, const HrRow<BX>& U, const HrRow<BX>& C,
+                                       const HrRow<BX>& D) {
+  const double wc = (double)(1.0f / 12.0f), we = (double)(1.0f / 6.0f);
+#pragma unroll
+  for (int i = 0; i < BX; i++) {
+    double a = 0.0, b = 0.0;  // float32 values held as float64: no conversions here
+    a = __fma_rn(U.u[i], wc, a);     b = __fma_rn(U.v[i], wc, b);
+    a = __fma_rn(U.u[i + 1], we, a); b = __fma_rn(U.v[i + 1], we, b);
+    a = __fma_rn(U.u[i + 2], wc, a); b = __fma_rn(U.v[i + 2], wc, b);
+    a = __fma_rn(C.u[i], we, a);     b = __fma_rn(C.v[i], we, b);
+    a = __fma_rn(C.u[i + 2], we, a); b = __fma_rn(C.v[i + 2], we, b);
+    a = __fma_rn(D.u[i], wc, a);     b = __fma_rn(D.v[i], wc, b);
+    a = __fma_rn(D.u[i + 1], we, a); b = __fma_rn(D.v[i + 1], we, b);
+    a = __fma_rn(D.u[i + 2], wc, a); b = __fma_rn(D.v[i + 2], wc, b);
+    const float2 m = make_float2((float)a, (float)b), g = K.g[j][i];
+    const float2 gm = __fmul2_rn(g, m);
+    const float num = __fadd_rn(__fadd_rn(gm.x, gm.y), K.gt[j][i]);
+    const float den = hr_den(g, K.a2);
+    float der;
+    if (DIV) {
+      der = __fdiv_rn(num, den);
+    } else {
+      const float y = K.y[j][i];
+      float q = __fmul_rn(num, y);
+      q = __fmaf_rn(__fmaf_rn(-q, den, num), y, q);
+      der = __fmaf_rn(__fmaf_rn(-q, den, num), y, q);
+      K.lo = min(K.lo, 2u * __float_as_uint(num) - 1u);
+      K.hi = hr_max_nan(K.hi, fabsf(num));
+    }
+    // m - g der with two roundings: the assembler would fuse a packed product into a packed
+    // sum, so the product goes through a multiply-add by minus one that it cannot see
+    const float2 r = __ffma2_rn(__fmul2_rn(g, make_float2(der, der)), make_float2(-K.one, -K.one), m);
+    K.u[j][i] = (double)r.x;
+    K.v[j][i] = (double)r.y;
+  }
+}
+
+// The block's boundary cells into the exchange buffer (r0, c0: its first region cell).
+template <int RW, int RH, int BX, int BY>
+__device__ __forceinline__ void hr_publish(const HrBlock<BX, BY>& K, double2* buf, int r0, int c0) {
+  using G = HrGeom<RW, RH, BX, BY>;
+#pragma unroll
+  for (int j = 0; j < BY; j++)
+#pragma unroll
+    for (int i = 0; i < BX; i++)
+      if (j == 0 || j == BY - 1 || i == 0 || i == BX - 1)
+        buf[r0 * RW + c0 / BX + j * RW + i * G::NX] = make_double2(K.u[j][i], K.v[j][i]);
+}
+
+// One sweep of the block from the exchange buffer `buf` (the other blocks' cells before the
+// sweep).  EDGE: the region touches the image border, where the neighbour beyond it is the
+// mirror cell: -1 shows 1 and n shows n - 2, which the window holds on the cell's other side
+// (gy0, gx0: image position of the block's first cell; H, W >= 2).  Cells outside the image
+// or on the region's rim get values that no exact cell reads.
+template <int RW, int RH, int BX, int BY, bool EDGE, bool DIV>
+__device__ __forceinline__ void hr_sweep(HrBlock<BX, BY>& K, const double2* buf, int r0, int c0, int gy0, int gx0,
+                                         int H, int W) {
+  using G = HrGeom<RW, RH, BX, BY>;
+  const int cb = c0 / BX;
+  // the columns beside the block (held inside the region at its rim)
+  const int cl = c0 > 0 ? (BX - 1) * G::NX + cb - 1 : cb, cr = c0 + BX < RW ? cb + 1 : cb;
+  auto fix = [&](HrRow<BX>& R) {  // the window's columns at the image border
+    if (!EDGE) return;
+    if (gx0 == 0) {
+      R.u[0] = R.u[2];
+      R.v[0] = R.v[2];
+    }
+    if (gx0 + BX >= W) {
+#pragma unroll
+      for (int i = 2; i < BX + 2; i++)
+        if (gx0 - 1 + i == W) {
+          R.u[i] = R.u[i - 2];
+          R.v[i] = R.v[i - 2];
+        }
+    }
+  };
+  auto ring = [&](HrRow<BX>& R, int row) {  // a row above or below the block
+    const double2* b = buf + row * RW;
+    double2 t = b[cl];
+    R.u[0] = t.x;
+    R.v[0] = t.y;
+#pragma unroll
+    for (int i = 0; i < BX; i++) {
+      t = b[i * G::NX + cb];
+      R.u[i + 1] = t.x;
+      R.v[i + 1] = t.y;
+    }
+    t = b[cr];
+    R.u[BX + 1] = t.x;
+    R.v[BX + 1] = t.y;
+    fix(R);
+  };
+  auto own = [&](HrRow<BX>& R, int j) {  // the block's row j with the cells beside it
+    const double2* b = buf + (r0 + j) * RW;
+    const double2 l = b[cl], r = b[cr];
+    R.u[0] = l.x;
+    R.v[0] = l.y;
+#pragma unroll
+    for (int i = 0; i < BX; i++) {
+      R.u[i + 1] = K.u[j][i];
+      R.v[i + 1] = K.v[j][i];
+    }
+    R.u[BX + 1] = r.x;
+    R.v[BX + 1] = r.y;
+    fix(R);
+  };
+  HrRow<BX> w[3];
+  ring(w[0], r0 > 0 ? r0 - 1 : 0);
+  own(w[1], 0);
+#pragma unroll
+  for (int j = 0; j < BY; j++) {
+    HrRow<BX>&U = w[j % 3], &C = w[(j + 1) % 3], &D = w[(j + 2) % 3];
+    if (j + 1 < BY)
+      own(D, j + 1);
+    else
+      ring(D, r0 + BY < RH ? r0 + BY : RH - 1);
+    if (EDGE && gy0 + j == 0) U = D;
+    if (EDGE && gy0 + j == H - 1) D = U;
+    hr_row<BX, BY, DIV>(K, j, U, C, D);
+  }
+}
+
 }  // namespace ofb
