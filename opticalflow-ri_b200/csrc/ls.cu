@@ -12,8 +12,6 @@
 // previous sweep's error from device memory, so the host enqueues maxnum sweeps with no
 // synchronisation and the sequence can be captured in a CUDA graph.
 // Inside the solver u is the row (y) component and v the column (x) component (:38-39).
-#include <stdlib.h>
-
 #include "common.cuh"
 #include "tma.cuh"
 
@@ -319,10 +317,8 @@ constexpr int LB_CPLANE = LB_RW * LB_CH * 4;                 // 7424 B
 static_assert(LB_CPLANE % 128 == 0, "the u, v planes after the coefficients must start 128-byte aligned");
 constexpr int LB_PL = LB_RW * LB_CH;                         // floats per coefficient plane
 constexpr int LB_COEF_BYTES = 8 * LB_CPLANE;
-// The float64-sum pass ping-pongs (u, v) between two buffers; the float32 pass updates one
-// buffer in place (each warp keeps the old values of its band's boundary rows in registers),
-// which brings it to 75.5 KB: 3 CTAs per SM.
-constexpr size_t lb_smem(bool fast) { return LB_COEF_BYTES + (fast ? 2 : 4) * LB_PLANE + 128 + 128; }
+// (u, v) ping-pong between two buffers.
+constexpr size_t LB_SMEM = LB_COEF_BYTES + 4 * LB_PLANE + 128 + 128;
 #ifndef OF_LS_PASS_WARPS
 #define OF_LS_PASS_WARPS 6
 #endif
@@ -487,209 +483,432 @@ __device__ __forceinline__ void lb_strip(const LbPlane* su, const LbPlane* sv, c
 // ---- float32 pass (OF_LS_FAST) ----------------------------------------------------------
 // The same sweep, tile and stop rule with float32 arithmetic throughout: no float64 stencil
 // sums, no conversions, fused multiply-adds.  The stencils share their parts: per field the
-// vertical difference vd = down - up and sum vs = up + down of the lane's four columns give
-// D (= vd / 2), F (= vs), M (= (vd[c+1] - vd[c-1]) / 4) and, with the centre row's
-// neighbours, D^T (= (right - left) / 2), F^T (= left + right) and H (= vs[c-1] + vs[c] +
-// vs[c+1] + left + right in the interior); the constant factors are folded into the
-// coefficients (exact power-of-two scalings).  Results differ from the reference's float32
-// fields by float32 rounding only (<= 1e-3 px of the float64 answer at the configurations).
-struct LbRowF {
-  float2 cu, cv;           // the lane's cell pair
-  float lu, ru, lv, rv;    // the window's outer columns (2 lane - 1, 2 lane + 2)
-};
-
-template <bool EDGE>
-__device__ __forceinline__ void lbf_load(LbRowF& R, const LbPlane* su, const LbPlane* sv, int row, const LbCols& c) {
-  if (EDGE) {
-    R.cu = f2(su[row][c.k[1]], su[row][c.k[2]]);
-    R.cv = f2(sv[row][c.k[1]], sv[row][c.k[2]]);
-  } else {
-    R.cu = *reinterpret_cast<const float2*>(&su[row][c.k[1]]);
-    R.cv = *reinterpret_cast<const float2*>(&sv[row][c.k[1]]);
-  }
-  R.lu = su[row][c.k[0]];
-  R.ru = su[row][c.k[3]];
-  R.lv = sv[row][c.k[0]];
-  R.rv = sv[row][c.k[3]];
-}
+// vertical difference vd = down - up and sum vs = up + down of a column give D (= vd / 2), F
+// (= vs), M (= (vd[c+1] - vd[c-1]) / 4) and, with the centre row's neighbours, D^T (= (right -
+// left) / 2), F^T (= left + right) and H (= vs[c-1] + vs[c] + vs[c+1] + left + right in the
+// interior); the constant factors are folded into the coefficients (exact power-of-two
+// scalings).  Results differ from the reference's float32 fields by float32 rounding only
+// (<= 1e-3 px of the float64 answer at the configurations).
+//
+// Registers hold what a sweep reads: a thread owns 2 x 4 cells of the region with their eight
+// coefficients for the whole pass, as (u, v) pairs, so that the stencils of both fields are one
+// packed f32x2 operation.  A warp is a row of blocks (64 columns x 4 rows): the cells beside a
+// block come from the neighbouring lanes, and only the blocks' first and last rows go through
+// shared memory (two buffers, one barrier per sweep).
+constexpr int LF_BY = 4, LF_NW = 8, LF_NT = 32 * LF_NW;
+static_assert(LB_RW == 64 && LF_NW * LF_BY >= LB_RH, "a warp covers the region's columns, the warps its rows");
+constexpr size_t LF_BUF = LF_NW * 2 * 32;  // float4 (u0, v0, u1, v1) of the blocks' first and last rows
 
 // Packed float32 arithmetic of the float32 pass: sm_100's builtins (the compiler pairs the
 // registers itself; contraction is welcome here).  a - b is one fused multiply-add.
 __device__ __forceinline__ float2 fadd2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 fsub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 
-// 8-neighbour sum of the pair with out-of-image neighbours as 0 (H's 'constant' border)
-__device__ __forceinline__ float2 lbf_hsum_edge(const LbRowF& U, const LbRowF& C, const LbRowF& D, bool T, bool B,
-                                                bool L0, bool R0, bool L1, bool R1, bool uv) {
-  const float2 u = uv ? U.cv : U.cu, c = uv ? C.cv : C.cu, d = uv ? D.cv : D.cu;
-  const float ul = uv ? U.lv : U.lu, ur = uv ? U.rv : U.ru, cl = uv ? C.lv : C.lu, cr = uv ? C.rv : C.ru;
-  const float dl = uv ? D.lv : D.lu, dr = uv ? D.rv : D.ru;
-  float h0 = (T || L0) ? 0.f : ul;
-  h0 = __fadd_rn(h0, T ? 0.f : u.x);
-  h0 = __fadd_rn(h0, (T || R0) ? 0.f : u.y);
-  h0 = __fadd_rn(h0, L0 ? 0.f : cl);
-  h0 = __fadd_rn(h0, R0 ? 0.f : c.y);
-  h0 = __fadd_rn(h0, (B || L0) ? 0.f : dl);
-  h0 = __fadd_rn(h0, B ? 0.f : d.x);
-  h0 = __fadd_rn(h0, (B || R0) ? 0.f : d.y);
-  float h1 = (T || L1) ? 0.f : u.x;
-  h1 = __fadd_rn(h1, T ? 0.f : u.y);
-  h1 = __fadd_rn(h1, (T || R1) ? 0.f : ur);
-  h1 = __fadd_rn(h1, L1 ? 0.f : c.x);
-  h1 = __fadd_rn(h1, R1 ? 0.f : cr);
-  h1 = __fadd_rn(h1, (B || L1) ? 0.f : d.x);
-  h1 = __fadd_rn(h1, B ? 0.f : d.y);
-  h1 = __fadd_rn(h1, (B || R1) ? 0.f : dr);
-  return f2(h0, h1);
-}
+struct LfBlock {
+  float2 w[LF_BY][2];                     // (u, v)
+  float2 iixy[LF_BY][2], ixyt[LF_BY][2];  // (IIx, IIy), (Ixt, Iyt)
+  float ii[LF_BY][2];
+  float2 b1[LF_BY][2];                    // (B11, B12)
+  float b22[LF_BY][2];                    // B22
+};
 
+struct LfRow {  // a window row: the cell left of the block, its two cells, the cell to the right
+  float2 c[4];
+};
+
+struct LfGeom {  // the block's place
+  int r0, c0;    // first region row and (even) column
+  int gy0, gx0;  // its image position
+  int H, W;
+  float h;
+};
+
+// A row of the window from its two cells: the outer ones from the neighbouring lanes.  EDGE:
+// columns beyond the image take the nearest column's value.
 template <bool EDGE>
-__device__ __forceinline__ void lbf_pair(const LbRowF& U, const LbRowF& C, const LbRowF& D, const LbStrip& S, int row,
-                                         int gy, bool own_row, float& acc_u, float& acc_v) {
-  const int o = (row - 1) * LB_RW + S.c0;  // coefficient rows start at region row 1
-  const float* sc = S.sc;
-  const float2 IIx = *reinterpret_cast<const float2*>(sc + o);
-  const float2 IIy = *reinterpret_cast<const float2*>(sc + LB_PL + o);
-  const float2 II = *reinterpret_cast<const float2*>(sc + 2 * LB_PL + o);
-  // vertical differences and sums at the pair and at the outer columns
-  const float2 vdu = fsub2(D.cu, U.cu), vsu = fadd2(U.cu, D.cu);
-  const float2 vdv = fsub2(D.cv, U.cv), vsv = fadd2(U.cv, D.cv);
-  const float2 vdo_u = fsub2(f2(D.lu, D.ru), f2(U.lu, U.ru));  // (left column, right column)
-  const float2 vdo_v = fsub2(f2(D.lv, D.rv), f2(U.lv, U.rv));
-  const float2 mdu = fsub2(f2(vdu.y, vdo_u.y), f2(vdo_u.x, vdu.x));  // 4 M
-  const float2 mdv = fsub2(f2(vdv.y, vdo_v.y), f2(vdo_v.x, vdv.x));
-  // centre-row neighbours of the pair
-  const float2 Lu = f2(C.lu, C.cu.x), Ru = f2(C.cu.y, C.ru);
-  const float2 Lv = f2(C.lv, C.cv.x), Rv = f2(C.cv.y, C.rv);
-  const float2 dtu = fsub2(Ru, Lu), dtv = fsub2(Rv, Lv);  // 2 D^T
-  const float2 hsv = fadd2(Lv, Rv);                       // F^T
-  float2 Hu, Hv;
+__device__ __forceinline__ void lf_row(LfRow& R, float2 a, float2 b, const LfGeom& G) {
+  R.c[1] = a;
+  R.c[2] = b;
+  R.c[0].x = __shfl_up_sync(0xffffffffu, b.x, 1);
+  R.c[0].y = __shfl_up_sync(0xffffffffu, b.y, 1);
+  R.c[3].x = __shfl_down_sync(0xffffffffu, a.x, 1);
+  R.c[3].y = __shfl_down_sync(0xffffffffu, a.y, 1);
   if (EDGE) {
-    const bool T = gy == 0, B = gy == S.H - 1;
-    const bool L0 = S.gx0 == 0, R0 = S.gx0 == S.W - 1, L1 = S.gx0 + 1 == 0, R1 = S.gx0 + 1 == S.W - 1;
-    Hu = lbf_hsum_edge(U, C, D, T, B, L0, R0, L1, R1, false);
-    Hv = lbf_hsum_edge(U, C, D, T, B, L0, R0, L1, R1, true);
-  } else {
-    const float2 vso_u = fadd2(f2(U.lu, U.ru), f2(D.lu, D.ru));
-    const float2 vso_v = fadd2(f2(U.lv, U.rv), f2(D.lv, D.rv));
-    Hu = fadd2(fadd2(vso_u, f2s(__fadd_rn(vsu.x, vsu.y))), fadd2(Lu, Ru));
-    Hv = fadd2(fadd2(vso_v, f2s(__fadd_rn(vsv.x, vsv.y))), hsv);
+    if (G.gx0 == 0) R.c[0] = R.c[1];
+    if (G.gx0 == G.W - 1) R.c[2] = R.c[1];
+    if (G.gx0 >= G.W - 2) R.c[3] = R.c[2];
   }
-  const float2 a2 = fmul2(IIx, f2s(0.5f)), a3 = fmul2(IIy, f2s(0.5f)), a5 = fmul2(II, f2s(0.25f));
-  const float2 h2 = f2s(S.h);
-  // bu = 2 IIx D u + IIx D^T v + IIy D v + II F u + II M v + h H u + Ixt
-  float2 bu = *reinterpret_cast<const float2*>(sc + 3 * LB_PL + o);
-  bu = ffma2(h2, Hu, bu);
-  bu = ffma2(a5, mdv, bu);
-  bu = ffma2(II, vsu, bu);
-  bu = ffma2(a3, vdv, bu);
-  bu = ffma2(a2, dtv, bu);
-  bu = ffma2(IIx, vdu, bu);
-  // bv = IIy D u + IIx D^T u + 2 IIy D^T v + II M u + II F^T v + h H v + Iyt
-  float2 bv = *reinterpret_cast<const float2*>(sc + 4 * LB_PL + o);
-  bv = ffma2(h2, Hv, bv);
-  bv = ffma2(a5, mdu, bv);
-  bv = ffma2(II, hsv, bv);
-  bv = ffma2(IIy, dtv, bv);
-  bv = ffma2(a2, dtu, bv);
-  bv = ffma2(a3, vdu, bv);
-  const float2 B11 = *reinterpret_cast<const float2*>(sc + 5 * LB_PL + o);
-  const float2 B12 = *reinterpret_cast<const float2*>(sc + 6 * LB_PL + o);
-  const float2 B22 = *reinterpret_cast<const float2*>(sc + 7 * LB_PL + o);
-  const float2 m1 = f2s(-1.0f);
-  const float2 nu = fmul2(ffma2(B11, bu, fmul2(B12, bv)), m1);
-  const float2 nv = fmul2(ffma2(B12, bu, fmul2(B22, bv)), m1);
-  const bool in0 = S.gx0 < S.W, in1 = S.gx0 + 1 < S.W;
-  if (S.ou) {
-    __syncwarp();  // in place: every lane has read this row (as its window's next row) already
-    *reinterpret_cast<float2*>(&S.ou[row][S.c0]) = nu;
-    *reinterpret_cast<float2*>(&S.ov[row][S.c0]) = nv;
-  } else if (own_row && S.own_col) {
-    const size_t gi = (size_t)row * S.pitch;
-    if (in1) {
-      *reinterpret_cast<float2*>(S.gu + gi) = nu;
-      *reinterpret_cast<float2*>(S.gv + gi) = nv;
-    } else if (in0) {
-      S.gu[gi] = nu.x;
-      S.gv[gi] = nv.x;
+}
+
+// 8-neighbour sum of cell k of the window with out-of-image neighbours as 0 (H's 'constant' border)
+__device__ __forceinline__ float2 lf_hsum_edge(const LfRow& U, const LfRow& C, const LfRow& D, int k, bool T, bool B,
+                                               bool L, bool R) {
+  const float2 z = make_float2(0.f, 0.f);
+  float2 h = (T || L) ? z : U.c[k - 1];
+  h = fadd2(h, T ? z : U.c[k]);
+  h = fadd2(h, (T || R) ? z : U.c[k + 1]);
+  h = fadd2(h, L ? z : C.c[k - 1]);
+  h = fadd2(h, R ? z : C.c[k + 1]);
+  h = fadd2(h, (B || L) ? z : D.c[k - 1]);
+  h = fadd2(h, B ? z : D.c[k]);
+  return fadd2(h, (B || R) ? z : D.c[k + 1]);
+}
+
+// The update of the block's row j from the old window rows U (above), C and D (below); the
+// squared changes of the cells for which `own` holds go to acc.
+template <bool EDGE>
+__device__ __forceinline__ void lf_update(LfBlock& K, int j, const LfRow& U, const LfRow& C, const LfRow& D,
+                                          const LfGeom& G, bool own, float2& acc) {
+  float2 vd[4], vs[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    vd[k] = fsub2(D.c[k], U.c[k]);
+    vs[k] = fadd2(U.c[k], D.c[k]);
+  }
+  const float2 mid = fadd2(vs[1], vs[2]), h2 = make_float2(G.h, G.h);
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int k = i + 1;
+    const float2 md = fsub2(vd[k + 1], vd[k - 1]);      // 4 M
+    const float2 dt = fsub2(C.c[k + 1], C.c[k - 1]);    // 2 D^T
+    const float2 hs = fadd2(C.c[k - 1], C.c[k + 1]);    // F^T
+    float2 Hs;
+    if (EDGE) {
+      const int gy = G.gy0 + j, gx = G.gx0 + i;
+      Hs = lf_hsum_edge(U, C, D, k, gy == 0, gy == G.H - 1, gx == 0, gx == G.W - 1);
+    } else {
+      Hs = fadd2(fadd2(vs[3 * i], mid), hs);
     }
-  }
-  if (own_row && S.own_col) {
-    const float2 eu = fsub2(nu, C.cu), ev = fsub2(nv, C.cv);
-    const float eu0 = in0 ? eu.x : 0.0f, ev0 = in0 ? ev.x : 0.0f;
-    const float eu1 = in1 ? eu.y : 0.0f, ev1 = in1 ? ev.y : 0.0f;
-    acc_u = __fmaf_rn(eu0, eu0, __fmaf_rn(eu1, eu1, acc_u));
-    acc_v = __fmaf_rn(ev0, ev0, __fmaf_rn(ev1, ev1, acc_v));
+    const float iix = K.iixy[j][i].x, iiy = K.iixy[j][i].y, ii = K.ii[j][i];
+    const float a2 = __fmul_rn(iix, 0.5f), a3 = __fmul_rn(iiy, 0.5f), a5 = __fmul_rn(ii, 0.25f);
+    // bu = 2 IIx D u + IIx D^T v + IIy D v + II F u + II M v + h H u + Ixt
+    // bv = IIy D u + IIx D^T u + 2 IIy D^T v + II M u + II F^T v + h H v + Iyt
+    const float2 b = ffma2(h2, Hs, K.ixyt[j][i]);
+    float bu = __fmaf_rn(a5, md.y, b.x), bv = __fmaf_rn(a5, md.x, b.y);
+    bu = __fmaf_rn(ii, vs[k].x, bu);
+    bv = __fmaf_rn(ii, hs.y, bv);
+    bu = __fmaf_rn(a3, vd[k].y, bu);
+    bv = __fmaf_rn(iiy, dt.y, bv);
+    bu = __fmaf_rn(a2, dt.y, bu);
+    bv = __fmaf_rn(a2, dt.x, bv);
+    bu = __fmaf_rn(iix, vd[k].x, bu);
+    bv = __fmaf_rn(a3, vd[k].x, bv);
+    const float2 b1 = K.b1[j][i];
+    float2 n;
+    n.x = __fmaf_rn(b1.x, bu, __fmul_rn(b1.y, bv));
+    n.y = __fmaf_rn(b1.y, bu, __fmul_rn(K.b22[j][i], bv));
+    n = __fmul2_rn(n, make_float2(-1.f, -1.f));
+    if (own && (!EDGE || G.gx0 + i < G.W)) {
+      const float2 e = fsub2(n, C.c[k]);
+      acc = ffma2(e, e, acc);
+    }
+    K.w[j][i] = n;
   }
 }
 
-// The old values a band needs from outside it, read before any warp of the CTA writes the
-// sweep's results in place: the row above the band and its first row (the window's start)
-// and the row below it.
+// One sweep of the block; buf: the blocks' first and last rows before it.  Rows beyond the image
+// take the nearest row's value (EDGE); cells outside the image or on the region's rim get
+// values that no exact cell reads.
 template <bool EDGE>
-__device__ __forceinline__ void lbf_edges(LbRowF& A, LbRowF& B, LbRowF& E, const LbPlane* su, const LbPlane* sv,
-                                          const LbCols& cols, int r0, int n, int rlo, int rhi) {
-  lbf_load<EDGE>(A, su, sv, EDGE ? clampi(r0 - 1, rlo, rhi) : r0 - 1, cols);
-  lbf_load<EDGE>(B, su, sv, r0, cols);
-  lbf_load<EDGE>(E, su, sv, EDGE ? clampi(r0 + n, rlo, rhi) : r0 + n, cols);
+__device__ __forceinline__ void lf_sweep(LfBlock& K, const float4* buf, int warp, int lane, const LfGeom& G,
+                                         bool own_col, float2& acc) {
+  LfRow w[3];
+  {
+    const float4 t = buf[((warp > 0 ? warp - 1 : 0) * 2 + 1) * 32 + lane];
+    lf_row<EDGE>(w[0], make_float2(t.x, t.y), make_float2(t.z, t.w), G);
+  }
+  lf_row<EDGE>(w[1], K.w[0][0], K.w[0][1], G);
+#pragma unroll
+  for (int j = 0; j < LF_BY; j++) {
+    LfRow &U = w[j % 3], &C = w[(j + 1) % 3], &D = w[(j + 2) % 3];
+    if (j + 1 < LF_BY) {
+      lf_row<EDGE>(D, K.w[j + 1][0], K.w[j + 1][1], G);
+    } else {
+      const float4 t = buf[(warp < LF_NW - 1 ? warp + 1 : warp) * 2 * 32 + lane];
+      lf_row<EDGE>(D, make_float2(t.x, t.y), make_float2(t.z, t.w), G);
+    }
+    if (EDGE && G.gy0 + j == 0) U = C;
+    if (EDGE && G.gy0 + j == G.H - 1) D = C;
+    const int r = G.r0 + j;
+    lf_update<EDGE>(K, j, U, C, D, G, own_col && r >= LB_T && r < LB_T + LB_TH && (!EDGE || G.gy0 + j < G.H), acc);
+  }
 }
 
-// One float32 sweep of a lane's band, rows [r0, r0 + n), in place: the window starts from
-// A, B (lbf_edges) and takes E for the row below the band; every other row is read from
-// shared memory before this warp overwrites it (the rows of the band belong to this warp).
+// The sweeps of a pass; chg: each thread's squared changes per sweep.  Unrolled by two, so that
+// the blocks' cells change registers without copies.
 template <bool EDGE>
-__device__ __forceinline__ void lbf_strip(const LbPlane* su, const LbPlane* sv, const LbStrip& S, const LbCols& cols,
-                                          int r0, int n, int rlo, int rhi, LbRowF& A, LbRowF& B, const LbRowF& E,
-                                          double& acc_u, double& acc_v) {
-  LbRowF C;
-  float au = 0.f, av = 0.f;
-  const int rend = r0 + n;
-#define LB_OWN(row) ((row) >= LB_T && (row) < LB_T + LB_TH)
-#define LB_NEXT(X, r)                                                     \
-  do {                                                                    \
-    if ((r) == rend)                                                      \
-      X = E;                                                              \
-    else                                                                  \
-      lbf_load<EDGE>(X, su, sv, EDGE ? clampi((r), rlo, rhi) : (r), cols); \
-  } while (0)
+__device__ __forceinline__ void lf_sweeps(LfBlock& K, float4 (*buf)[LF_BUF], float2 (*chg)[LF_NT], int warp, int lane,
+                                          const LfGeom& G, bool own_col, int nsw) {
+  auto one = [&](int s, float4* cur) {
+    float4* b = cur + warp * 2 * 32 + lane;
+    b[0] = make_float4(K.w[0][0].x, K.w[0][0].y, K.w[0][1].x, K.w[0][1].y);
+    b[32] = make_float4(K.w[LF_BY - 1][0].x, K.w[LF_BY - 1][0].y, K.w[LF_BY - 1][1].x, K.w[LF_BY - 1][1].y);
+    __syncthreads();
+    float2 acc = make_float2(0.f, 0.f);
+    // a warp whose rows this and later sweeps do not need sits out
+    if (G.r0 + LF_BY > 1 + s && G.r0 < LB_RH - 1 - s) lf_sweep<EDGE>(K, cur, warp, lane, G, own_col, acc);
+    chg[s][warp * 32 + lane] = acc;
+  };
 #pragma unroll 1
-  for (int r = 0; r < n; r += 3) {
-    const int row = r0 + r;
-    LB_NEXT(C, row + 1);
-    lbf_pair<EDGE>(A, B, C, S, row, S.gy0 + r, LB_OWN(row), au, av);
-    if (r + 1 < n) {
-      LB_NEXT(A, row + 2);
-      lbf_pair<EDGE>(B, C, A, S, row + 1, S.gy0 + r + 1, LB_OWN(row + 1), au, av);
-    }
-    if (r + 2 < n) {
-      LB_NEXT(B, row + 3);
-      lbf_pair<EDGE>(C, A, B, S, row + 2, S.gy0 + r + 2, LB_OWN(row + 2), au, av);
-    }
+  for (int s = 0; s < nsw; s += 2) {
+    one(s, buf[0]);
+    if (s + 1 < nsw) one(s + 1, buf[1]);
   }
-#undef LB_NEXT
-#undef LB_OWN
-  acc_u += (double)au;
-  acc_v += (double)av;
 }
 
-template <bool FAST, int NW>
-__global__ void __launch_bounds__(32 * NW, (FAST && NW == 6) ? 3 : 2) ls_pass_kernel(const __grid_constant__ CUtensorMap tm_coef,
+// Staged tile of the float32 pass: the 8 coefficient planes, u and v over the region's rows
+// rounded up to whole blocks (zeros outside the image), as the TMA delivers them.
+constexpr int LF_RH = LF_NW * LF_BY, LF_PL = LB_RW * LF_RH;  // floats per plane
+constexpr int LF_COEF_BYTES = 8 * LF_PL * 4, LF_UV_BYTES = 2 * LF_PL * 4;
+static_assert((LF_PL * 4) % 128 == 0, "TMA destinations");
+constexpr size_t LF_SMEM = LF_COEF_BYTES + LF_UV_BYTES + 128;
+
+// The block's cells and coefficients from the staged tile.
+__device__ __forceinline__ void lf_fill(LfBlock& K, const float* st, const LfGeom& G) {
+  const float* p = st + G.r0 * LB_RW + G.c0;
+#pragma unroll
+  for (int j = 0; j < LF_BY; j++) {
+    float2 t[10];
+#pragma unroll
+    for (int k = 0; k < 10; k++) t[k] = *reinterpret_cast<const float2*>(p + k * LF_PL + j * LB_RW);
+    K.iixy[j][0] = make_float2(t[0].x, t[1].x);
+    K.iixy[j][1] = make_float2(t[0].y, t[1].y);
+    K.ii[j][0] = t[2].x;
+    K.ii[j][1] = t[2].y;
+    K.ixyt[j][0] = make_float2(t[3].x, t[4].x);
+    K.ixyt[j][1] = make_float2(t[3].y, t[4].y);
+    K.b1[j][0] = make_float2(t[5].x, t[6].x);
+    K.b1[j][1] = make_float2(t[5].y, t[6].y);
+    K.b22[j][0] = t[7].x;
+    K.b22[j][1] = t[7].y;
+    K.w[j][0] = make_float2(t[8].x, t[9].x);
+    K.w[j][1] = make_float2(t[8].y, t[9].y);
+  }
+}
+
+// What a pass needs of the solve (both arithmetics).
+struct LsPassArgs {
+  const float* coef;   // 8 planes
+  float *ub0, *vb0, *ub1, *vb1;
+  size_t plane;
+  int H, W, pitch;
+  float h;
+  LsCtrl* ctrl;
+  double* ss;
+  int* run;
+  unsigned int* done;
+  int* redo;
+  double inv_n, tol;
+};
+
+// Which sweeps a launch runs.  Pass p reads ping-pong buffer p & 1 and writes the other.  A pass
+// that the stop rule cancelled (and the launch after the last pass) instead rolls the previous
+// pass back when that pass ran past its stopping sweep: it recomputes it from the same input
+// with the sweep count the stop rule chose (redo[p - 1]) and keeps no error sums.
+__device__ __forceinline__ bool ls_pass_plan(const LbPass& P, const LsPassArgs& A, int& k0, int& nsw, int& pass,
+                                             bool& rollback) {
+  k0 = P.k0;
+  nsw = P.nsweep;
+  pass = P.pass;
+  rollback = false;
+  if (P.last || (k0 > 0 && *(volatile int*)(A.run + k0) == 0)) {
+    const int r = pass > 0 ? *(volatile int*)(A.redo + pass - 1) : 0;
+    if (r == 0) return false;
+    rollback = true;
+    pass -= 1;
+    k0 -= LB_T;
+    nsw = r;
+  }
+  return true;
+}
+
+// Per-sweep squared changes of the CTA -> ss[k0 + s]; the last CTA applies the stop rule.
+// Called by a whole warp: lane 2 s + c handles sum c of sweep s, so that the adds, and the last
+// CTA's reads, are one memory round trip each instead of a chain of them (a pass of a small
+// image takes little longer than that).  red[s][c][warp]: the warps' sums.
+template <int NW>
+__device__ __forceinline__ void ls_pass_end(const LsPassArgs& A, const double (*red)[2][NW], int k0, int nsw, int pass) {
+  const int lane = threadIdx.x & 31, s = lane >> 1, c = lane & 1;
+  const bool on = s < nsw;
+  double* const sum = A.ss + 2 * (k0 + s) + c;
+  if (on) {
+    double a = 0.0;
+    for (int w = 0; w < NW; w++) a += red[s][c][w];
+    atomicAdd(sum, a);
+    __threadfence();
+  }
+  __syncwarp();
+  unsigned int before = 0;
+  if (lane == 0) before = atomicAdd(A.done + pass, 1u);
+  if (__shfl_sync(0xffffffffu, before, 0) != gridDim.x * gridDim.y - 1) return;
+  __threadfence();
+  const double v = on ? atomicAdd(sum, 0.0) : 0.0;
+  const double r = sqrt(v), other = __shfl_xor_sync(0xffffffffu, r, 1);
+  const unsigned stops = __ballot_sync(0xffffffffu, on && c == 0 && !((r + other) * A.inv_n > A.tol));
+  if (lane == 0) {
+    if (stops == 0) {
+      A.run[k0 + nsw] = 1;
+      A.ctrl->K = k0 + nsw;
+    } else {
+      const int stop = (__ffs(stops) - 1) >> 1;
+      A.run[k0 + nsw] = 0;
+      A.ctrl->K = k0 + stop + 1;
+      A.redo[pass] = (stop < nsw - 1) ? stop + 1 : 0;
+    }
+    A.ctrl->final_buf = (pass & 1) ^ 1;
+  }
+}
+
+// Passes after the first are launched as programmatic dependents of the previous pass: every
+// CTA lets the next pass be scheduled at once, so its CTAs take the SM slots this pass's tail
+// frees and fetch their coefficients (which do not change during a solve);
+// griddepcontrol.wait then holds them until the previous pass has completed and its memory (u,
+// v and the stop-rule flags) is visible.  Launched without the attribute, both instructions
+// have no effect.
+//
+// The float32 pass: CTAs that stay for the launch, at most two per SM, each taking every
+// gridDim-th tile.  A tile's planes are copied to registers as soon as they have landed, so
+// that the next tile's copies run during this one's sweeps.
+//
+// What bounds it: issue slots (about 60 instructions per cell update, a fifth of them moves
+// that form register pairs) and the barriers between sweeps, at 16 warps per SM (128
+// registers); DRAM moves 2 TB/s.  A 60-sweep solve against the pass that kept coefficients and
+// field in shared memory: 256 x 256 0.286 -> 0.219 ms, 512 x 512 0.353 -> 0.292, 1024 x 1024
+// 0.582 -> 0.537, 2048 x 2048 1.71 -> 1.47.  Tried: coefficients by plain loads without staying
+// CTAs (10 % faster up to 512 x 512, 10 % slower at 2048 x 2048), scalar arithmetic (as fast),
+// one CTA per SM without spills (slower).
+__global__ void __launch_bounds__(LF_NT, 2) ls_fast_kernel(const __grid_constant__ CUtensorMap tm_coef,
+                                                           const __grid_constant__ CUtensorMap tm_u0,
+                                                           const __grid_constant__ CUtensorMap tm_v0,
+                                                           const __grid_constant__ CUtensorMap tm_u1,
+                                                           const __grid_constant__ CUtensorMap tm_v1,
+                                                           const LsPassArgs A, const LbPass P, int tiles_x, int tiles,
+                                                           int* err_flag) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  extern __shared__ __align__(128) unsigned char lf_raw[];
+  float* const st = reinterpret_cast<float*>(lf_raw + ((128 - (smem_u32(lf_raw) & 127)) & 127));
+  __shared__ float4 buf[2][LF_BUF];
+  __shared__ float2 chg[LB_T][LF_NT];  // every thread's squared changes of a tile, per sweep
+  __shared__ double red[LB_T][2][1];
+  __shared__ uint64_t bar[2];  // coefficients; u, v
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  LfGeom G;
+  G.r0 = warp * LF_BY;
+  G.c0 = 2 * lane;
+  G.H = A.H;
+  G.W = A.W;
+  G.h = A.h;
+  const bool own_col = G.c0 >= LB_T && G.c0 < LB_T + LB_TW;
+  if (tid == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+  }
+  __syncthreads();
+  // image position of a tile's region cell (0, 0).  The columns are rotated from row to row: the
+  // grid may be a multiple of the tiles per row, and no CTA should get border tiles only
+  auto place = [&](int tile, int& x, int& y) {
+    const int r = tile / tiles_x;
+    x = ((tile - r * tiles_x + 5 * r) % tiles_x) * LB_TW - LB_T;
+    y = r * LB_TH - LB_T;
+  };
+  auto load_coef = [&](int tile) {  // thread 0
+    int x, y;
+    place(tile, x, y);
+    mbar_expect_tx(&bar[0], LF_COEF_BYTES);
+    tma_load_3d(st, &tm_coef, x, y, 0, &bar[0]);
+  };
+  const bool pre = !P.last;  // the launch after the last pass only rolls back: no prefetch
+  if (pre && tid == 0) load_coef(blockIdx.x);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  int k0, nsw, pass;
+  bool rollback;
+  if (!ls_pass_plan(P, A, k0, nsw, pass, rollback)) {
+    if (pre && !mbar_wait(&bar[0], 0, LS_WAIT_LIMIT) && tid == 0) atomicExch(err_flag, 1);  // the prefetch lands
+    return;
+  }
+  const bool in1 = pass & 1;  // pass p reads buffer p & 1
+  float* const un = in1 ? A.ub0 : A.ub1;
+  float* const vn = in1 ? A.vb0 : A.vb1;
+  auto load_uv = [&](int tile) {  // thread 0
+    int x, y;
+    place(tile, x, y);
+    mbar_expect_tx(&bar[1], LF_UV_BYTES);
+    tma_load_2d(st + 8 * LF_PL, in1 ? &tm_u1 : &tm_u0, x, y, &bar[1]);
+    tma_load_2d(st + 9 * LF_PL, in1 ? &tm_v1 : &tm_v0, x, y, &bar[1]);
+  };
+  if (tid == 0) {
+    if (!pre) load_coef(blockIdx.x);
+    load_uv(blockIdx.x);
+  }
+  double au = 0.0, av = 0.0;  // warp s: the lane's share of sweep s's squared changes
+  uint32_t phase = 0;
+#pragma unroll 1
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, phase ^= 1) {
+    const bool ok_c = mbar_wait(&bar[0], phase, LS_WAIT_LIMIT), ok_uv = mbar_wait(&bar[1], phase, LS_WAIT_LIMIT);
+    if (__syncthreads_or(!ok_c || !ok_uv)) {
+      if (tid == 0) atomicExch(err_flag, 1);
+      if (!ok_c) mbar_wait(&bar[0], phase, LS_WAIT_LIMIT);  // one more bounded wait for the copies in flight
+      if (!ok_uv) mbar_wait(&bar[1], phase, LS_WAIT_LIMIT);
+      break;
+    }
+    int x0, y0;
+    place(tile, x0, y0);
+    G.gy0 = y0 + G.r0;
+    G.gx0 = x0 + G.c0;
+    LfBlock K;
+    lf_fill(K, st, G);
+    __syncthreads();  // the staged tile has been read (and the last tile's changes summed)
+    if (tid == 0 && tile + (int)gridDim.x < tiles) {
+      load_coef(tile + gridDim.x);
+      load_uv(tile + gridDim.x);
+    }
+    if (y0 < 0 || x0 < 0 || y0 + LB_RH > A.H || x0 + LB_RW > A.W)
+      lf_sweeps<true>(K, buf, chg, warp, lane, G, own_col, nsw);
+    else
+      lf_sweeps<false>(K, buf, chg, warp, lane, G, own_col, nsw);
+    if (own_col && G.gx0 < A.W) {
+#pragma unroll
+      for (int j = 0; j < LF_BY; j++) {
+        const int r = G.r0 + j;
+        if (r >= LB_T && r < LB_T + LB_TH && G.gy0 + j < A.H) {
+          const size_t gi = (size_t)(G.gy0 + j) * A.pitch + G.gx0;
+          *reinterpret_cast<float2*>(un + gi) = make_float2(K.w[j][0].x, K.w[j][1].x);  // the pitch covers a pair
+          *reinterpret_cast<float2*>(vn + gi) = make_float2(K.w[j][0].y, K.w[j][1].y);  // at column W - 1
+        }
+      }
+    }
+    __syncthreads();
+    if (!rollback && warp < nsw)
+      for (int k = lane; k < LF_NT; k += 32) {
+        const float2 e = chg[warp][k];
+        au += (double)e.x;
+        av += (double)e.y;
+      }
+  }
+  if (rollback) return;
+  if (warp < nsw) {
+    for (int o = 16; o > 0; o >>= 1) {
+      au += __shfl_down_sync(0xffffffffu, au, o);
+      av += __shfl_down_sync(0xffffffffu, av, o);
+    }
+    if (lane == 0) {
+      red[warp][0][0] = au;
+      red[warp][1][0] = av;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) ls_pass_end<1>(A, red, k0, nsw, pass);
+}
+
+// The float64-sum pass (OF_LS_EXACT), launched like the float32 one.
+template <int NW>
+__global__ void __launch_bounds__(32 * NW, 2) ls_pass_kernel(const __grid_constant__ CUtensorMap tm_coef,
                                                          const __grid_constant__ CUtensorMap tm_u0,
                                                          const __grid_constant__ CUtensorMap tm_v0,
                                                          const __grid_constant__ CUtensorMap tm_u1,
                                                          const __grid_constant__ CUtensorMap tm_v1,
-                                                         float* ub0, float* vb0, float* ub1, float* vb1, int H, int W,
-                                                         int pitch, float h, LbPass P, LsCtrl* ctrl, double* ss,
-                                                         int* run, unsigned int* done, int* redo, double inv_n,
-                                                         double tol, int* err_flag, float one) {
-  // Passes after the first are launched as programmatic dependents of the previous pass:
-  // every CTA lets the next pass be scheduled at once, so its CTAs take the SM slots this
-  // pass's tail frees and prefetch their coefficient tile (the coefficients do not change
-  // during a solve); griddepcontrol.wait then holds them until the previous pass has
-  // completed and its memory (u, v and the stop-rule flags) is visible.  Launched without
-  // the attribute, both instructions have no effect.
+                                                         const LsPassArgs A, const LbPass P, int* err_flag, float one) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ __align__(128) unsigned char lb_smem_raw[];
   unsigned char* base = lb_smem_raw + ((128 - (smem_u32(lb_smem_raw) & 127)) & 127);
@@ -697,9 +916,10 @@ __global__ void __launch_bounds__(32 * NW, (FAST && NW == 6) ? 3 : 2) ls_pass_ke
   // ping-pong buffer q: u at base + COEF + 2q planes, v right after it
 #define LB_U(q) reinterpret_cast<LbPlane*>(base + LB_COEF_BYTES + (2 * (q)) * LB_PLANE)
 #define LB_V(q) reinterpret_cast<LbPlane*>(base + LB_COEF_BYTES + (2 * (q) + 1) * LB_PLANE)
-  // the barriers follow the (u, v) buffers: 2 planes in place (float32 pass), else 4
-  uint64_t* bar = reinterpret_cast<uint64_t*>(base + LB_COEF_BYTES + (FAST ? 2 : 4) * LB_PLANE);  // coefficients
-  uint64_t* bar2 = bar + 1;                                                           // u, v
+  // the barriers follow the (u, v) buffers
+  uint64_t* bar = reinterpret_cast<uint64_t*>(base + LB_COEF_BYTES + 4 * LB_PLANE);  // coefficients
+  uint64_t* bar2 = bar + 1;                                                          // u, v
+  const int H = A.H, W = A.W, pitch = A.pitch;
   const int x0 = blockIdx.x * LB_TW, y0 = blockIdx.y * LB_TH;
   const int lane = threadIdx.x, warp = threadIdx.y;
   const int t = warp * 32 + lane;
@@ -714,28 +934,17 @@ __global__ void __launch_bounds__(32 * NW, (FAST && NW == 6) ? 3 : 2) ls_pass_ke
     tma_load_3d((void*)sc, &tm_coef, x0 - LB_T, y0 - LB_T + 1, 0, bar);
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  // Pass p reads ping-pong buffer p & 1 and writes the other.  A pass that the stop rule
-  // cancelled (and the launch after the last pass) instead rolls the previous pass back
-  // when that pass ran past its stopping sweep: it recomputes it from the same input with
-  // the sweep count the stop rule chose (redo[p - 1]) and keeps no error sums.
-  int k0 = P.k0, nsw = P.nsweep, pass = P.pass;
-  bool rollback = false;
-  if (P.last || (k0 > 0 && *(volatile int*)(run + k0) == 0)) {
-    const int r = pass > 0 ? *(volatile int*)(redo + pass - 1) : 0;
-    if (r == 0) {
-      if (pre && !mbar_wait(bar, 0, LS_WAIT_LIMIT) && t == 0) atomicExch(err_flag, 1);  // the prefetch lands
-      return;
-    }
-    rollback = true;
-    pass -= 1;
-    k0 -= LB_T;
-    nsw = r;
+  int k0, nsw, pass;
+  bool rollback;
+  if (!ls_pass_plan(P, A, k0, nsw, pass, rollback)) {
+    if (pre && !mbar_wait(bar, 0, LS_WAIT_LIMIT) && t == 0) atomicExch(err_flag, 1);  // the prefetch lands
+    return;
   }
   const int in = pass & 1, out = in ^ 1;
   const CUtensorMap* tm_u = in ? &tm_u1 : &tm_u0;
   const CUtensorMap* tm_v = in ? &tm_v1 : &tm_v0;
-  float* un = out ? ub1 : ub0;
-  float* vn = out ? vb1 : vb0;
+  float* un = out ? A.ub1 : A.ub0;
+  float* vn = out ? A.vb1 : A.vb0;
   if (t == 0) {
     if (!pre) {
       mbar_expect_tx(bar, LB_COEF_BYTES);
@@ -776,15 +985,14 @@ __global__ void __launch_bounds__(32 * NW, (FAST && NW == 6) ? 3 : 2) ls_pass_ke
   S.gx0 = x0 - LB_T + c0;
   S.H = H;
   S.W = W;
-  S.h = h;
+  S.h = A.h;
   S.one = one;
   S.own_col = c0 >= LB_T && c0 < LB_T + LB_TW;
   __shared__ double red[LB_T][2][NW];
   __syncthreads();
 #pragma unroll 1
   for (int s = 0; s < nsw; s++) {
-    // the float32 pass updates buffer 0 in place; the float64-sum pass ping-pongs
-    const int in = FAST ? 0 : s & 1, out = FAST ? 0 : in ^ 1;
+    const int in = s & 1, out = in ^ 1;
     const bool last = s == nsw - 1;
     double au = 0.0, av = 0.0;
     // sweep s computes the rows at least s + 1 from the region's edge (later sweeps read no
@@ -792,16 +1000,6 @@ __global__ void __launch_bounds__(32 * NW, (FAST && NW == 6) ? 3 : 2) ls_pass_ke
     const int lo = max(1 + s, rlo), hi = min(LB_RH - 1 - s, rhi + 1);
     const int n = hi - lo;
     const int ra = lo + (n * warp) / NW, rb = lo + (n * (warp + 1)) / NW;
-    LbRowF A, B, E;
-    if (FAST) {
-      if (rb > ra) {
-        if (edge)
-          lbf_edges<true>(A, B, E, LB_U(0), LB_V(0), cols, ra, rb - ra, rlo, rhi);
-        else
-          lbf_edges<false>(A, B, E, LB_U(0), LB_V(0), cols, ra, rb - ra, rlo, rhi);
-      }
-      if (!last) __syncthreads();  // every band's boundary rows are read before any row is rewritten
-    }
     if (rb > ra) {
       S.su = LB_U(in);
       S.sv = LB_V(in);
@@ -811,17 +1009,10 @@ __global__ void __launch_bounds__(32 * NW, (FAST && NW == 6) ? 3 : 2) ls_pass_ke
       S.gu = un + ((ptrdiff_t)(y0 - LB_T) * pitch + S.gx0);
       S.gv = vn + ((ptrdiff_t)(y0 - LB_T) * pitch + S.gx0);
       S.gy0 = y0 - LB_T + ra;
-      if (FAST) {
-        if (edge)
-          lbf_strip<true>(LB_U(0), LB_V(0), S, cols, ra, rb - ra, rlo, rhi, A, B, E, au, av);
-        else
-          lbf_strip<false>(LB_U(0), LB_V(0), S, cols, ra, rb - ra, rlo, rhi, A, B, E, au, av);
-      } else {
-        if (edge)
-          lb_strip<true>(LB_U(in), LB_V(in), S, cols, ra, rb - ra, rlo, rhi, au, av);
-        else
-          lb_strip<false>(LB_U(in), LB_V(in), S, cols, ra, rb - ra, rlo, rhi, au, av);
-      }
+      if (edge)
+        lb_strip<true>(LB_U(in), LB_V(in), S, cols, ra, rb - ra, rlo, rhi, au, av);
+      else
+        lb_strip<false>(LB_U(in), LB_V(in), S, cols, ra, rb - ra, rlo, rhi, au, av);
     }
     if (!rollback) {
       for (int o = 16; o > 0; o >>= 1) {
@@ -836,39 +1027,7 @@ __global__ void __launch_bounds__(32 * NW, (FAST && NW == 6) ? 3 : 2) ls_pass_ke
     __syncthreads();
   }
   if (rollback) return;
-  // per-sweep squared changes -> ss[k0 + s]; the last CTA applies the stop rule
-  if (t == 0) {
-    for (int s = 0; s < nsw; s++) {
-      double a = 0.0, b = 0.0;
-      for (int w = 0; w < NW; w++) {
-        a += red[s][0][w];
-        b += red[s][1][w];
-      }
-      atomicAdd(ss + 2 * (k0 + s), a);
-      atomicAdd(ss + 2 * (k0 + s) + 1, b);
-    }
-    __threadfence();
-    if (atomicAdd(done + pass, 1u) == gridDim.x * gridDim.y - 1) {
-      __threadfence();
-      int stop = -1;
-      for (int s = 0; s < nsw; s++) {
-        double s0 = atomicAdd(ss + 2 * (k0 + s), 0.0), s1 = atomicAdd(ss + 2 * (k0 + s) + 1, 0.0);
-        if (!((sqrt(s0) + sqrt(s1)) * inv_n > tol)) {
-          stop = s;
-          break;
-        }
-      }
-      if (stop < 0) {
-        run[k0 + nsw] = 1;
-        ctrl->K = k0 + nsw;
-      } else {
-        run[k0 + nsw] = 0;
-        ctrl->K = k0 + stop + 1;
-        redo[pass] = (stop < nsw - 1) ? stop + 1 : 0;
-      }
-      ctrl->final_buf = out;
-    }
-  }
+  if (warp == 0) ls_pass_end<NW>(A, red, k0, nsw, pass);
 }
 
 #undef LB_U
@@ -951,24 +1110,23 @@ extern "C" int of_ls_solve_mode(const float* I0, const float* I1, float* U, floa
   float* ub[2] = {uv, uv + 2 * N};
   float* vb[2] = {uv + N, uv + 3 * N};
   // tensor maps over the whole solve: the 8 coefficient planes (3-D) and the four u / v
-  // planes (2-D), all with the 32 x 72 region box of a pass
+  // planes (2-D), with the region box of a pass
   CUtensorMap tm_coef, tm_u[2], tm_v[2];
   {
     uint64_t d3[3] = {(uint64_t)W, (uint64_t)H, 8}, s3[2] = {(uint64_t)P * 4, (uint64_t)N * 4};
-    uint32_t b3[3] = {LB_RW, LB_CH, 8};  // region rows 1 .. LB_RH - 2
+    uint32_t b3[3] = {LB_RW, (uint32_t)(fast ? LF_RH : LB_CH), 8};  // the float64-sum pass: region rows 1 .. LB_RH - 2
     int rc = tmap_f32(&tm_coef, coef, 3, d3, s3, b3);
     if (rc) return rc;
     uint64_t d2[2] = {(uint64_t)W, (uint64_t)H}, s2[1] = {(uint64_t)P * 4};
-    uint32_t b2[2] = {LB_RW, LB_RH};
+    uint32_t b2[2] = {LB_RW, (uint32_t)(fast ? LF_RH : LB_RH)};
     for (int q = 0; q < 2; q++) {
       if ((rc = tmap_f32(&tm_u[q], ub[q], 2, d2, s2, b2))) return rc;
       if ((rc = tmap_f32(&tm_v[q], vb[q], 2, d2, s2, b2))) return rc;
     }
   }
   {
-    cudaError_t e = OF_SMEM_OPT_IN((ls_pass_kernel<false, LB_WARPS>), lb_smem(false));
-    if (e == cudaSuccess) e = OF_SMEM_OPT_IN((ls_pass_kernel<true, 6>), lb_smem(true));
-    if (e == cudaSuccess) e = OF_SMEM_OPT_IN((ls_pass_kernel<true, 8>), lb_smem(true));
+    cudaError_t e = OF_SMEM_OPT_IN(ls_pass_kernel<LB_WARPS>, LB_SMEM);
+    if (e == cudaSuccess) e = OF_SMEM_OPT_IN(ls_fast_kernel, LF_SMEM);
     if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_ls_solve: %s", cudaGetErrorString(e));
   }
   // control block, flags, counters, redo counts and sums are contiguous: one memset
@@ -981,15 +1139,8 @@ extern "C" int of_ls_solve_mode(const float* I0, const float* I1, float* U, floa
   ls_prep_kernel<<<dim3((W + 31) / 32, (H + 7) / 8), 256, 0, st>>>(I0, I1, pitch, ctrl->maxkey, V, U, coef, N,
                                                                  ub[0], vb[0], H, W, P, h);
   double inv_n = 1.0 / ((double)H * (double)W);
-  // warps per CTA: 6 for the float64 pass (its registers allow 2 CTAs of 6); 6 for the
-  // float32 pass too (96 registers and 75.5 KB of shared memory: 3 CTAs per SM;
-  // OFB_LS_FAST_WARPS=8 selects 8 warps, 2 CTAs per SM)
-  static const int fast_nw = [] {
-    const char* e = getenv("OFB_LS_FAST_WARPS");
-    return (e && atoi(e) == 8) ? 8 : 6;
-  }();
-  const int nw = fast ? fast_nw : LB_WARPS;
-  dim3 pgrd((W + LB_TW - 1) / LB_TW, (H + LB_TH - 1) / LB_TH), pblk(32, nw);
+  dim3 pgrd((W + LB_TW - 1) / LB_TW, (H + LB_TH - 1) / LB_TH);
+  const int tiles = (int)(pgrd.x * pgrd.y);
   long long nl = 3;
   int p = 0, k0 = 0;
   // pass 0 waits for the set-up in stream order; later passes (and the rollback launch)
@@ -997,19 +1148,20 @@ extern "C" int of_ls_solve_mode(const float* I0, const float* I1, float* U, floa
   cudaLaunchAttribute pdl[1];
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl[0].val.programmaticStreamSerializationAllowed = 1;
+  const LsPassArgs A{coef, ub[0], vb[0], ub[1], vb[1], N, H, W, P, h, ctrl, ss, run, done, redo, inv_n, tol};
   auto launch_pass = [&](LbPass PP, bool dependent) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = pgrd;
-    cfg.blockDim = pblk;
-    cfg.dynamicSmemBytes = lb_smem(fast);
+    cfg.gridDim = fast ? dim3(tiles < 2 * kNumSMs ? tiles : 2 * kNumSMs) : pgrd;
+    cfg.blockDim = fast ? dim3(LF_NT) : dim3(32, LB_WARPS);
+    cfg.dynamicSmemBytes = fast ? LF_SMEM : LB_SMEM;
     cfg.stream = st;
     cfg.attrs = dependent ? pdl : nullptr;
     cfg.numAttrs = dependent ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, !fast ? ls_pass_kernel<false, LB_WARPS> : nw == 6 ? ls_pass_kernel<true, 6>
-                                                                               : ls_pass_kernel<true, 8>,
-                              tm_coef, tm_u[0], tm_v[0],
-                              tm_u[1], tm_v[1], ub[0], vb[0], ub[1], vb[1], H, W, P, h, PP, ctrl, ss, run, done, redo,
-                              inv_n, tol, err_flag, 1.0f);
+    if (fast)
+      return cudaLaunchKernelEx(&cfg, ls_fast_kernel, tm_coef, tm_u[0], tm_v[0], tm_u[1], tm_v[1], A, PP, (int)pgrd.x, tiles,
+                                err_flag);
+    return cudaLaunchKernelEx(&cfg, ls_pass_kernel<LB_WARPS>, tm_coef, tm_u[0], tm_v[0], tm_u[1], tm_v[1], A, PP,
+                              err_flag, 1.0f);
   };
   for (; k0 < maxnum; k0 += LB_T, p++) {
     LbPass P0{k0, maxnum - k0 < LB_T ? maxnum - k0 : LB_T, p, 0};
