@@ -361,6 +361,11 @@ int of_warp_liushen_ofe(const float* I, const float* du, const float* dv, float*
 int of_cnn_conv3x3(const void* x, int n, int H, int W, int cin, int x_ctot, int x_coff, const void* w, int cout,
                    const float* bias, int flags, void* y, int y_ctot, int y_coff, int cout_store, unsigned* err,
                    void* stream);
+/* Input gradient with the ReLU of the layer below applied: dx = conv3x3(dy, w) where the
+ * activation `act` (a slice at dx's pixels and channels) is > 0, else 0. */
+int of_cnn_conv3x3_relu_bwd(const void* dy, int n, int H, int W, int cin, int dy_ctot, int dy_coff, const void* w,
+                            int cout, const void* act, int act_ctot, int act_coff, void* dx, int dx_ctot, int dx_coff,
+                            int cout_store, unsigned* err, void* stream);
 /* dw[tap][co][ci] += sum_p dy[p][co] * x[p + tap][ci] on the tensor cores (tcgen05, both
  * operands MN-major from NHWC, f32 accumulate, split over pixel ranges and added with
  * atomics).  W a divisor or a multiple of 64, H likewise for 64 / min(W, 64); cin, cout <= 512. */
@@ -382,6 +387,12 @@ int of_cnn_upsample2(const void* x, int x_ctot, int x_coff, int n, int h, int w,
                      int y_coff, void* stream);
 int of_cnn_upsample2_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int h, int w, int C, void* dx, int dx_ctot,
                          int dx_coff, void* stream);
+/* The two backward passes followed by the mask of of_cnn_relu_bwd on dx, in one pass. */
+int of_cnn_avgpool2_relu_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int H, int W, int C, void* dx,
+                             int dx_ctot, int dx_coff, int accumulate, const void* act, int act_ctot, int act_coff,
+                             void* stream);
+int of_cnn_upsample2_relu_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int h, int w, int C, void* dx,
+                              int dx_ctot, int dx_coff, const void* act, int act_ctot, int act_coff, void* stream);
 /* g *= (y > 0) over P pixels x C channels. */
 int of_cnn_relu_bwd(void* g, int g_ctot, int g_coff, const void* y, int y_ctot, int y_coff, long long P, int C,
                     void* stream);
@@ -395,6 +406,9 @@ int of_cnn_adam(float* w, const float* g, float* m, float* v, long long n, float
  * the input-gradient operand [9][cin_pad][cout_pad] with the taps mirrored. */
 int of_cnn_pack_weights(const float* w, int cout, int cin, int cout_pad, int cin_pad, int transpose_flip, void* out,
                         void* stream);
+/* of_cnn_pack_weights of up to 64 layers in one launch; host arrays w[count], out[count] and
+ * dims[count][5] = cout, cin, cout_pad, cin_pad, transpose_flip (pads at most 4096). */
+int of_cnn_pack_weights_many(int count, const float* const* w, const int* dims, void* const* out, void* stream);
 /* (h, w, 2) interleaved f32 flow -> U, V planes at (factor h, factor w) (row pitch
  * `pitch`): bilinear, pixel-centre aligned, edges clamped, displacements times `scale`. */
 int of_cnn_flow_up(const float* flow, int h, int w, int factor, float* U, float* V, int pitch, float scale,

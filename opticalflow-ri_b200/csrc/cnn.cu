@@ -11,13 +11,16 @@
 //                   warps 2-5 read TMEM back (one pixel per thread) and apply bias, ReLU
 //                   and the bf16 / f32 store, into a channel slice of a wider tensor when
 //                   the output feeds a concatenation.  The same kernel computes the input
-//                   gradient (transposed, flipped weights).
+//                   gradient
+//                   (transposed, flipped weights), with the mask of the ReLU below it in the
+//                   epilogue.
 //  of_cnn_conv3x3_wgrad  weight gradient (CUDA cores, f32 FMA over bf16 operands).
 //  pooling, nearest upsampling, ReLU masks, loss, Adam and weight packing: elementwise.
 //
 // Every wait on an mbarrier is bounded by time (about one second); a CTA that gives up
 // sets a bit in the caller's error word, waits (bounded) for its copies in flight and
 // for its MMAs, frees its TMEM and exits.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -25,6 +28,7 @@
 
 namespace ofb {
 
+namespace cg = cooperative_groups;
 typedef __nv_bfloat16 bf16;
 
 constexpr int CV_M = 128;
@@ -41,6 +45,8 @@ struct ConvParams {
   const float* bias;
   void* y;
   int y_ctot, y_coff;
+  const bf16* act;  // ReLU backward in the epilogue: the output is 0 where this activation is not > 0
+  int act_ctot, act_coff;
   unsigned* err;
   uint32_t a_bytes, b_bytes, stage_bytes, tmem_cols;
 };
@@ -111,8 +117,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ float2 bf2f(unsigned int u) {
+  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+__device__ __forceinline__ unsigned int f2bf(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const unsigned int*>(&h);
+}
+// Two bf16 gradients g where the two activations y are > 0, else +0.
+__device__ __forceinline__ unsigned int relu_mask(unsigned int g, unsigned int y) {
+  const float2 a = bf2f(y);
+  return (a.x > 0.f ? g & 0xffffu : 0u) | (a.y > 0.f ? g & 0xffff0000u : 0u);
+}
+__device__ __forceinline__ uint4 relu_mask8(uint4 g, uint4 y) {
+  return make_uint4(relu_mask(g.x, y.x), relu_mask(g.y, y.y), relu_mask(g.z, y.z), relu_mask(g.w, y.w));
+}
+
 // TMEM accumulator row (this thread's pixel) -> bias, ReLU, bf16 / f32 store of the N tile
-// starting at channel n0.  taddr: the warp's TMEM lane quarter, column 0.
+// starting at channel n0.  With p.act the gradient is masked before its store, which replaces
+// a pass that read it and the activation and wrote it again.  taddr: the warp's TMEM lane quarter, column 0.
 __device__ __forceinline__ void cv_epilogue(const ConvParams& p, uint32_t taddr, size_t pix, int n0) {
   for (int c = 0; c < p.bn; c += 16) {
     uint32_t r[16];
@@ -142,12 +165,19 @@ __device__ __forceinline__ void cv_epilogue(const ConvParams& p, uint32_t taddr,
           __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
           w[j] = *reinterpret_cast<uint32_t*>(&h2);
         }
-        reinterpret_cast<uint4*>(yo)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        reinterpret_cast<uint4*>(yo)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        uint4 lo = make_uint4(w[0], w[1], w[2], w[3]), hi = make_uint4(w[4], w[5], w[6], w[7]);
+        if (p.act) {
+          const uint4* ao = reinterpret_cast<const uint4*>(p.act + pix * p.act_ctot + p.act_coff + co);
+          lo = relu_mask8(lo, ao[0]);
+          hi = relu_mask8(hi, ao[1]);
+        }
+        reinterpret_cast<uint4*>(yo)[0] = lo;
+        reinterpret_cast<uint4*>(yo)[1] = hi;
       } else {
+        const bf16* ao = p.act ? p.act + pix * p.act_ctot + p.act_coff + co : nullptr;
 #pragma unroll
         for (int j = 0; j < 16; j++)
-          if (j < nvalid) yo[j] = __float2bfloat16_rn(v[j]);
+          if (j < nvalid) yo[j] = __float2bfloat16_rn(ao && !(__bfloat162float(ao[j]) > 0.f) ? 0.f : v[j]);
       }
     }
   }
@@ -474,6 +504,52 @@ __global__ void bias_grad_kernel(const bf16* __restrict__ dY, int dct, int dco, 
   if (c < cout) atomicAdd(&db[c], s);
 }
 
+// The same sum, 8 channels (16 bytes) per thread: the scalar kernel is bound by the latency of
+// one 2-byte load per pixel and thread (the 12 layers of a training step of 16 crops of
+// 128 x 128: 146 us, 40 us here).  A CTA of 256 threads holds 256 / (channel groups) pixels at a time and four loads in flight per
+// thread, adds the pixel rows in shared memory and issues one atomic per channel.
+// A last group that is not full reads, and drops, channels of the same pixel.
+constexpr int BG_THREADS = 256;
+__global__ void __launch_bounds__(BG_THREADS) bias_grad_v8_kernel(const bf16* __restrict__ dY, int dct, int dco,
+                                                                  long long P, int cout, float* __restrict__ db) {
+  __shared__ float part[BG_THREADS][9];
+  const int c8 = (cout + 7) / 8, rows = BG_THREADS / c8;
+  const int row = threadIdx.x / c8, grp = threadIdx.x - row * c8;
+  float s[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) s[k] = 0.f;
+  if (row < rows) {
+    const bf16* src = dY + dco + 8 * grp;
+    const long long step = (long long)gridDim.x * rows;
+    long long p = (long long)blockIdx.x * rows + row;
+    auto add = [&](const uint4& q) {
+      const unsigned int u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const float2 v = bf2f(u[k]);
+        s[2 * k] = __fadd_rn(s[2 * k], v.x);
+        s[2 * k + 1] = __fadd_rn(s[2 * k + 1], v.y);
+      }
+    };
+    for (; p + 3 * step < P; p += 4 * step) {
+      uint4 q[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) q[j] = *reinterpret_cast<const uint4*>(src + (p + j * step) * dct);
+#pragma unroll
+      for (int j = 0; j < 4; j++) add(q[j]);
+    }
+    for (; p < P; p += step) add(*reinterpret_cast<const uint4*>(src + p * dct));
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k++) part[threadIdx.x][k] = s[k];
+  __syncthreads();
+  for (int c = threadIdx.x; c < cout; c += BG_THREADS) {
+    float t = 0.f;
+    for (int r = 0; r < rows; r++) t = __fadd_rn(t, part[r * c8 + (c >> 3)][c & 7]);
+    atomicAdd(&db[c], t);
+  }
+}
+
 // ----------------------------------------------------------------------------- elementwise
 // out[img][y][x][0..cpad) = (I0 / max I0, I1 / max I1, 0, ...)  in bf16; max over the frame
 __global__ void frame_max_kernel(const float* __restrict__ I, int H, int W, int pitch, unsigned* __restrict__ mx) {
@@ -514,18 +590,26 @@ __global__ void pack_pair_kernel(const float* __restrict__ I0, const float* __re
   pack_store(out + (size_t)e * cpad, cpad, a, b);
 }
 
-// Both maxima and the packing in one CTA, for the small frames the network runs on (up to
-// 64 K pixels): the maxima are the same (max is exact and order-free, NaN-free through
-// fmaxf as in frame_max_kernel) and the packing is pack_pair_kernel's per pixel.
-constexpr int PK1_THREADS = 1024;
-__global__ void __launch_bounds__(PK1_THREADS) pack_pair_one_kernel(const float* __restrict__ I0,
-                                                                     const float* __restrict__ I1, int H, int W,
-                                                                     int pitch, unsigned* __restrict__ mx,
-                                                                     bf16* __restrict__ out, int cpad) {
-  __shared__ float r0[32], r1[32];
-  const int n = H * W;
+// Both maxima and the packing in one cluster of 8 CTAs, for the small frames the network runs
+// on (up to 64 K pixels): each CTA reduces an eighth of the pixels, the CTAs exchange their
+// two maxima through distributed shared memory, and each packs its own eighth (which its L1
+// still holds).  One CTA alone is bound by its own load latency: 28.5 us for a 128 x 128 pair,
+// 8.3 us here; three launches (the path for larger frames) wait for each other.  The maxima are the same
+// (max is exact and order-free, NaN-free through fmaxf as in frame_max_kernel) and the packing
+// is pack_pair_kernel's per pixel.
+constexpr int PKC_CTAS = 8, PKC_THREADS = 512, PKC_PIX = 65536;
+__global__ void __cluster_dims__(PKC_CTAS, 1, 1) __launch_bounds__(PKC_THREADS)
+    pack_pair_cluster_kernel(const float* __restrict__ I0, const float* __restrict__ I1, int H, int W, int pitch,
+                             unsigned* __restrict__ mx, bf16* __restrict__ out, int cpad) {
+  __shared__ float r0[PKC_THREADS / 32], r1[PKC_THREADS / 32];
+  __shared__ float2 all[PKC_CTAS];
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank();
+  const int n = H * W, per = (n + PKC_CTAS - 1) / PKC_CTAS;
+  const int e0 = rank * per, e1 = e0 + per < n ? e0 + per : n;
   float m0 = 0.f, m1 = 0.f;
-  for (int e = threadIdx.x; e < n; e += PK1_THREADS) {
+#pragma unroll 4
+  for (int e = e0 + (int)threadIdx.x; e < e1; e += PKC_THREADS) {
     const int y = e / W, x = e - y * W;
     m0 = fmaxf(m0, I0[(size_t)y * pitch + x]);
     m1 = fmaxf(m1, I1[(size_t)y * pitch + x]);
@@ -538,18 +622,30 @@ __global__ void __launch_bounds__(PK1_THREADS) pack_pair_one_kernel(const float*
     r0[threadIdx.x >> 5] = m0;
     r1[threadIdx.x >> 5] = m1;
   }
-  __syncthreads();
-  m0 = r0[0];
-  m1 = r1[0];
-  for (int w = 1; w < PK1_THREADS / 32; w++) {
-    m0 = fmaxf(m0, r0[w]);
-    m1 = fmaxf(m1, r1[w]);
+  cl.sync();  // this CTA's partial maxima, and every CTA of the cluster runs
+  if (threadIdx.x < PKC_CTAS) {
+    m0 = r0[0];
+    m1 = r1[0];
+    for (int w = 1; w < PKC_THREADS / 32; w++) {
+      m0 = fmaxf(m0, r0[w]);
+      m1 = fmaxf(m1, r1[w]);
+    }
+    *cl.map_shared_rank(&all[rank], threadIdx.x) = make_float2(m0, m1);
   }
-  if (threadIdx.x == 0) {
+  cl.sync();  // no remote access after this one: a CTA may exit
+  m0 = all[0].x;
+  m1 = all[0].y;
+#pragma unroll
+  for (int r = 1; r < PKC_CTAS; r++) {
+    m0 = fmaxf(m0, all[r].x);
+    m1 = fmaxf(m1, all[r].y);
+  }
+  if (rank == 0 && threadIdx.x == 0) {
     mx[0] = __float_as_uint(m0);
     mx[1] = __float_as_uint(m1);
   }
-  for (int e = threadIdx.x; e < n; e += PK1_THREADS) {
+#pragma unroll 4
+  for (int e = e0 + (int)threadIdx.x; e < e1; e += PKC_THREADS) {
     const int y = e / W, x = e - y * W;
     const float a = m0 > 0.f ? __fdiv_rn(I0[(size_t)y * pitch + x], m0) : 0.f;
     const float b = m1 > 0.f ? __fdiv_rn(I1[(size_t)y * pitch + x], m1) : 0.f;
@@ -575,14 +671,6 @@ __global__ void avgpool2_kernel(const bf16* __restrict__ x, int xct, int xco, in
 // (image * rows + row) and 32-bit index arithmetic: used when the channel counts, channel
 // offsets and row strides are multiples of 8 and the bases 16-byte aligned (every layer of
 // the network).  Per channel the arithmetic is the scalar kernels'.
-__device__ __forceinline__ float2 bf2f(unsigned int u) {
-  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
-}
-__device__ __forceinline__ unsigned int f2bf(float a, float b) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const unsigned int*>(&h);
-}
-
 __global__ void avgpool2_v8_kernel(const bf16* __restrict__ x, int xct, int xco, int H, int W, int C,
                                    bf16* __restrict__ y, int yct, int yco) {
   const int h = H / 2, w = W / 2, c8 = C / 8;
@@ -625,7 +713,8 @@ static bool v8_ok(const void* x, int xct, int xco, const void* y, int yct, int y
 
 // dx (fine) = dy (coarse parent) / 4, added to dx when accumulate
 __global__ void avgpool2_bwd_kernel(const bf16* __restrict__ dy, int dct, int dco, int n, int H, int W, int C,
-                                    bf16* __restrict__ dx, int xct, int xco, int accumulate) {
+                                    bf16* __restrict__ dx, int xct, int xco, int accumulate,
+                                    const bf16* __restrict__ act, int act_ct, int act_co) {
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (long long)n * H * W * C) return;
   int c = (int)(e % C);
@@ -635,6 +724,7 @@ __global__ void avgpool2_bwd_kernel(const bf16* __restrict__ dy, int dct, int dc
   float g = __fmul_rn(__bfloat162float(dy[(((size_t)img * h + yy / 2) * w + xx / 2) * dct + dco + c]), 0.25f);
   bf16* o = dx + (((size_t)img * H + yy) * W + xx) * xct + xco + c;
   if (accumulate) g = __fadd_rn(g, __bfloat162float(*o));
+  if (act && !(__bfloat162float(act[(((size_t)img * H + yy) * W + xx) * act_ct + act_co + c]) > 0.f)) g = 0.f;
   *o = __float2bfloat16_rn(g);
 }
 
@@ -651,7 +741,8 @@ __global__ void upsample2_kernel(const bf16* __restrict__ x, int xct, int xco, i
 }
 
 __global__ void upsample2_bwd_kernel(const bf16* __restrict__ dy, int dct, int dco, int n, int h, int w, int C,
-                                     bf16* __restrict__ dx, int xct, int xco) {
+                                     bf16* __restrict__ dx, int xct, int xco, const bf16* __restrict__ act, int act_ct,
+                                     int act_co) {
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (long long)n * h * w * C) return;
   int c = (int)(e % C);
@@ -661,7 +752,88 @@ __global__ void upsample2_bwd_kernel(const bf16* __restrict__ dy, int dct, int d
   const bf16* b = dy + (((size_t)img * H + 2 * oy) * W + 2 * ox) * dct + dco + c;
   float s = __fadd_rn(__fadd_rn(__bfloat162float(b[0]), __bfloat162float(b[dct])),
                       __fadd_rn(__bfloat162float(b[(size_t)W * dct]), __bfloat162float(b[(size_t)W * dct + dct])));
+  if (act && !(__bfloat162float(act[(((size_t)img * h + oy) * w + ox) * act_ct + act_co + c]) > 0.f)) s = 0.f;
   dx[(((size_t)img * h + oy) * w + ox) * xct + xco + c] = __float2bfloat16_rn(s);
+}
+
+// The backward passes on 8 channels per thread, under the rule of the forward ones and with
+// the same arithmetic per channel.  They should be bound by memory; one element per thread was
+// bound by its 64-bit index arithmetic.  The mask of the ReLU whose output was pooled or
+// upsampled goes in before the store.  The three poolings of a training step of 16 crops of
+// 128 x 128: 111 us and their masks before, 26 us with the masks now; the three upsamplings
+// 60 us and masks before, 17 us now; all eleven masks were 167 us.
+__global__ void avgpool2_bwd_v8_kernel(const bf16* __restrict__ dy, int dct, int dco, int H, int W, int C,
+                                       bf16* __restrict__ dx, int xct, int xco, int accumulate,
+                                       const bf16* __restrict__ act, int act_ct, int act_co) {
+  // one thread: 2 x 2 outputs of one input
+  const int h = H / 2, w = W / 2, c8 = C / 8;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= w * c8) return;
+  const int ox = t / c8, c = 8 * (t - ox * c8);
+  const int img = blockIdx.y / h, oy = blockIdx.y - img * h;
+  const size_t pix = ((size_t)img * H + 2 * oy) * W + 2 * ox;
+  const uint4 q = *reinterpret_cast<const uint4*>(dy + (((size_t)img * h + oy) * w + ox) * dct + dco + c);
+  const unsigned int u[4] = {q.x, q.y, q.z, q.w};
+  float2 g[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const float2 v = bf2f(u[k]);
+    g[k] = make_float2(__fmul_rn(v.x, 0.25f), __fmul_rn(v.y, 0.25f));
+  }
+  uint4 old[4], a[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const size_t o = pix + (size_t)(j >> 1) * W + (j & 1);
+    if (accumulate) old[j] = *reinterpret_cast<const uint4*>(dx + o * xct + xco + c);
+    if (act) a[j] = *reinterpret_cast<const uint4*>(act + o * act_ct + act_co + c);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const size_t o = pix + (size_t)(j >> 1) * W + (j & 1);
+    unsigned int r[4];
+    const unsigned int d[4] = {old[j].x, old[j].y, old[j].z, old[j].w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      float2 v = g[k];
+      if (accumulate) {
+        const float2 e = bf2f(d[k]);
+        v = make_float2(__fadd_rn(v.x, e.x), __fadd_rn(v.y, e.y));
+      }
+      r[k] = f2bf(v.x, v.y);
+    }
+    uint4 out = make_uint4(r[0], r[1], r[2], r[3]);
+    if (act) out = relu_mask8(out, a[j]);
+    *reinterpret_cast<uint4*>(dx + o * xct + xco + c) = out;
+  }
+}
+
+__global__ void upsample2_bwd_v8_kernel(const bf16* __restrict__ dy, int dct, int dco, int h, int w, int C,
+                                        bf16* __restrict__ dx, int xct, int xco, const bf16* __restrict__ act,
+                                        int act_ct, int act_co) {
+  const int H = 2 * h, W = 2 * w, c8 = C / 8;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= w * c8) return;
+  const int ox = t / c8, c = 8 * (t - ox * c8);
+  const int img = blockIdx.y / h, oy = blockIdx.y - img * h;
+  const bf16* b = dy + (((size_t)img * H + 2 * oy) * W + 2 * ox) * dct + dco + c;
+  const size_t o = ((size_t)img * h + oy) * w + ox;
+  const uint4 p0 = *reinterpret_cast<const uint4*>(b), p1 = *reinterpret_cast<const uint4*>(b + dct);
+  const uint4 p2 = *reinterpret_cast<const uint4*>(b + (size_t)W * dct);
+  const uint4 p3 = *reinterpret_cast<const uint4*>(b + (size_t)W * dct + dct);
+  uint4 a = make_uint4(0u, 0u, 0u, 0u);
+  if (act) a = *reinterpret_cast<const uint4*>(act + o * act_ct + act_co + c);
+  const unsigned int a0[4] = {p0.x, p0.y, p0.z, p0.w}, a1[4] = {p1.x, p1.y, p1.z, p1.w};
+  const unsigned int a2[4] = {p2.x, p2.y, p2.z, p2.w}, a3[4] = {p3.x, p3.y, p3.z, p3.w};
+  unsigned int r[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const float2 v0 = bf2f(a0[k]), v1 = bf2f(a1[k]), v2 = bf2f(a2[k]), v3 = bf2f(a3[k]);
+    r[k] = f2bf(__fadd_rn(__fadd_rn(v0.x, v1.x), __fadd_rn(v2.x, v3.x)),
+                __fadd_rn(__fadd_rn(v0.y, v1.y), __fadd_rn(v2.y, v3.y)));
+  }
+  uint4 out = make_uint4(r[0], r[1], r[2], r[3]);
+  if (act) out = relu_mask8(out, a);
+  *reinterpret_cast<uint4*>(dx + o * xct + xco + c) = out;
 }
 
 // g = g * (y > 0) over a channel slice (the ReLU derivative from the layer's output)
@@ -676,7 +848,20 @@ __global__ void relu_bwd_kernel(bf16* __restrict__ g, int gct, int gco, const bf
 
 // mean squared flow error: loss += sum (pred - label)^2 / (2 P);  dpred = (pred - label) / P
 // (bf16, padded to gct channels, the padding zeroed)
-__global__ void flow_mse_kernel(const float* __restrict__ pred, const float* __restrict__ label, long long P,
+__global__ void relu_bwd_v8_kernel(bf16* __restrict__ g, int gct, int gco, const bf16* __restrict__ y, int yct, int yco,
+                                   long long P, int C) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int c8 = C / 8;
+  const long long p = e / c8;
+  if (p >= P) return;
+  const int c = 8 * (int)(e - p * c8);
+  uint4* o = reinterpret_cast<uint4*>(g + p * gct + gco + c);
+  *o = relu_mask8(*o, *reinterpret_cast<const uint4*>(y + p * yct + yco + c));
+}
+
+// One pixel per thread; the CTA adds its warps' sums in double and issues one atomic (one per
+// warp serialised on the loss's address: 16 x 128 x 128 pixels 25.4 us, 4.8 us here).
+__global__ void __launch_bounds__(256) flow_mse_kernel(const float* __restrict__ pred, const float* __restrict__ label, long long P,
                                 bf16* __restrict__ dpred, int gct, double* __restrict__ loss) {
   long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   float l = 0.f;
@@ -685,14 +870,18 @@ __global__ void flow_mse_kernel(const float* __restrict__ pred, const float* __r
     float du = __fadd_rn(pred[2 * p], -label[2 * p]), dv = __fadd_rn(pred[2 * p + 1], -label[2 * p + 1]);
     l = __fadd_rn(__fmul_rn(du, du), __fmul_rn(dv, dv));
     if (dpred) {
-      bf16* o = dpred + p * gct;
-      o[0] = __float2bfloat16_rn(__fmul_rn(du, inv));
-      o[1] = __float2bfloat16_rn(__fmul_rn(dv, inv));
-      for (int c = 2; c < gct; c++) o[c] = __float2bfloat16_rn(0.f);
+      pack_store(dpred + p * gct, gct, __fmul_rn(du, inv), __fmul_rn(dv, inv));
     }
   }
   for (int o = 16; o; o >>= 1) l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, o));
-  if ((threadIdx.x & 31) == 0 && p - (threadIdx.x & 31) < P) atomicAdd(loss, (double)l / (2.0 * (double)P));
+  __shared__ double part[8];
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = (double)l / (2.0 * (double)P);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = part[0];
+    for (int w = 1; w < 8; w++) t += part[w];
+    atomicAdd(loss, t);
+  }
 }
 
 __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
@@ -725,6 +914,27 @@ __global__ void pack_weights_kernel(const float* __restrict__ w, int cout, int c
   int k = transpose_flip ? 8 - tap : tap;
   float v = (co < cout && ci < cin) ? w[((size_t)k * cout + co) * cin + ci] : 0.f;
   out[e] = __float2bfloat16_rn(v);
+}
+
+// Every layer's operands in one launch: 23 launches of 2.5 us each (57 us, and more than that
+// on the host) against 14.6 us.  blockIdx.y picks the entry, the CTAs of a row walk it.
+constexpr int PW_MAX = 64;
+struct PackMany {
+  const float* w[PW_MAX];
+  bf16* out[PW_MAX];
+  short cout[PW_MAX], cin[PW_MAX], cout_pad[PW_MAX], cin_pad[PW_MAX], flip[PW_MAX];
+};
+__global__ void pack_weights_many_kernel(const __grid_constant__ PackMany p) {
+  const int i = blockIdx.y;
+  const int cp = p.cout_pad[i], ip = p.cin_pad[i], cout = p.cout[i], cin = p.cin[i], flip = p.flip[i];
+  const int per = cp * ip, cols = flip ? cp : ip;
+  const float* w = p.w[i];
+  bf16* out = p.out[i];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 9 * per; e += gridDim.x * blockDim.x) {
+    const int tap = e / per, r = e - tap * per, row = r / cols, col = r - row * cols;
+    const int co = flip ? col : row, ci = flip ? row : col, k = flip ? 8 - tap : tap;
+    out[e] = __float2bfloat16_rn(co < cout && ci < cin ? w[((size_t)k * cout + co) * cin + ci] : 0.f);
+  }
 }
 
 // (h, w, 2) interleaved f32 flow -> two planes with row pitch `pitch`
@@ -768,9 +978,9 @@ static int blocks_for(long long n, int t = 256) { return (int)((n + t - 1) / t);
 
 using namespace ofb;
 
-extern "C" int of_cnn_conv3x3(const void* x, int n, int H, int W, int cin, int x_ctot, int x_coff, const void* w,
-                              int cout, const float* bias, int flags, void* y, int y_ctot, int y_coff, int cout_store,
-                              unsigned* err, void* stream) {
+static int conv3x3(const void* x, int n, int H, int W, int cin, int x_ctot, int x_coff, const void* w, int cout,
+                   const float* bias, int flags, void* y, int y_ctot, int y_coff, int cout_store, const void* act,
+                   int act_ctot, int act_coff, unsigned* err, void* stream) {
   OF_REQUIRE(x && w && y && err && n > 0 && H > 0 && W > 0, "of_cnn_conv3x3: bad arguments");
   int ck = cin % 64 == 0 ? 64 : (cin % 32 == 0 ? 32 : (cin == 16 ? 16 : 0));
   OF_REQUIRE(ck, "of_cnn_conv3x3: input channels %d (need 16, a multiple of 32)", cin);
@@ -823,6 +1033,9 @@ extern "C" int of_cnn_conv3x3(const void* x, int n, int H, int W, int cin, int x
   p.y = y;
   p.y_ctot = y_ctot;
   p.y_coff = y_coff;
+  p.act = static_cast<const bf16*>(act);
+  p.act_ctot = act_ctot;
+  p.act_coff = act_coff;
   p.err = err;
   p.a_bytes = (uint32_t)(CV_M * ck * 2);
   p.b_bytes = (uint32_t)(bn * ck * 2);
@@ -843,6 +1056,23 @@ extern "C" int of_cnn_conv3x3(const void* x, int n, int H, int W, int cin, int x
   return check_launch("of_cnn_conv3x3");
 }
 
+extern "C" int of_cnn_conv3x3(const void* x, int n, int H, int W, int cin, int x_ctot, int x_coff, const void* w,
+                              int cout, const float* bias, int flags, void* y, int y_ctot, int y_coff, int cout_store,
+                              unsigned* err, void* stream) {
+  return conv3x3(x, n, H, W, cin, x_ctot, x_coff, w, cout, bias, flags, y, y_ctot, y_coff, cout_store, nullptr, 0, 0, err,
+                 stream);
+}
+
+extern "C" int of_cnn_conv3x3_relu_bwd(const void* dy, int n, int H, int W, int cin, int dy_ctot, int dy_coff,
+                                       const void* w, int cout, const void* act, int act_ctot, int act_coff, void* dx,
+                                       int dx_ctot, int dx_coff, int cout_store, unsigned* err, void* stream) {
+  OF_REQUIRE(act && act_ctot % 8 == 0 && act_coff % 8 == 0 && act_coff >= 0 && cout_store > 0 &&
+                 act_coff + cout_store <= act_ctot && ((uintptr_t)act & 15) == 0,
+             "of_cnn_conv3x3_relu_bwd: activation channel slice");
+  return conv3x3(dy, n, H, W, cin, dy_ctot, dy_coff, w, cout, nullptr, 0, dx, dx_ctot, dx_coff, cout_store, act, act_ctot,
+                 act_coff, err, stream);
+}
+
 extern "C" int of_cnn_conv3x3_wgrad(const void* x, int x_ctot, int x_coff, const void* dy, int dy_ctot, int dy_coff,
                                     int n, int H, int W, int cin, int cout, float* dw, void* stream) {
   OF_REQUIRE(x && dy && dw && n > 0 && H > 0 && W > 0 && cin > 0 && cout > 0, "of_cnn_conv3x3_wgrad: bad arguments");
@@ -858,6 +1088,15 @@ extern "C" int of_cnn_conv3x3_wgrad(const void* x, int x_ctot, int x_coff, const
 extern "C" int of_cnn_bias_grad(const void* dy, int dy_ctot, int dy_coff, long long P, int cout, float* db,
                                 void* stream) {
   OF_REQUIRE(dy && db && P > 0 && cout > 0 && cout <= 1024, "of_cnn_bias_grad: bad arguments");
+  if (dy_ctot % 8 == 0 && dy_coff % 8 == 0 && dy_coff + (cout + 7) / 8 * 8 <= dy_ctot && ((uintptr_t)dy & 15) == 0) {
+    const int rows = BG_THREADS / ((cout + 7) / 8);
+    // two CTAs per SM, fewer where a CTA would see less than 4 rounds of pixels
+    long long g = (P + 4LL * rows - 1) / (4LL * rows);
+    if (g > 2 * kNumSMs) g = 2 * kNumSMs;
+    bias_grad_v8_kernel<<<(int)g, BG_THREADS, 0, as_stream(stream)>>>(static_cast<const bf16*>(dy), dy_ctot, dy_coff, P,
+                                                                      cout, db);
+    return check_launch("of_cnn_bias_grad");
+  }
   int t = (cout + 31) / 32 * 32;
   int g = (int)(P < 2LL * kNumSMs * 8 ? P : 2LL * kNumSMs * 8);
   bias_grad_kernel<<<g, t, 0, as_stream(stream)>>>(static_cast<const bf16*>(dy), dy_ctot, dy_coff, P, cout, db);
@@ -868,8 +1107,8 @@ extern "C" int of_cnn_pack_pair(const float* I0, const float* I1, int H, int W, 
                                 int cpad, void* stream) {
   OF_REQUIRE(I0 && I1 && max2 && out && H > 0 && W > 0 && pitch >= W && cpad >= 2, "of_cnn_pack_pair: bad arguments");
   cudaStream_t st = as_stream(stream);
-  if ((long long)H * W <= 65536) {
-    pack_pair_one_kernel<<<1, PK1_THREADS, 0, st>>>(I0, I1, H, W, pitch, max2, static_cast<bf16*>(out), cpad);
+  if ((long long)H * W <= PKC_PIX) {
+    pack_pair_cluster_kernel<<<PKC_CTAS, PKC_THREADS, 0, st>>>(I0, I1, H, W, pitch, max2, static_cast<bf16*>(out), cpad);
     return check_launch("of_cnn_pack_pair");
   }
   cudaMemsetAsync(max2, 0, 2 * sizeof(unsigned), st);
@@ -895,13 +1134,33 @@ extern "C" int of_cnn_avgpool2(const void* x, int x_ctot, int x_coff, int n, int
   return check_launch("of_cnn_avgpool2");
 }
 
+static int avgpool2_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int H, int W, int C, void* dx, int dx_ctot,
+                        int dx_coff, int accumulate, const void* act, int act_ctot, int act_coff, void* stream) {
+  OF_REQUIRE(dy && dx && H % 2 == 0 && W % 2 == 0 && C > 0, "of_cnn_avgpool2_bwd: bad arguments");
+  const bf16 *d = static_cast<const bf16*>(dy), *a = static_cast<const bf16*>(act);
+  if (v8_ok(dy, dy_ctot, dy_coff, dx, dx_ctot, dx_coff, C) && (!act || v8_ok(act, act_ctot, act_coff, dx, 0, 0, C)) &&
+      (long long)n * (H / 2) <= 65535) {
+    avgpool2_bwd_v8_kernel<<<dim3(blocks_for((long long)(W / 2) * (C / 8)), n * (H / 2)), 256, 0, as_stream(stream)>>>(
+        d, dy_ctot, dy_coff, H, W, C, static_cast<bf16*>(dx), dx_ctot, dx_coff, accumulate, a, act_ctot, act_coff);
+    return check_launch("of_cnn_avgpool2_bwd");
+  }
+  long long tot = (long long)n * H * W * C;
+  avgpool2_bwd_kernel<<<blocks_for(tot), 256, 0, as_stream(stream)>>>(d, dy_ctot, dy_coff, n, H, W, C,
+                                                                       static_cast<bf16*>(dx), dx_ctot, dx_coff,
+                                                                       accumulate, a, act_ctot, act_coff);
+  return check_launch("of_cnn_avgpool2_bwd");
+}
+
 extern "C" int of_cnn_avgpool2_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int H, int W, int C, void* dx,
                                    int dx_ctot, int dx_coff, int accumulate, void* stream) {
-  OF_REQUIRE(dy && dx && H % 2 == 0 && W % 2 == 0 && C > 0, "of_cnn_avgpool2_bwd: bad arguments");
-  long long tot = (long long)n * H * W * C;
-  avgpool2_bwd_kernel<<<blocks_for(tot), 256, 0, as_stream(stream)>>>(
-      static_cast<const bf16*>(dy), dy_ctot, dy_coff, n, H, W, C, static_cast<bf16*>(dx), dx_ctot, dx_coff, accumulate);
-  return check_launch("of_cnn_avgpool2_bwd");
+  return avgpool2_bwd(dy, dy_ctot, dy_coff, n, H, W, C, dx, dx_ctot, dx_coff, accumulate, nullptr, 0, 0, stream);
+}
+
+extern "C" int of_cnn_avgpool2_relu_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int H, int W, int C, void* dx,
+                                        int dx_ctot, int dx_coff, int accumulate, const void* act, int act_ctot,
+                                        int act_coff, void* stream) {
+  OF_REQUIRE(act, "of_cnn_avgpool2_relu_bwd: bad arguments");
+  return avgpool2_bwd(dy, dy_ctot, dy_coff, n, H, W, C, dx, dx_ctot, dx_coff, accumulate, act, act_ctot, act_coff, stream);
 }
 
 extern "C" int of_cnn_upsample2(const void* x, int x_ctot, int x_coff, int n, int h, int w, int C, void* y, int y_ctot,
@@ -918,18 +1177,42 @@ extern "C" int of_cnn_upsample2(const void* x, int x_ctot, int x_coff, int n, in
   return check_launch("of_cnn_upsample2");
 }
 
-extern "C" int of_cnn_upsample2_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int h, int w, int C, void* dx,
-                                    int dx_ctot, int dx_coff, void* stream) {
+static int upsample2_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int h, int w, int C, void* dx, int dx_ctot,
+                         int dx_coff, const void* act, int act_ctot, int act_coff, void* stream) {
   OF_REQUIRE(dy && dx && h > 0 && w > 0 && C > 0, "of_cnn_upsample2_bwd: bad arguments");
+  const bf16 *d = static_cast<const bf16*>(dy), *a = static_cast<const bf16*>(act);
+  if (v8_ok(dy, dy_ctot, dy_coff, dx, dx_ctot, dx_coff, C) && (!act || v8_ok(act, act_ctot, act_coff, dx, 0, 0, C)) &&
+      (long long)n * h <= 65535) {
+    upsample2_bwd_v8_kernel<<<dim3(blocks_for((long long)w * (C / 8)), n * h), 256, 0, as_stream(stream)>>>(
+        d, dy_ctot, dy_coff, h, w, C, static_cast<bf16*>(dx), dx_ctot, dx_coff, a, act_ctot, act_coff);
+    return check_launch("of_cnn_upsample2_bwd");
+  }
   long long tot = (long long)n * h * w * C;
   upsample2_bwd_kernel<<<blocks_for(tot), 256, 0, as_stream(stream)>>>(
-      static_cast<const bf16*>(dy), dy_ctot, dy_coff, n, h, w, C, static_cast<bf16*>(dx), dx_ctot, dx_coff);
+      d, dy_ctot, dy_coff, n, h, w, C, static_cast<bf16*>(dx), dx_ctot, dx_coff, a, act_ctot, act_coff);
   return check_launch("of_cnn_upsample2_bwd");
+}
+
+extern "C" int of_cnn_upsample2_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int h, int w, int C, void* dx,
+                                    int dx_ctot, int dx_coff, void* stream) {
+  return upsample2_bwd(dy, dy_ctot, dy_coff, n, h, w, C, dx, dx_ctot, dx_coff, nullptr, 0, 0, stream);
+}
+
+extern "C" int of_cnn_upsample2_relu_bwd(const void* dy, int dy_ctot, int dy_coff, int n, int h, int w, int C, void* dx,
+                                         int dx_ctot, int dx_coff, const void* act, int act_ctot, int act_coff,
+                                         void* stream) {
+  OF_REQUIRE(act, "of_cnn_upsample2_relu_bwd: bad arguments");
+  return upsample2_bwd(dy, dy_ctot, dy_coff, n, h, w, C, dx, dx_ctot, dx_coff, act, act_ctot, act_coff, stream);
 }
 
 extern "C" int of_cnn_relu_bwd(void* g, int g_ctot, int g_coff, const void* y, int y_ctot, int y_coff, long long P,
                                int C, void* stream) {
   OF_REQUIRE(g && y && P > 0 && C > 0, "of_cnn_relu_bwd: bad arguments");
+  if (v8_ok(g, g_ctot, g_coff, y, y_ctot, y_coff, C)) {
+    relu_bwd_v8_kernel<<<blocks_for(P * (C / 8)), 256, 0, as_stream(stream)>>>(
+        static_cast<bf16*>(g), g_ctot, g_coff, static_cast<const bf16*>(y), y_ctot, y_coff, P, C);
+    return check_launch("of_cnn_relu_bwd");
+  }
   relu_bwd_kernel<<<blocks_for(P * C), 256, 0, as_stream(stream)>>>(static_cast<bf16*>(g), g_ctot, g_coff,
                                                                      static_cast<const bf16*>(y), y_ctot, y_coff, P, C);
   return check_launch("of_cnn_relu_bwd");
@@ -958,6 +1241,30 @@ extern "C" int of_cnn_pack_weights(const float* w, int cout, int cin, int cout_p
   pack_weights_kernel<<<blocks_for(tot), 256, 0, as_stream(stream)>>>(w, cout, cin, cout_pad, cin_pad, transpose_flip,
                                                                        static_cast<bf16*>(out));
   return check_launch("of_cnn_pack_weights");
+}
+
+extern "C" int of_cnn_pack_weights_many(int count, const float* const* w, const int* dims, void* const* out,
+                                        void* stream) {
+  OF_REQUIRE(count > 0 && count <= PW_MAX && w && dims && out, "of_cnn_pack_weights_many: %d entries (1..%d)", count,
+             PW_MAX);
+  PackMany p;
+  int most = 0;
+  for (int i = 0; i < count; i++) {
+    const int *d = dims + 5 * i, cout = d[0], cin = d[1], cp = d[2], ip = d[3];
+    OF_REQUIRE(w[i] && out[i] && cout > 0 && cin > 0 && cp >= cout && ip >= cin && cp <= 4096 && ip <= 4096,
+               "of_cnn_pack_weights_many: entry %d", i);
+    p.w[i] = w[i];
+    p.out[i] = static_cast<bf16*>(out[i]);
+    p.cout[i] = (short)cout;
+    p.cin[i] = (short)cin;
+    p.cout_pad[i] = (short)cp;
+    p.cin_pad[i] = (short)ip;
+    p.flip[i] = d[4] != 0;
+    if (9 * cp * ip > most) most = 9 * cp * ip;
+  }
+  const int g = blocks_for(most) < 2 * kNumSMs ? blocks_for(most) : 2 * kNumSMs;
+  pack_weights_many_kernel<<<dim3(g, count), 256, 0, as_stream(stream)>>>(p);
+  return check_launch("of_cnn_pack_weights_many");
 }
 
 extern "C" int of_cnn_split_flow(const float* flow, int h, int w, float* u, float* v, int pitch, void* stream) {

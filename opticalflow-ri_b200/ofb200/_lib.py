@@ -115,18 +115,22 @@ _SIGS = {
     "of_warp_liushen_scatter": ([_P, _P, _P, _P, _P, _P, _I, _I, _I, _P, _P, _Z, _P], _I),
     "of_warp_liushen_ofe": ([_P, _P, _P, _P, _I, _I, _I, _P], _I),
     "of_cnn_conv3x3": ([_P, _I, _I, _I, _I, _I, _I, _P, _I, _P, _I, _P, _I, _I, _I, _P, _P], _I),
+    "of_cnn_conv3x3_relu_bwd": ([_P, _I, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P, _I, _I, _I, _P, _P], _I),
     "of_cnn_conv3x3_wgrad_tc": ([_P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P], _I),
     "of_cnn_conv3x3_wgrad": ([_P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P], _I),
     "of_cnn_bias_grad": ([_P, _I, _I, _L, _I, _P, _P], _I),
     "of_cnn_pack_pair": ([_P, _P, _I, _I, _I, _P, _P, _I, _P], _I),
     "of_cnn_avgpool2": ([_P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P], _I),
     "of_cnn_avgpool2_bwd": ([_P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _I, _P], _I),
+    "of_cnn_avgpool2_relu_bwd": ([_P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _I, _P, _I, _I, _P], _I),
     "of_cnn_upsample2": ([_P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P], _I),
     "of_cnn_upsample2_bwd": ([_P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P], _I),
+    "of_cnn_upsample2_relu_bwd": ([_P, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P, _I, _I, _P], _I),
     "of_cnn_relu_bwd": ([_P, _I, _I, _P, _I, _I, _L, _I, _P], _I),
     "of_cnn_flow_mse": ([_P, _P, _L, _P, _I, _P, _P], _I),
     "of_cnn_adam": ([_P, _P, _P, _P, _L, _F, _F, _F, _F, _I, _P], _I),
     "of_cnn_pack_weights": ([_P, _I, _I, _I, _I, _I, _P, _P], _I),
+    "of_cnn_pack_weights_many": ([_I, _P, _P, _P, _P], _I),
     "of_cnn_flow_up": ([_P, _I, _I, _I, _P, _P, _I, _F, _P], _I),
     "of_cnn_split_flow": ([_P, _I, _I, _P, _P, _I, _P], _I),
     "of_lk_dense": ([_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P], _I),

@@ -105,12 +105,16 @@ class WarmStartNet:
     # ------------------------------------------------------------------ parameters
     def pack(self):
         """bf16 forward and input-gradient operands from the master weights."""
+        w, dims, out = [], [], []
+        base = self.params.data_ptr()
         for name, ci, co in LAYERS:
-            wo, _, _, _ = self.off[name]
-            w = ctypes.c_void_p(self.params.data_ptr() + 4 * wo)
-            call("of_cnn_pack_weights", w, co, ci, _pad16(co), _cin_pad(ci), 0, _p(self.wf[name]), _sp())
-            if name != "c0a":
-                call("of_cnn_pack_weights", w, co, ci, _pad16(co), _cin_pad(ci), 1, _p(self.wb[name]), _sp())
+            for flip in (0, 1) if name != "c0a" else (0,):
+                w.append(base + 4 * self.off[name][0])
+                dims += (co, ci, _pad16(co), _cin_pad(ci), flip)
+                out.append((self.wb if flip else self.wf)[name].data_ptr())
+        n = len(w)
+        call("of_cnn_pack_weights_many", n, (ctypes.c_void_p * n)(*w), (ctypes.c_int * (5 * n))(*dims),
+             (ctypes.c_void_p * n)(*out), _sp())
 
     def _bias(self, name):
         return ctypes.c_void_p(self.params.data_ptr() + 4 * self.off[name][1])
@@ -245,63 +249,60 @@ class WarmStartNet:
              _p(self.err), _sp())
         call("of_cnn_bias_grad", _p(dy), dct, dco, n * H * W, co, self._gb(name), _sp())
 
-    def _relu_bwd(self, gt, gct, gco, yt, yct, yco, P, C):
-        call("of_cnn_relu_bwd", _p(gt), gct, gco, _p(yt), yct, yco, P, C, _sp())
+    def _dgrad(self, name, dy, dct, dco, cin, n, H, W, dx, act, act_ct, act_co=0):
+        """Input gradient of layer `name` into dx, masked by the ReLU output `act` that the layer read."""
+        ci = self.off[name][2]
+        call("of_cnn_conv3x3_relu_bwd", _p(dy), n, H, W, cin, dct, dco, _p(self.wb[name]), _cin_pad(ci), _p(act), act_ct,
+             act_co, _p(dx), ci, 0, ci, _p(self.err), _sp())
 
     def backward(self, b, g):
         """Gradients of the loss (dout from loss()) into self.grads (zeroed here)."""
         n, S = b["x0"].shape[0], b["x0"].shape[1]
         s1, s2, s3 = S // 2, S // 4, S // 8
-        P0, P1, P2, P3 = n * S * S, n * s1 * s1, n * s2 * s2, n * s3 * s3
         self.grads.zero_()
-        cv, wg, rb = self._conv, self._wgrad, self._relu_bwd
+        cv, wg, dg = self._conv, self._wgrad, self._dgrad
         # head (no ReLU)
         wg("head", b["d0"], 32, 0, g["dout"], 16, 0, n, S, S)
-        cv("head", g["dout"], 16, 0, 16, n, S, S, g["d0"], 32, 0, flags=0, backward=True)
-        rb(g["d0"], 32, 0, b["d0"], 32, 0, P0, 32)
+        dg("head", g["dout"], 16, 0, 16, n, S, S, g["d0"], b["d0"], 32)
         # dec0
         wg("d0", b["cat0"], 96, 0, g["d0"], 32, 0, n, S, S)
         cv("d0", g["d0"], 32, 0, 32, n, S, S, g["cat0"], 96, 0, flags=0, backward=True)
-        call("of_cnn_upsample2_bwd", _p(g["cat0"]), 96, 0, n, s1, s1, 64, _p(g["d1"]), 64, 0, _sp())
-        rb(g["d1"], 64, 0, b["d1"], 64, 0, P1, 64)
+        call("of_cnn_upsample2_relu_bwd", _p(g["cat0"]), 96, 0, n, s1, s1, 64, _p(g["d1"]), 64, 0, _p(b["d1"]), 64,
+             0, _sp())
         # dec1
         wg("d1", b["cat1"], 192, 0, g["d1"], 64, 0, n, s1, s1)
         cv("d1", g["d1"], 64, 0, 64, n, s1, s1, g["cat1"], 192, 0, flags=0, backward=True)
-        call("of_cnn_upsample2_bwd", _p(g["cat1"]), 192, 0, n, s2, s2, 128, _p(g["d2"]), 128, 0, _sp())
-        rb(g["d2"], 128, 0, b["d2"], 128, 0, P2, 128)
+        call("of_cnn_upsample2_relu_bwd", _p(g["cat1"]), 192, 0, n, s2, s2, 128, _p(g["d2"]), 128, 0, _p(b["d2"]), 128,
+             0, _sp())
         # dec2
         wg("d2", b["cat2"], 384, 0, g["d2"], 128, 0, n, s2, s2)
         cv("d2", g["d2"], 128, 0, 128, n, s2, s2, g["cat2"], 384, 0, flags=0, backward=True)
-        call("of_cnn_upsample2_bwd", _p(g["cat2"]), 384, 0, n, s3, s3, 256, _p(g["e3"]), 256, 0, _sp())
-        rb(g["e3"], 256, 0, b["e3"], 256, 0, P3, 256)
+        call("of_cnn_upsample2_relu_bwd", _p(g["cat2"]), 384, 0, n, s3, s3, 256, _p(g["e3"]), 256, 0, _p(b["e3"]), 256,
+             0, _sp())
         # enc3
         wg("c3b", b["a3"], 256, 0, g["e3"], 256, 0, n, s3, s3)
-        cv("c3b", g["e3"], 256, 0, 256, n, s3, s3, g["a3"], 256, 0, flags=0, backward=True)
-        rb(g["a3"], 256, 0, b["a3"], 256, 0, P3, 256)
+        dg("c3b", g["e3"], 256, 0, 256, n, s3, s3, g["a3"], b["a3"], 256)
         wg("c3a", b["p3"], 128, 0, g["a3"], 256, 0, n, s3, s3)
         cv("c3a", g["a3"], 256, 0, 256, n, s3, s3, g["p3"], 128, 0, flags=0, backward=True)
-        call("of_cnn_avgpool2_bwd", _p(g["p3"]), 128, 0, n, s2, s2, 128, _p(g["cat2"]), 384, 256, 1, _sp())
-        rb(g["cat2"], 384, 256, b["cat2"], 384, 256, P2, 128)
+        call("of_cnn_avgpool2_relu_bwd", _p(g["p3"]), 128, 0, n, s2, s2, 128, _p(g["cat2"]), 384, 256, 1, _p(b["cat2"]),
+             384, 256, _sp())
         # enc2
         wg("c2b", b["a2"], 128, 0, g["cat2"], 384, 256, n, s2, s2)
-        cv("c2b", g["cat2"], 384, 256, 128, n, s2, s2, g["a2"], 128, 0, flags=0, backward=True)
-        rb(g["a2"], 128, 0, b["a2"], 128, 0, P2, 128)
+        dg("c2b", g["cat2"], 384, 256, 128, n, s2, s2, g["a2"], b["a2"], 128)
         wg("c2a", b["p2"], 64, 0, g["a2"], 128, 0, n, s2, s2)
         cv("c2a", g["a2"], 128, 0, 128, n, s2, s2, g["p2"], 64, 0, flags=0, backward=True)
-        call("of_cnn_avgpool2_bwd", _p(g["p2"]), 64, 0, n, s1, s1, 64, _p(g["cat1"]), 192, 128, 1, _sp())
-        rb(g["cat1"], 192, 128, b["cat1"], 192, 128, P1, 64)
+        call("of_cnn_avgpool2_relu_bwd", _p(g["p2"]), 64, 0, n, s1, s1, 64, _p(g["cat1"]), 192, 128, 1, _p(b["cat1"]),
+             192, 128, _sp())
         # enc1
         wg("c1b", b["a1"], 64, 0, g["cat1"], 192, 128, n, s1, s1)
-        cv("c1b", g["cat1"], 192, 128, 64, n, s1, s1, g["a1"], 64, 0, flags=0, backward=True)
-        rb(g["a1"], 64, 0, b["a1"], 64, 0, P1, 64)
+        dg("c1b", g["cat1"], 192, 128, 64, n, s1, s1, g["a1"], b["a1"], 64)
         wg("c1a", b["p1"], 32, 0, g["a1"], 64, 0, n, s1, s1)
         cv("c1a", g["a1"], 64, 0, 64, n, s1, s1, g["p1"], 32, 0, flags=0, backward=True)
-        call("of_cnn_avgpool2_bwd", _p(g["p1"]), 32, 0, n, S, S, 32, _p(g["cat0"]), 96, 64, 1, _sp())
-        rb(g["cat0"], 96, 64, b["cat0"], 96, 64, P0, 32)
+        call("of_cnn_avgpool2_relu_bwd", _p(g["p1"]), 32, 0, n, S, S, 32, _p(g["cat0"]), 96, 64, 1, _p(b["cat0"]),
+             96, 64, _sp())
         # enc0
         wg("c0b", b["a0"], 32, 0, g["cat0"], 96, 64, n, S, S)
-        cv("c0b", g["cat0"], 96, 64, 32, n, S, S, g["a0"], 32, 0, flags=0, backward=True)
-        rb(g["a0"], 32, 0, b["a0"], 32, 0, P0, 32)
+        dg("c0b", g["cat0"], 96, 64, 32, n, S, S, g["a0"], b["a0"], 32)
         wg("c0a", b["x0"], IN_CH, 0, g["a0"], 32, 0, n, S, S)
 
     def check(self):
