@@ -11,9 +11,8 @@
 //                   warps 2-5 read TMEM back (one pixel per thread) and apply bias, ReLU
 //                   and the bf16 / f32 store, into a channel slice of a wider tensor when
 //                   the output feeds a concatenation.  The same kernel computes the input
-//                   gradient
-//                   (transposed, flipped weights), with the mask of the ReLU below it in the
-//                   epilogue.
+//                   gradient (transposed, flipped weights), with the mask of the ReLU
+//                   below it in the epilogue.
 //  of_cnn_conv3x3_wgrad  weight gradient (CUDA cores, f32 FMA over bf16 operands).
 //  pooling, nearest upsampling, ReLU masks, loss, Adam and weight packing: elementwise.
 //
@@ -286,10 +285,15 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
 // count.  NHWC keeps the channels contiguous, so both operands are MN-major: a TMA box of
 // 64 channels x 64 pixels lands as 64 rows of 128 B (128-byte swizzle), which is the
 // canonical MN-major layout (8-row groups 1024 B apart, 64-channel atoms 8 KB apart).
-// A is the wider channel side (M = 128, channels past its end are zero-filled by TMA and
-// their rows ignored), B the narrower (N <= 256).  X is shifted by the tap through the box
-// coordinates (zero padding from TMA's out-of-bounds fill).  CTAs split the pixel range;
-// each adds its 128 x N partial sums into dW with atomics.
+// A is the wider channel side (M = 128, channels past its end are ignored rows), B the
+// narrower (N <= 256), shifted by the tap through its box coordinates (zero padding from TMA's
+// out-of-bounds fill): by +tap where B is X, by -tap where B is dY.  A CTA takes `tg` taps (9, 3
+// or 1) of its pixels with one TMEM accumulator each, so that A is loaded once for all of them:
+// with one tap per CTA the kernel is bound by the boxes it loads, 9 x (2 + B's) per 64 pixels.
+// CTAs split the pixel range; each adds its sums into dW with atomics, four input channels at
+// a time where the lanes run over output channels (scalar ones touch a sector each there).
+// The 12 layers of a training step of 16 crops of 128 x 128: 634 us with one tap per CTA and
+// scalar atomics, 407 us here.
 constexpr int WT_KP = 64;  // pixels per K chunk
 constexpr int WT_STAGES = 4;
 
@@ -298,6 +302,7 @@ struct WgParams {
   int chunks_per_cta, mtiles, ntiles;
   int a_is_dy, a_ch, b_ch;   // channel counts of the A and B sides
   int nmma, batoms;          // MMA N and 64-channel atoms loaded for B
+  int tg, cstride, stages;   // taps per CTA, TMEM columns from one tap's accumulator to the next
   int cin, cout;
   float* dw;
   unsigned* err;
@@ -324,12 +329,12 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
   __shared__ volatile int abort_flag;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wg_smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tap = blockIdx.z, mt = blockIdx.y / p.ntiles, nt = blockIdx.y - mt * p.ntiles;
+  const int tap0 = blockIdx.z * p.tg, mt = blockIdx.y / p.ntiles, nt = blockIdx.y - mt * p.ntiles;
   const int m0 = mt * 128, n0 = nt * 256;
   const int c0 = blockIdx.x * p.chunks_per_cta;
   const int c1 = c0 + p.chunks_per_cta < p.nchunk ? c0 + p.chunks_per_cta : p.nchunk;
   const int kiters = c1 > c0 ? c1 - c0 : 0;
-  const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+  const bool atom1 = m0 + 64 < p.a_ch;  // A's second 64 channels; absent, their rows are ignored
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < WT_STAGES; s++) {
@@ -353,9 +358,11 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
   if (warp == 0) {
     if (lane == 0) {
       int issued = 0;
+      const uint32_t bytes = (atom1 ? 2u : 1u) * 8192u + p.tg * p.b_bytes;
+      const int sgn = p.a_is_dy ? 1 : -1;
       for (int it = 0; it < kiters && !abort_flag; it++) {
-        const int s = it % WT_STAGES;
-        if (!cv_wait(&empty[s], ((uint32_t)(it / WT_STAGES) & 1u) ^ 1u, &abort_flag)) {
+        const int s = it % p.stages;
+        if (!cv_wait(&empty[s], ((uint32_t)(it / p.stages) & 1u) ^ 1u, &abort_flag)) {
           atomicOr(p.err, 1u);
           abort_flag = 1;
           break;
@@ -363,35 +370,38 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
         const int ch = c0 + it, grp = ch / p.tiles_per_group, t_in = ch - grp * p.tiles_per_group;
         const int ty = t_in / p.tiles_x, tx = t_in - ty * p.tiles_x;
         const int x0 = tx * p.bw, y0 = ty * p.bh, img0 = grp * p.nb;
-        // the A side is dY (unshifted) or X (shifted), the B side the other
-        const int ax = p.a_is_dy ? x0 : x0 + dx, ay = p.a_is_dy ? y0 : y0 + dy;
-        const int bx = p.a_is_dy ? x0 + dx : x0, by = p.a_is_dy ? y0 + dy : y0;
         uint8_t* a = smem + (size_t)s * p.stage_bytes;
-        mbar_expect_tx(&full[s], p.a_bytes + p.b_bytes);
-        tma_load_4d(a, &tm_a, m0, ax, ay, img0, &full[s]);
-        tma_load_4d(a + 8192, &tm_a, m0 + 64, ax, ay, img0, &full[s]);
-        for (int j = 0; j < p.batoms; j++)
-          tma_load_4d(a + p.a_bytes + j * 8192, &tm_b, n0 + 64 * j, bx, by, img0, &full[s]);
+        mbar_expect_tx(&full[s], bytes);
+        tma_load_4d(a, &tm_a, m0, x0, y0, img0, &full[s]);
+        if (atom1) tma_load_4d(a + 8192, &tm_a, m0 + 64, x0, y0, img0, &full[s]);
+        for (int t = 0; t < p.tg; t++) {
+          const int dy = sgn * ((tap0 + t) / 3 - 1), dx = sgn * ((tap0 + t) % 3 - 1);
+          for (int j = 0; j < p.batoms; j++)
+            tma_load_4d(a + p.a_bytes + t * p.b_bytes + j * 8192, &tm_b, n0 + 64 * j, x0 + dx, y0 + dy, img0, &full[s]);
+        }
         issued = it + 1;
       }
-      for (int it = issued > WT_STAGES ? issued - WT_STAGES : 0; it < issued; it++)
-        if (!cv_wait(&full[it % WT_STAGES], (uint32_t)(it / WT_STAGES) & 1u, nullptr)) atomicOr(p.err, 2u);
+      for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; it++)
+        if (!cv_wait(&full[it % p.stages], (uint32_t)(it / p.stages) & 1u, nullptr)) atomicOr(p.err, 2u);
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc = umma_idesc_bf16_mn(128, p.nmma);
       for (int it = 0; it < kiters; it++) {
-        const int s = it % WT_STAGES;
-        if (!cv_wait(&full[s], (uint32_t)(it / WT_STAGES) & 1u, &abort_flag)) {
+        const int s = it % p.stages;
+        if (!cv_wait(&full[s], (uint32_t)(it / p.stages) & 1u, &abort_flag)) {
           atomicOr(p.err, 4u);
           abort_flag = 1;
           break;
         }
         tc_fence_after();
-        const uint32_t a = smem_u32(smem + (size_t)s * p.stage_bytes), b = a + p.a_bytes;
-        const uint64_t ad = umma_desc_mn128(a, 8192), bd = umma_desc_mn128(b, 8192);
-        for (int kk = 0; kk < WT_KP / 16; kk++)  // 16 pixels = two 8-row groups: +2048 B (128 descriptor units)
-          umma_bf16(tmem, ad + 128ull * kk, bd + 128ull * kk, idesc, (it | kk) != 0);
+        const uint32_t a = smem_u32(smem + (size_t)s * p.stage_bytes);
+        const uint64_t ad = umma_desc_mn128(a, 8192);
+        for (int t = 0; t < p.tg; t++) {
+          const uint64_t bd = umma_desc_mn128(a + p.a_bytes + t * p.b_bytes, 8192);
+          for (int kk = 0; kk < WT_KP / 16; kk++)  // 16 pixels = two 8-row groups: +2048 B (128 descriptor units)
+            umma_bf16(tmem + t * p.cstride, ad + 128ull * kk, bd + 128ull * kk, idesc, (it | kk) != 0);
+        }
         umma_commit(&empty[s]);
       }
       umma_commit(&accf);
@@ -405,18 +415,30 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
     tc_fence_after();
     const int am = m0 + m;  // this thread's A-side channel
     if (ok && !abort_flag && kiters > 0) {
-      for (int c = 0; c < p.nmma; c += 16) {
-        uint32_t r[16];
-        tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c, r);
-        if (am >= p.a_ch) continue;
+      const bool vec = p.a_is_dy && (p.cin & 3) == 0 && (reinterpret_cast<uintptr_t>(p.dw) & 15) == 0;
+      for (int t = 0; t < p.tg; t++)
+        for (int c = 0; c < p.nmma; c += 16) {
+          uint32_t r[16];
+          tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(t * p.cstride + c), r);
+          if (am >= p.a_ch) continue;
+          float* dw = p.dw + (size_t)(tap0 + t) * p.cout * p.cin;
+          if (vec) {
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-          const int bn = n0 + c + j;
-          if (bn >= p.b_ch) break;
-          const int co = p.a_is_dy ? am : bn, ci = p.a_is_dy ? bn : am;
-          atomicAdd(&p.dw[((size_t)tap * p.cout + co) * p.cin + ci], __uint_as_float(r[j]));
+            for (int j = 0; j < 16; j += 4)
+              if (n0 + c + j < p.b_ch)
+                atomicAdd(reinterpret_cast<float4*>(dw + (size_t)am * p.cin + n0 + c + j),
+                          make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
+                                      __uint_as_float(r[j + 3])));
+            continue;
+          }
+#pragma unroll
+          for (int j = 0; j < 16; j++) {
+            const int bn = n0 + c + j;
+            if (bn >= p.b_ch) break;
+            const int co = p.a_is_dy ? am : bn, ci = p.a_is_dy ? bn : am;
+            atomicAdd(&dw[(size_t)co * p.cin + ci], __uint_as_float(r[j]));
+          }
         }
-      }
     }
   }
   tc_fence_before();
@@ -1311,12 +1333,26 @@ extern "C" int of_cnn_conv3x3_wgrad_tc(const void* x, int x_ctot, int x_coff, co
   p.err = err;
   p.a_bytes = 2 * 8192;
   p.b_bytes = (uint32_t)p.batoms * 8192;
-  p.stage_bytes = p.a_bytes + p.b_bytes;
-  p.tmem_cols = p.nmma <= 32 ? 32 : (p.nmma <= 64 ? 64 : (p.nmma <= 128 ? 128 : 256));
-  // split the pixel chunks so that about 4 CTAs per SM run, at least 8 chunks each
-  const long long tiles = 9LL * p.mtiles * p.ntiles;
-  long long ks = (4LL * kNumSMs + tiles - 1) / tiles;
-  if (ks > p.nchunk / 8) ks = p.nchunk / 8;
+  // As many taps per CTA as TMEM holds accumulators for, fewer where the chip would then not
+  // have a CTA of at least 4 chunks for each SM.
+  p.cstride = (p.nmma + 31) / 32 * 32;
+  const int tiles_mn = p.mtiles * p.ntiles;
+  p.tg = 9 * p.cstride <= 512 ? 9 : (3 * p.cstride <= 512 ? 3 : 1);
+  while (p.tg > 1 && (long long)(9 / p.tg) * tiles_mn * (p.nchunk / 4) < kNumSMs) p.tg /= 3;
+  p.stage_bytes = p.a_bytes + p.tg * p.b_bytes;
+  p.stages = (int)(200 * 1024 / p.stage_bytes);  // at least 2: 88 KB at most
+  if (p.stages > WT_STAGES) p.stages = WT_STAGES;
+  const int cols = p.tg * p.cstride;
+  p.tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
+  size_t smem = 1024 + (size_t)p.stages * p.stage_bytes;
+  size_t floor_smem = (size_t)p.tmem_cols * 448;  // resident CTAs never exceed 512 TMEM columns
+  if (smem < floor_smem) smem = floor_smem;
+  // split the pixel chunks over one wave of resident CTAs
+  const long long resident = 228 * 1024 / (long long)(smem + 2048);
+  const long long tiles = 9LL / p.tg * tiles_mn;
+  const int least = p.tg > 1 ? 4 : 8;
+  long long ks = kNumSMs * (resident > 1 ? resident : 1) / tiles;
+  if (ks > p.nchunk / least) ks = p.nchunk / least;
   if (ks < 1) ks = 1;
   p.chunks_per_cta = (int)((p.nchunk + ks - 1) / ks);
   ks = (p.nchunk + p.chunks_per_cta - 1) / p.chunks_per_cta;
@@ -1339,15 +1375,12 @@ extern "C" int of_cnn_conv3x3_wgrad_tc(const void* x, int x_ctot, int x_coff, co
     int rc = tmap_bf16(&tmb, static_cast<const bf16*>(bp) + bco, 4, dims, st, box, 128);
     if (rc) return rc;
   }
-  size_t smem = 1024 + (size_t)WT_STAGES * p.stage_bytes;
-  size_t floor_smem = (size_t)p.tmem_cols * 456 + 1024;  // resident CTAs never exceed 512 TMEM columns
-  if (smem < floor_smem) smem = floor_smem;
   {
     cudaError_t e = OF_SMEM_OPT_IN(wgrad_tc_kernel, smem);
     if (e != cudaSuccess)
       return set_error(OF_ERR_CUDA, "of_cnn_conv3x3_wgrad_tc: %zu B of shared memory: %s", smem, cudaGetErrorString(e));
   }
-  dim3 grid((unsigned)ks, p.mtiles * p.ntiles, 9);
+  dim3 grid((unsigned)ks, tiles_mn, 9 / p.tg);
   wgrad_tc_kernel<<<grid, CV_THREADS, smem, as_stream(stream)>>>(tma, tmb, p);
   return check_launch("of_cnn_conv3x3_wgrad_tc");
 }

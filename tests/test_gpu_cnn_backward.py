@@ -134,3 +134,24 @@ def test_pack_weights_of_all_layers(torch):
          (ctypes.c_int * (5 * n))(*[d for s in shapes for d in s]), (ctypes.c_void_p * n)(*[o.data_ptr() for o in many]), _sp())
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(many, one))
+
+
+@pytest.mark.parametrize("n,H,W,cin,cout,coff", [(10, 64, 64, 32, 2, 0), (10, 64, 64, 2, 32, 0), (10, 64, 64, 96, 32, 8),
+                                                 (10, 64, 64, 20, 30, 4), (4, 64, 64, 64, 64, 0), (2, 64, 64, 192, 64, 0),
+                                                 (4, 64, 64, 40, 128, 0), (64, 16, 16, 128, 144, 0), (5, 64, 64, 48, 48, 0)])
+def test_weight_gradient_taps_per_cta(torch, n, H, W, cin, cout, coff):
+    """Sizes with work enough for nine or three taps per CTA.  Sums of n H W products of two bfloat16
+    values of unit variance, accumulated in float32 in any order: 1e-4 of the largest, as for one tap."""
+    import cnn_oracle as O
+    from ofb200._lib import call
+    rng = np.random.default_rng(cin + cout)
+    xct, dct = (max(16, cin + coff) + 7) // 8 * 8, max(16, (cout + 7) // 8 * 8)
+    coff = coff // 8 * 8
+    x, dy = _bf(torch, rng, n, H, W, xct), _bf(torch, rng, n, H, W, dct)
+    dw = torch.zeros((9, cout, cin), dtype=torch.float32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    call("of_cnn_conv3x3_wgrad_tc", _P(x), xct, coff, _P(dy), dct, 0, n, H, W, cin, cout, _P(dw), _P(err), _sp())
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    want = O.conv3x3_wgrad(_f(x)[..., coff:coff + cin], _f(dy)[..., :cout])
+    assert np.max(np.abs(dw.cpu().numpy() - want)) <= 1e-4 * np.max(np.abs(want))
