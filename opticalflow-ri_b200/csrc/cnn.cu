@@ -68,12 +68,36 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
 
 // Waits for phase `parity`; gives up after CV_WAIT_NS or when *abort becomes nonzero.
 __device__ bool cv_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
+  if (mbar_try(bar, parity)) return true;  // the clock is read only when there is something to wait for
   unsigned long long t0 = globaltimer_ns();
   while (!mbar_try(bar, parity)) {
     if (abort && *abort) return false;
     if (globaltimer_ns() - t0 > CV_WAIT_NS) return false;
   }
   return true;
+}
+
+// The same wait by a whole warp, with one result for all its lanes.
+__device__ bool cv_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort) {
+  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  unsigned long long t0 = globaltimer_ns();
+  while (!__all_sync(0xffffffffu, mbar_try(bar, parity))) {
+    const bool stop = (abort && *abort) || globaltimer_ns() - t0 > CV_WAIT_NS;
+    if (__any_sync(0xffffffffu, stop)) return false;
+  }
+  return true;
+}
+
+// 1 in one lane of a converged warp.  The warps that issue copies and MMAs run their loops
+// converged and let this lane issue: inside a one-lane branch the operands are not uniform for
+// the compiler, and moving them to uniform registers costs more than a small MMA takes
+// (128 x 16 x 16 from shared memory: 171 cycles with index divisions, 53 unrolled, 39 converged).
+// In a training step of 16 crops of 128 x 128: the convolutions 564 -> 505 us, the weight
+// gradients 407 -> 355 us; both are now bound by the boxes they load, nine per pixel.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+  return e;
 }
 
 // Shared-memory matrix descriptor (sm_100 UMMA), K-major operand with a 32/64/128-byte
@@ -89,12 +113,13 @@ __host__ __device__ inline uint32_t umma_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
+// Issued by the lane whose `elect` is 1; all other operands are the same in every lane.
+__device__ __forceinline__ void umma_bf16(uint32_t elect, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                          uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-          tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 e, %5, 0;\n"
+      " @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elect)
       : "memory");
 }
 
@@ -182,6 +207,8 @@ __device__ __forceinline__ void cv_epilogue(const ConvParams& p, uint32_t taddr,
   }
 }
 
+// KSTEPS: MMAs of 16 channels per chunk of `ck`.
+template <int KSTEPS>
 __global__ void __launch_bounds__(CV_THREADS, 1)
     conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                       const ConvParams p) {
@@ -214,53 +241,56 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
   if (warp == 0) {
-    if (lane == 0) {
-      int issued = 0;
-      for (int it = 0; it < kiters && !abort_flag; it++) {
-        const int s = it % CV_STAGES;
-        const uint32_t ph = (uint32_t)(it / CV_STAGES) & 1u;
-        if (!cv_wait(&empty[s], ph ^ 1u, &abort_flag)) {
-          atomicOr(p.err, 1u);
-          abort_flag = 1;
-          break;
-        }
-        const int tap = it / p.nchunks, ch = it - tap * p.nchunks;
-        const int dy = tap / 3 - 1, dx = tap % 3 - 1;
-        uint8_t* a = smem + (size_t)s * p.stage_bytes;
+    const uint32_t el = elect_one();
+    int issued = 0, ch = 0, tap = 0;
+    for (int it = 0; it < kiters && !__any_sync(0xffffffffu, abort_flag); it++) {
+      const int s = it % CV_STAGES;
+      if (!cv_wait_warp(&empty[s], ((uint32_t)(it / CV_STAGES) & 1u) ^ 1u, &abort_flag)) {
+        if (el) atomicOr(p.err, 1u);
+        abort_flag = 1;
+        break;
+      }
+      uint8_t* a = smem + (size_t)s * p.stage_bytes;
+      if (el) {
         mbar_expect_tx(&full[s], p.a_bytes + p.b_bytes);
-        tma_load_4d(a, &tm_x, ch * p.ck, x0 + dx, y0 + dy, img0, &full[s]);
+        tma_load_4d(a, &tm_x, ch * p.ck, x0 + tap % 3 - 1, y0 + tap / 3 - 1, img0, &full[s]);
         tma_load_3d(a + p.a_bytes, &tm_w, ch * p.ck, n0, tap, &full[s]);
-        issued = it + 1;
       }
-      // the copies of the last stages must land before the CTA's shared memory is released
-      for (int it = issued > CV_STAGES ? issued - CV_STAGES : 0; it < issued; it++) {
-        const int s = it % CV_STAGES;
-        if (!cv_wait(&full[s], (uint32_t)(it / CV_STAGES) & 1u, nullptr)) atomicOr(p.err, 2u);
+      if (++ch == p.nchunks) {
+        ch = 0;
+        tap++;
       }
+      issued = it + 1;
+    }
+    // the copies of the last stages must land before the CTA's shared memory is released
+    for (int it = issued > CV_STAGES ? issued - CV_STAGES : 0; it < issued; it++) {
+      const int s = it % CV_STAGES;
+      if (!cv_wait_warp(&full[s], (uint32_t)(it / CV_STAGES) & 1u, nullptr) && el) atomicOr(p.err, 2u);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16(CV_M, p.bn);
-      const int swz = p.ck * 2, ksteps = p.ck / 16;
-      for (int it = 0; it < kiters; it++) {
-        const int s = it % CV_STAGES;
-        if (!cv_wait(&full[s], (uint32_t)(it / CV_STAGES) & 1u, &abort_flag)) {
-          atomicOr(p.err, 4u);
-          abort_flag = 1;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t a = smem_u32(smem + (size_t)s * p.stage_bytes), b = a + p.a_bytes;
-        const uint64_t ad = umma_desc_k(a, swz), bd = umma_desc_k(b, swz);
-        for (int kk = 0; kk < ksteps; kk++)  // +32 bytes of K per step (descriptor address unit: 16 B)
-          umma_bf16(tmem, ad + 2ull * kk, bd + 2ull * kk, idesc, (it | kk) != 0);
-        umma_commit(&empty[s]);
+    const uint32_t el = elect_one();
+    const uint32_t idesc = umma_idesc_bf16(CV_M, p.bn);
+    const uint32_t a0 = smem_u32(smem);
+    const uint64_t ad0 = umma_desc_k(a0, KSTEPS * 32), bd0 = umma_desc_k(a0 + p.a_bytes, KSTEPS * 32);
+    for (int it = 0; it < kiters; it++) {
+      const int s = it % CV_STAGES;
+      if (!cv_wait_warp(&full[s], (uint32_t)(it / CV_STAGES) & 1u, &abort_flag)) {
+        if (el) atomicOr(p.err, 4u);
+        abort_flag = 1;
+        break;
       }
-      umma_commit(&accf);  // arrives once every MMA issued above has completed
+      tc_fence_after();
+      const uint64_t off = (uint64_t)(s * (p.stage_bytes >> 4));
+#pragma unroll
+      for (int kk = 0; kk < KSTEPS; kk++)  // +32 bytes of K per step (descriptor address unit: 16 B)
+        umma_bf16(el, tmem, ad0 + off + 2ull * kk, bd0 + off + 2ull * kk, idesc, (it | kk) != 0);
+      if (el) umma_commit(&empty[s]);
+      __syncwarp();
     }
+    if (el) umma_commit(&accf);  // arrives once every MMA issued above has completed
     __syncwarp();
   } else {
     const int q = warp & 3;  // a warp reads the TMEM lanes 32 * (warp % 4) ...
@@ -293,7 +323,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
 // CTAs split the pixel range; each adds its sums into dW with atomics, four input channels at
 // a time where the lanes run over output channels (scalar ones touch a sector each there).
 // The 12 layers of a training step of 16 crops of 128 x 128: 634 us with one tap per CTA and
-// scalar atomics, 407 us here.
+// scalar atomics, 355 us here.
 constexpr int WT_KP = 64;  // pixels per K chunk
 constexpr int WT_STAGES = 4;
 
@@ -353,20 +383,21 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
   if (warp == 0) {
-    if (lane == 0) {
-      int issued = 0;
-      const uint32_t bytes = (atom1 ? 2u : 1u) * 8192u + p.tg * p.b_bytes;
-      const int sgn = p.a_is_dy ? 1 : -1;
-      for (int it = 0; it < kiters && !abort_flag; it++) {
-        const int s = it % p.stages;
-        if (!cv_wait(&empty[s], ((uint32_t)(it / p.stages) & 1u) ^ 1u, &abort_flag)) {
-          atomicOr(p.err, 1u);
-          abort_flag = 1;
-          break;
-        }
+    const uint32_t el = elect_one();
+    int issued = 0, s = 0;
+    uint32_t ph = 1;
+    const uint32_t bytes = (atom1 ? 2u : 1u) * 8192u + p.tg * p.b_bytes;
+    const int sgn = p.a_is_dy ? 1 : -1;
+    for (int it = 0; it < kiters && !__any_sync(0xffffffffu, abort_flag); it++) {
+      if (!cv_wait_warp(&empty[s], ph, &abort_flag)) {
+        if (el) atomicOr(p.err, 1u);
+        abort_flag = 1;
+        break;
+      }
+      if (el) {
         const int ch = c0 + it, grp = ch / p.tiles_per_group, t_in = ch - grp * p.tiles_per_group;
         const int ty = t_in / p.tiles_x, tx = t_in - ty * p.tiles_x;
         const int x0 = tx * p.bw, y0 = ty * p.bh, img0 = grp * p.nb;
@@ -374,38 +405,53 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
         mbar_expect_tx(&full[s], bytes);
         tma_load_4d(a, &tm_a, m0, x0, y0, img0, &full[s]);
         if (atom1) tma_load_4d(a + 8192, &tm_a, m0 + 64, x0, y0, img0, &full[s]);
-        for (int t = 0; t < p.tg; t++) {
-          const int dy = sgn * ((tap0 + t) / 3 - 1), dx = sgn * ((tap0 + t) % 3 - 1);
-          for (int j = 0; j < p.batoms; j++)
-            tma_load_4d(a + p.a_bytes + t * p.b_bytes + j * 8192, &tm_b, n0 + 64 * j, x0 + dx, y0 + dy, img0, &full[s]);
+        uint8_t* b = a + p.a_bytes;
+        for (int t = tap0; t < tap0 + p.tg; t++) {
+          const int dy = sgn * (t / 3 - 1), dx = sgn * (t % 3 - 1);
+          for (int j = 0; j < p.batoms; j++, b += 8192)
+            tma_load_4d(b, &tm_b, n0 + 64 * j, x0 + dx, y0 + dy, img0, &full[s]);
         }
-        issued = it + 1;
       }
-      for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; it++)
-        if (!cv_wait(&full[it % p.stages], (uint32_t)(it / p.stages) & 1u, nullptr)) atomicOr(p.err, 2u);
+      if (++s == p.stages) {
+        s = 0;
+        ph ^= 1u;
+      }
+      issued = it + 1;
     }
+    for (int it = issued > p.stages ? issued - p.stages : 0; it < issued; it++)
+      if (!cv_wait_warp(&full[it % p.stages], (uint32_t)(it / p.stages) & 1u, nullptr) && el) atomicOr(p.err, 2u);
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16_mn(128, p.nmma);
-      for (int it = 0; it < kiters; it++) {
-        const int s = it % p.stages;
-        if (!cv_wait(&full[s], (uint32_t)(it / p.stages) & 1u, &abort_flag)) {
-          atomicOr(p.err, 4u);
-          abort_flag = 1;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t a = smem_u32(smem + (size_t)s * p.stage_bytes);
-        const uint64_t ad = umma_desc_mn128(a, 8192);
-        for (int t = 0; t < p.tg; t++) {
-          const uint64_t bd = umma_desc_mn128(a + p.a_bytes + t * p.b_bytes, 8192);
-          for (int kk = 0; kk < WT_KP / 16; kk++)  // 16 pixels = two 8-row groups: +2048 B (128 descriptor units)
-            umma_bf16(tmem + t * p.cstride, ad + 128ull * kk, bd + 128ull * kk, idesc, (it | kk) != 0);
-        }
-        umma_commit(&empty[s]);
+    const uint32_t el = elect_one();
+    const uint32_t idesc = umma_idesc_bf16_mn(128, p.nmma);
+    const uint32_t a0 = smem_u32(smem);
+    const uint64_t ad0 = umma_desc_mn128(a0, 8192), bd0 = umma_desc_mn128(a0 + p.a_bytes, 8192);
+    int s = 0;
+    uint32_t ph = 0;
+    for (int it = 0; it < kiters; it++) {
+      if (!cv_wait_warp(&full[s], ph, &abort_flag)) {
+        if (el) atomicOr(p.err, 4u);
+        abort_flag = 1;
+        break;
       }
-      umma_commit(&accf);
+      tc_fence_after();
+      const uint64_t ad = ad0 + (uint64_t)(s * (p.stage_bytes >> 4));
+      uint64_t bd = bd0 + (uint64_t)(s * (p.stage_bytes >> 4));
+      uint32_t d = tmem;
+      for (int t = 0; t < p.tg; t++) {
+#pragma unroll
+        for (int kk = 0; kk < WT_KP / 16; kk++)  // 16 pixels = two 8-row groups: +2048 B (128 descriptor units)
+          umma_bf16(el, d, ad + 128ull * kk, bd + 128ull * kk, idesc, (it | kk) != 0);
+        d += p.cstride;
+        bd += p.b_bytes >> 4;
+      }
+      if (el) umma_commit(&empty[s]);
+      __syncwarp();
+      if (++s == p.stages) {
+        s = 0;
+        ph ^= 1u;
+      }
     }
+    if (el) umma_commit(&accf);
     __syncwarp();
   } else {
     const int q = warp & 3;
@@ -1068,13 +1114,15 @@ static int conv3x3(const void* x, int n, int H, int W, int cin, int x_ctot, int 
   size_t smem = 1024 + (size_t)CV_STAGES * p.stage_bytes;
   size_t floor_smem = (size_t)p.tmem_cols * 456 + 1024;
   if (smem < floor_smem) smem = floor_smem;
-  {
-    cudaError_t e = OF_SMEM_OPT_IN(conv3x3_tc_kernel, smem);
-    if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_cnn_conv3x3: %zu B of shared memory: %s", smem,
-                                           cudaGetErrorString(e));
-  }
+  cudaError_t e = ck == 64   ? OF_SMEM_OPT_IN(conv3x3_tc_kernel<4>, smem)
+                  : ck == 32 ? OF_SMEM_OPT_IN(conv3x3_tc_kernel<2>, smem)
+                             : OF_SMEM_OPT_IN(conv3x3_tc_kernel<1>, smem);
+  if (e != cudaSuccess)
+    return set_error(OF_ERR_CUDA, "of_cnn_conv3x3: %zu B of shared memory: %s", smem, cudaGetErrorString(e));
   dim3 grid((n / nb) * p.tiles_per_group, ntile);
-  conv3x3_tc_kernel<<<grid, CV_THREADS, smem, as_stream(stream)>>>(tmx, tmw, p);
+  (ck == 64   ? conv3x3_tc_kernel<4>
+   : ck == 32 ? conv3x3_tc_kernel<2>
+              : conv3x3_tc_kernel<1>)<<<grid, CV_THREADS, smem, as_stream(stream)>>>(tmx, tmw, p);
   return check_launch("of_cnn_conv3x3");
 }
 
