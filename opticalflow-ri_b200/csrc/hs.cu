@@ -77,8 +77,8 @@ __global__ void hs_sweep_kernel(const float* __restrict__ fx, const float* __res
 //
 // What bounds it: the issue slots (65 instructions per cell update, 16 of them float64
 // multiply-adds) at 50 % busy, and the latency of the pass's loads and barriers behind two
-// CTAs per SM (128 registers a thread).  600 sweeps, one pair alone: 256 x 256 2.75 -> 1.46 ms,
-// 512 x 512 3.3 -> 1.55 ms; 100 sweeps of 2048 x 2048 3.96 -> 2.3 ms (106 -> 180 G cell updates
+// CTAs per SM (128 registers a thread).  600 sweeps, one pair alone: 256 x 256 2.75 -> 1.19 ms,
+// 512 x 512 3.3 -> 1.25 ms; 100 sweeps of 2048 x 2048 3.96 -> 2.27 ms (106 -> 185 G cell updates
 // per second) against the column walk with one cell per thread and row it replaces.  4 x 4
 // blocks spill at 12 warps per SM (113 G/s), a 64 x 64 region in one CTA of 512 threads does
 // less halo work but leaves its loads exposed (164 G/s).
@@ -139,9 +139,9 @@ __device__ __forceinline__ void hb_load_uv(HbBlock& K, const HbPass& P, int gy0,
 }
 
 // The sweeps of a pass; on return the CTA's last sweep is in the blocks only.
-template <bool EDGE, bool DIV>
-__device__ __forceinline__ void hb_sweeps(HbBlock& K, const HbPass& P, double2* sm, bool in, int r0, int c0, int gy0,
-                                          int gx0) {
+template <bool RAG, bool DIV>
+__device__ __forceinline__ void hb_sweeps(HbBlock& K, const HbPass& P, double2* sm, bool in, int r0, int c0,
+                                          const HrWin& win) {
   if (in) hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, sm, r0, c0);
   __syncthreads();
   // a warp whose rows no later sweep reads (the outermost, in the last sweep) sits out
@@ -150,11 +150,11 @@ __device__ __forceinline__ void hb_sweeps(HbBlock& K, const HbPass& P, double2* 
   for (int s = 0; s < P.nsw; s += 2) {
     double2* const b0 = sm;
     double2* const b1 = sm + HB_RW * HB_RH;
-    if (needed(s)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, EDGE, DIV>(K, b0, r0, c0, gy0, gx0, P.H, P.W);
+    if (needed(s)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, RAG, DIV>(K, b0, r0, c0, win);
     if (s + 1 >= P.nsw) break;
     if (needed(s)) hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, b1, r0, c0);
     __syncthreads();
-    if (needed(s + 1)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, EDGE, DIV>(K, b1, r0, c0, gy0, gx0, P.H, P.W);
+    if (needed(s + 1)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, RAG, DIV>(K, b1, r0, c0, win);
     if (s + 2 >= P.nsw) break;
     if (needed(s + 1)) hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, b0, r0, c0);
     __syncthreads();
@@ -188,13 +188,16 @@ __global__ void __launch_bounds__(HbGeom::NT, 2) hs_pass_kernel(const HbPass P) 
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (in) hb_load_uv(K, P, gy0, gx0, inside);
-  if (edge)
-    hb_sweeps<true, false>(K, P, hb_sm, in, r0, c0, gy0, gx0);
+  const HrWin win = hr_window<HB_RW, HB_RH, HB_BX, HB_BY>(r0, c0, gy0, gx0, P.H, P.W);
+  // the region holds blocks that the image ends inside of
+  const bool rag = (P.W % HB_BX && x0 + HB_RW > P.W) || (P.H % HB_BY && y0 + HB_RH > P.H);
+  if (rag)
+    hb_sweeps<true, false>(K, P, hb_sm, in, r0, c0, win);
   else
-    hb_sweeps<false, false>(K, P, hb_sm, in, r0, c0, gy0, gx0);
+    hb_sweeps<false, false>(K, P, hb_sm, in, r0, c0, win);
   if (__syncthreads_or(in && !(ok && hr_in_range(K)))) {  // rare: see hr_row
     if (in) hb_load_uv(K, P, gy0, gx0, inside);
-    hb_sweeps<true, true>(K, P, hb_sm, in, r0, c0, gy0, gx0);
+    hb_sweeps<true, true>(K, P, hb_sm, in, r0, c0, win);
   }
   if (in && c0 >= HB_T && c0 < HB_T + HB_TW && r0 >= HB_T && r0 < HB_T + HB_TH) {
 #pragma unroll
@@ -261,9 +264,9 @@ extern "C" int of_hs_derivatives(const float* I0, const float* I1, float* fx, fl
 }
 
 // of_hs_solve_persistent: one pair through the persistent kernels of hsq.cu (of_hs_batch,
-// automatic schedule: the resident schedule when all the launch's CTAs run at once, else the
-// device work queue, whose items only wait for items of running CTAs, so it is correct
-// beside any other work on the GPU, if slower there).
+// automatic schedule: tagged halos, or counters for up to 8 sweeps and thin images, when all
+// the launch's CTAs run at once, else the device work queue, whose items only wait for items
+// of running CTAs, so it is correct beside any other work on the GPU, if slower there).
 constexpr int kHsSolveShape = 3;  // of_hs_batch tile shape for one pair: 32 x 32 regions, 8 sweeps per pass
 
 static size_t hs_persistent_ws(int H, int W, int pitch) {
@@ -282,6 +285,7 @@ extern "C" size_t of_hs_workspace_size(int H, int W, int pitch) {
   q.take<double>(2);
   q.take<int>(1);
   q.take<unsigned char>(hs_persistent_ws(H, W, pitch));
+  q.take<unsigned char>(hs_halo_bytes(H, W));
   return s.off > q.off ? s.off : q.off;
 }
 
@@ -371,6 +375,11 @@ extern "C" int of_hs_solve_persistent(const float* I0, const float* I1, float* U
   if (!workspace || workspace_bytes < of_hs_workspace_size(H, W, pitch))
     return set_error(OF_ERR_WORKSPACE, "of_hs_solve_persistent: workspace too small (%zu < %zu)", workspace_bytes,
                      of_hs_workspace_size(H, W, pitch));
+  const size_t hbs = hs_halo_bytes(H, W);
+  // Images with more tiles than SMs: a launch per pass, whose tiles all SMs share, beats the
+  // persistent queue (600 sweeps of 512 x 512: 1.23 ms against 2.98).
+  if (!hbs && H >= 16 && W >= 16)
+    return of_hs_solve(I0, I1, U, V, H, W, pitch, alpha, niter, err_out, workspace, workspace_bytes, stream);
   cudaStream_t st = as_stream(stream);
   const size_t N = (size_t)H * pitch;
   Carver c(workspace, workspace_bytes);
@@ -380,6 +389,7 @@ extern "C" int of_hs_solve_persistent(const float* I0, const float* I1, float* U
   int* status = c.take<int>(1);
   const size_t bws = hs_persistent_ws(H, W, pitch);
   void* bw = c.take<unsigned char>(bws);
+  void* halo = hbs ? c.take<unsigned char>(hbs) : nullptr;
   long long n = 0;
   if (err_out) {
     copy2_kernel<<<dim3((W + 255) / 256, H), 256, 0, st>>>(U, V, U0, V0, W, pitch);
@@ -389,7 +399,7 @@ extern "C" int of_hs_solve_persistent(const float* I0, const float* I1, float* U
   if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_hs_solve_persistent: %s", cudaGetErrorString(e));
   OfHsBatchPair q = {I0, I1, U, V, H, W, pitch, alpha, niter};
   OfTuning tun = {kHsSolveShape, 0, OF_HS_EXACT, OF_HS_SCHED_AUTO};
-  const int rc = of_hs_batch(&q, 1, &tun, status, 1ll << 20, bw, bws, stream);
+  const int rc = hs_batch(&q, 1, &tun, status, 1ll << 20, bw, bws, halo, stream);
   if (rc != OF_OK) return rc;
   if (err_out) {
     cudaMemsetAsync(acc, 0, 2 * sizeof(double), st);

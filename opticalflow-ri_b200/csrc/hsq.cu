@@ -519,6 +519,212 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2)
                                   err_flag);
 }
 
+// ---- One pair, register blocks and tagged halos ------------------------------------------
+// The resident schedule for one pair whose tiles all get an SM: the sweeps are hsweep.cuh's
+// register-blocked ones, 8 per stage, and a stage's halo needs neither counters nor fences.
+// Every owned cell is published as two 8-byte words, (u, stage) and (v, stage), each one
+// atomic access; a reader polls exactly the cells it needs until both words carry the stage.
+// An exchange is then one store and one load through L2, where counters cost the stores, a
+// fence, an atomic, a poll, a barrier and the loads in turn.
+// The published cells alternate between two buffers (halo, H x W cells each).  A buffer is
+// overwritten by stage p + 2, which a CTA starts only after it has read stage p + 1 from each
+// of its neighbours; they published that after a barrier behind their reads of stage p.
+// Tags start at 1 and the buffers at 0.  The last stage writes U, V, which a neighbour read
+// before its first publication: there are at least two stages.
+//
+// Shapes, region / T / block: one CTA per SM, the smallest region whose tiles fit the SMs.
+// What bounds a stage is latency (256 x 256: FP64 pipe 18 % busy, shared memory 37 %): more
+// threads with smaller blocks beat fewer with larger ones until registers run out (48 x 32:
+// 2 x 2 blocks 0.54 ms, 2 x 4 0.61), fewer exchanges beat less redundant cells (T = 4 on
+// 40 x 24 0.67 ms, T = 6 0.61, T = 10 0.58), and two CTAs per SM on 32 x 32 take 0.60.
+// Polling one cell at a time to spare L2 adds a round trip (0.56 to 0.59).  All 600 sweeps.
+// 600 sweeps, square images, before (counters, or their work queue) and now, ms:
+//   48 x 32  to 148 tiles of 32 x 16:  96 0.65 -> 0.51, 192 0.65 -> 0.53, 256 0.80 -> 0.56
+//   64 x 32  to 148 tiles of 48 x 16:  304 1.2 -> 0.66
+//   64 x 48  to 148 tiles of 48 x 32:  384 1.70 -> 0.99, 448 2.30 -> 1.02
+// Larger images: one launch per pass (hs.cu), 512 2.98 -> 1.23.
+template <int RW_, int RH_, int T_, int BX_, int BY_>
+struct HrShape {
+  static constexpr int RW = RW_, RH = RH_, T = T_, BX = BX_, BY = BY_, TW = RW - 2 * T, TH = RH - 2 * T;
+  using G = HrGeom<RW, RH, BX, BY>;
+  using K = HrBlock<BX, BY>;
+  static constexpr int NT = G::NT;
+  static_assert(T % BX == 0 && T % BY == 0, "blocks aligned to the image's first row and column");
+  static_assert(NT % 32 == 0, "the queue schedule runs in the same CTAs");
+  // two exchange buffers and each thread's cells at the start of the stage
+  static constexpr size_t OWN = 2 * G::BUF + (size_t)RW * RH * sizeof(float2);
+  static constexpr size_t SMEM = OWN > HqTile<32, 32, 8>::smem(false) ? OWN : HqTile<32, 32, 8>::smem(false);
+  static __host__ long long tiles(int H, int W) {
+    return (long long)((W + TW - 1) / TW) * ((H + TH - 1) / TH);
+  }
+};
+using HrSmall = HrShape<48, 32, 8, 2, 2>;
+using HrMid = HrShape<64, 32, 8, 2, 2>;
+using HrLarge = HrShape<64, 48, 8, 2, 4>;
+
+struct HrCell {
+  unsigned long long u, v;  // value (low word) and stage (high word)
+};
+
+__device__ __forceinline__ void hr_put(HrCell* p, float u, float v, unsigned int stage) {
+  const unsigned long long t = (unsigned long long)stage << 32;
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(t | __float_as_uint(u)),
+               "l"(t | __float_as_uint(v))
+               : "memory");
+}
+
+__device__ __forceinline__ HrCell hr_get(const HrCell* p) {
+  HrCell c;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(c.u), "=l"(c.v) : "l"(p) : "memory");
+  return c;
+}
+
+// nsw sweeps from the blocks' cells; the last one's results are in the blocks only.
+template <class S, bool RAG, bool DIV>
+__device__ __forceinline__ void hr_stage(typename S::K& K, double2* sm, bool in, int r0, int c0, const HrWin& win,
+                                         int nsw) {
+  // a block whose rows no later sweep reads sits out
+  auto needed = [&](int k) { return in && r0 + S::BY > 1 + k && r0 < S::RH - 1 - k; };
+#pragma unroll 1
+  for (int s = 0; s < nsw; s += 2) {
+    double2* const b0 = sm;
+    double2* const b1 = sm + S::RW * S::RH;
+    if (s == 0 ? in : needed(s - 1)) hr_publish<S::RW, S::RH, S::BX, S::BY>(K, b0, r0, c0);
+    __syncthreads();
+    if (needed(s)) hr_sweep<S::RW, S::RH, S::BX, S::BY, RAG, DIV>(K, b0, r0, c0, win);
+    if (s + 1 >= nsw) break;
+    if (needed(s)) hr_publish<S::RW, S::RH, S::BX, S::BY>(K, b1, r0, c0);
+    __syncthreads();
+    if (needed(s + 1)) hr_sweep<S::RW, S::RH, S::BX, S::BY, RAG, DIV>(K, b1, r0, c0, win);
+  }
+}
+
+template <class S>
+__device__ __forceinline__ void hrb_body(const HsqPair& P, HrCell* __restrict__ halo, int* status, long long wait_limit,
+                                         int* err_flag, float one) {
+  extern __shared__ __align__(16) double2 hr_sm[];
+  const int H = P.H, W = P.W, pitch = P.pitch, niter = P.niter, ntx = (W + S::TW - 1) / S::TW;
+  const int ty = (int)blockIdx.x / ntx, tx = (int)blockIdx.x - ty * ntx;
+  const int x0 = tx * S::TW - S::T, y0 = ty * S::TH - S::T;  // image position of region cell (0, 0)
+  const int c0 = ((int)threadIdx.x % S::G::NX) * S::BX, r0 = ((int)threadIdx.x / S::G::NX) * S::BY;
+  const int gx0 = x0 + c0, gy0 = y0 + r0;
+  const bool in = gx0 + S::BX > 0 && gy0 + S::BY > 0 && gx0 < W && gy0 < H;  // the block has cells in the image
+  const HrWin win = hr_window<S::RW, S::RH, S::BX, S::BY>(r0, c0, gy0, gx0, H, W);
+  // the region holds blocks that the image ends inside of
+  const bool rag = (W % S::BX && x0 + S::RW > W) || (H % S::BY && y0 + S::RH > H);
+  const size_t cells = (size_t)H * W;
+  float2* const start = reinterpret_cast<float2*>(hr_sm + 2 * S::RW * S::RH) + threadIdx.x;
+  typename S::K K;
+  unsigned int own = 0, ring = 0;  // the block's cells in the image, owned by this CTA or by others (bit j * BX + i)
+  bool fin = true, ok = true;
+#pragma unroll
+  for (int j = 0; j < S::BY; j++)
+#pragma unroll
+    for (int i = 0; i < S::BX; i++) {
+      const int r = r0 + j, c = c0 + i, gy = y0 + r, gx = x0 + c;
+      K.g[j][i] = make_float2(0.f, 0.f);
+      K.gt[j][i] = 0.f;
+      K.u[j][i] = K.v[j][i] = 0.0;
+      if (gy < 0 || gy >= H || gx < 0 || gx >= W) continue;
+      float fx, fy, ft;
+      const bool f = hq_deriv(P, gy, gx, fx, fy, ft);
+      K.g[j][i] = make_float2(fx, fy);
+      K.gt[j][i] = ft;
+      const size_t gi = (size_t)gy * pitch + gx;
+      K.u[j][i] = (double)__ldcg(P.U + gi);
+      K.v[j][i] = (double)__ldcg(P.V + gi);
+      const unsigned int bit = 1u << (j * S::BX + i);
+      if (r >= S::T && r < S::T + S::TH && c >= S::T && c < S::T + S::TW) {
+        own |= bit;
+        fin = fin && f;  // each pixel checked once
+      } else {
+        ring |= bit;
+      }
+    }
+  if (__syncthreads_or(!fin) && threadIdx.x == 0) atomicOr(status, OF_ST_NONFINITE_INPUT);
+  ok = hr_init_den(K, P.a2, one) || !in;
+  const bool den_ok = ok;
+  const int np = (niter + S::T - 1) / S::T;
+  bool gave_up = false;
+  for (int p = 0; p < np; p++) {
+    if (p > 0) {  // the halo: the neighbours' results of the previous stage, tag p
+      const HrCell* src = halo + (size_t)((p - 1) & 1) * cells;
+      unsigned int miss = ring;
+      for (long long k = 0; miss; k++) {
+        HrCell got[S::BX * S::BY];
+#pragma unroll
+        for (int b = 0; b < S::BX * S::BY; b++)
+          if (miss >> b & 1) got[b] = hr_get(src + (size_t)(gy0 + b / S::BX) * W + gx0 + b % S::BX);
+#pragma unroll
+        for (int b = 0; b < S::BX * S::BY; b++)
+          if ((miss >> b & 1) &&
+              (gave_up || ((unsigned int)(got[b].u >> 32) == (unsigned int)p && (unsigned int)(got[b].v >> 32) == (unsigned int)p))) {
+            K.u[b / S::BX][b % S::BX] = (double)__uint_as_float((unsigned int)got[b].u);
+            K.v[b / S::BX][b % S::BX] = (double)__uint_as_float((unsigned int)got[b].v);
+            miss &= ~(1u << b);
+          }
+        // after a wait that gave up, here or in another CTA, nothing waits any more
+        if (miss && (k >= wait_limit || ((k & 255) == 255 && (*(volatile int*)status & OF_ST_WAIT_TIMEOUT)))) {
+          gave_up = true;
+          atomicOr(status, OF_ST_WAIT_TIMEOUT);
+          atomicExch(err_flag, 1);
+        }
+      }
+    }
+    // the stage's first values, for a repeat with DIV
+#pragma unroll
+    for (int b = 0; b < S::BX * S::BY; b++)
+      start[b * S::NT] = make_float2((float)K.u[b / S::BX][b % S::BX], (float)K.v[b / S::BX][b % S::BX]);
+    const int nsw = min(S::T, niter - p * S::T);
+    if (rag)
+      hr_stage<S, true, false>(K, hr_sm, in, r0, c0, win, nsw);
+    else
+      hr_stage<S, false, false>(K, hr_sm, in, r0, c0, win, nsw);
+    if (__syncthreads_or(in && !(den_ok && hr_in_range(K)))) {  // rare: see hr_row
+#pragma unroll
+      for (int b = 0; b < S::BX * S::BY; b++) {
+        const float2 s = start[b * S::NT];
+        K.u[b / S::BX][b % S::BX] = (double)s.x;
+        K.v[b / S::BX][b % S::BX] = (double)s.y;
+      }
+      hr_stage<S, true, true>(K, hr_sm, in, r0, c0, win, nsw);
+      K.lo = 0xffffffffu;
+      K.hi = 0.f;
+      __syncthreads();
+    }
+    HrCell* dst = halo + (size_t)(p & 1) * cells;
+    fin = true;
+#pragma unroll
+    for (int b = 0; b < S::BX * S::BY; b++)
+      if (own >> b & 1) {
+        const int gy = gy0 + b / S::BX, gx = gx0 + b % S::BX;
+        const float u = (float)K.u[b / S::BX][b % S::BX], v = (float)K.v[b / S::BX][b % S::BX];
+        if (p < np - 1) {
+          hr_put(dst + (size_t)gy * W + gx, u, v, (unsigned int)(p + 1));
+        } else {
+          P.U[(size_t)gy * pitch + gx] = u;
+          P.V[(size_t)gy * pitch + gx] = v;
+          fin = fin && isfinite(u) && isfinite(v);
+        }
+      }
+  }
+  if (np > 0 && __syncthreads_or(!fin) && threadIdx.x == 0) atomicOr(status, OF_ST_NONFINITE_OUTPUT);
+}
+
+// One CTA per tile of the above, or per item of the queue schedule (shape 32 x 32, T = 8) when
+// they do not all run at once, decided as in hsa_kernel.
+template <class S>
+__global__ void __launch_bounds__(S::NT, 1)
+    hrb_kernel(const HsqPair* __restrict__ pairs, unsigned int tiles_total, int max_passes, unsigned long long* ticket,
+               unsigned int* done, int* status, long long wait_limit, int* err_flag, unsigned int* arrived, int* mode,
+               HrCell* __restrict__ halo, float one) {
+  if (hq_decide_mode(arrived, mode) == HQ_MODE_RESIDENT)
+    hrb_body<S>(pairs[0], halo, status, wait_limit, err_flag, one);
+  else
+    hsq_body<32, 32, 8, false, S::NT>(pairs, 1, tiles_total, max_passes, ticket, done, status, wait_limit,
+                                           err_flag);
+}
+
 // ---- One pair on one thread-block cluster ------------------------------------------------
 // For images that one cluster of at most 16 CTAs covers with tiles of at most HC_T x HC_T
 // cells (256 x 256 and smaller).  CTA (cx, cy) owns a tile and holds the tile plus a
@@ -940,8 +1146,33 @@ extern "C" size_t of_hs_batch_workspace_size(const OfHsBatchPair* pairs, int n) 
   return s.off;
 }
 
+size_t ofb::hs_halo_bytes(int H, int W) {
+  return H >= 16 && W >= 16 && HrLarge::tiles(H, W) <= kNumSMs ? 2 * sizeof(HrCell) * (size_t)H * (size_t)W : 0;
+}
+
+// Launches the tagged-halo schedule of shape S when every tile gets an SM of the device.
+template <class S>
+static cudaError_t hrb_launch(const OfHsBatchPair& q, int sms, const HsqPair* dpairs, unsigned int tiles_total,
+                              int max_passes, const HsqControl& c, int* status, long long wait_limit, void* halo,
+                              cudaStream_t st, bool* launched) {
+  const long long tiles = S::tiles(q.H, q.W);
+  if (*launched || tiles > sms) return cudaSuccess;
+  cudaError_t e = OF_SMEM_OPT_IN(hrb_kernel<S>, S::SMEM);
+  if (e == cudaSuccess) e = cudaMemsetAsync(halo, 0, hs_halo_bytes(q.H, q.W), st);
+  if (e != cudaSuccess) return e;
+  hrb_kernel<S><<<(int)tiles, S::NT, S::SMEM, st>>>(dpairs, tiles_total, max_passes, c.ticket, c.done, status, wait_limit,
+                                                    c.err_flag, c.arrived, c.mode, static_cast<HrCell*>(halo), 1.0f);
+  *launched = true;
+  return cudaGetLastError();
+}
+
 extern "C" int of_hs_batch(const OfHsBatchPair* pairs, int n, const OfTuning* tuning, int* status,
                            long long wait_limit, void* workspace, size_t workspace_bytes, void* stream) {
+  return hs_batch(pairs, n, tuning, status, wait_limit, workspace, workspace_bytes, nullptr, stream);
+}
+
+int ofb::hs_batch(const OfHsBatchPair* pairs, int n, const OfTuning* tuning, int* status, long long wait_limit,
+             void* workspace, size_t workspace_bytes, void* halo, void* stream) {
   OF_REQUIRE(pairs && n > 0 && n <= (1 << 20), "of_hs_batch: bad pair list");
   OF_REQUIRE(status, "of_hs_batch: status (a device array of n ints) is required");
   OF_REQUIRE(wait_limit > 0, "of_hs_batch: wait_limit must be positive");
@@ -1050,6 +1281,17 @@ extern "C" int of_hs_batch(const OfHsBatchPair* pairs, int n, const OfTuning* tu
   // RESIDENT: one CTA per tile, all of them running at once (refused when the device cannot
   // hold them); AUTO: the adaptive kernel with one CTA per tile when the device can hold them
   // (it falls back to the queue itself when they do not all get an SM), else the queue
+  // With a halo buffer: one pair of at least two stages by the tagged-halo schedule.
+  if (halo && n == 1 && !fast && shape == 3 && sched == OF_HS_SCHED_AUTO && pairs[0].niter > HrSmall::T) {
+    bool launched = false;
+    e = hrb_launch<HrSmall>(pairs[0], sms, dpairs, tiles_total, max_passes, ctl, status, wait_limit, halo, st, &launched);
+    if (e == cudaSuccess)
+      e = hrb_launch<HrMid>(pairs[0], sms, dpairs, tiles_total, max_passes, ctl, status, wait_limit, halo, st, &launched);
+    if (e == cudaSuccess)
+      e = hrb_launch<HrLarge>(pairs[0], sms, dpairs, tiles_total, max_passes, ctl, status, wait_limit, halo, st, &launched);
+    if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_hs_batch: launch: %s", cudaGetErrorString(e));
+    if (launched) return check_launch("of_hs_batch", nl + 1);
+  }
   HqKind kind = HQ_QUEUE;
   long long cap = 0;
   if (sched == OF_HS_SCHED_RESIDENT || sched == OF_HS_SCHED_AUTO) {

@@ -11,6 +11,12 @@ namespace ofb {
 
 constexpr int HQ_THREADS = 256;  // threads per CTA of the region sweeps
 
+// of_hs_batch with a scratch buffer of hs_halo_bytes(H, W) bytes (0: the size has none) through
+// which one pair may run by the tagged-halo schedule.
+int hs_batch(const OfHsBatchPair* pairs, int n, const OfTuning* tuning, int* status, long long wait_limit,
+             void* workspace, size_t workspace_bytes, void* halo, void* stream);
+size_t hs_halo_bytes(int H, int W);
+
 // (u, v) as held in shared memory: float64 copies of the float32 values for the bit-exact
 // arithmetic (the reference's float64 stencil sums then need no conversion per
 // neighbour), float32 for the float32 averaging.
@@ -109,57 +115,6 @@ __device__ __forceinline__ void hq_update(const HqRow<FAST>& U, const HqRow<FAST
   hq_cell<FAST, false>(U, C, D, i, sfx, sfy, sft, nullptr, a2, du[i], dv[i]);
 }
 
-// Sweep s of the region: thread t owns column t % RW and walks a band of the rows the sweep
-// computes (band t / RW of NT / RW, NT the CTA's threads) with a 3-row register window, so each row it
-// visits costs one row of loads.  The input and output buffers are distinct (ping-pong), so
-// the pointers are restrict: the loads of the next rows may move ahead of this row's
-// stores and the rows' float64 chains overlap.  On image borders the neighbour columns and the window's
-// outer rows go through the 'mirror' map; inside the image the mapped row is the row.
-template <int RW, int RH, int T, bool EDGE, bool FAST, int NT = HQ_THREADS>
-__device__ __forceinline__ void hq_sweep(const float* __restrict__ sfx, const float* __restrict__ sfy,
-                                         const float* __restrict__ sft, const HqVal<FAST>* __restrict__ su,
-                                         const HqVal<FAST>* __restrict__ sv, HqVal<FAST>* __restrict__ du,
-                                         HqVal<FAST>* __restrict__ dv, int s, int x0, int y0, int H, int W,
-                                         float a2) {
-  static_assert(NT % RW == 0, "a whole number of bands");
-  constexpr int NB = NT / RW;
-  const int c = (int)threadIdx.x % RW, band = (int)threadIdx.x / RW;
-  if (c < 1 + s || c >= RW - 1 - s) return;
-  const int gx = x0 - T + c;
-  if (EDGE && (gx < 0 || gx >= W)) return;
-  int cm = c - 1, cp = c + 1;
-  if (EDGE) {
-    cm = mirror1(gx - 1, W) - (x0 - T);
-    cp = mirror1(gx + 1, W) - (x0 - T);
-  }
-  int lo = 1 + s, hi = RH - 1 - s;
-  if (EDGE) {  // rows in the image only
-    lo = max(lo, T - y0);
-    hi = min(hi, H + T - y0);
-  }
-  const int n = hi - lo;
-  if (n <= 0) return;
-  const int ra = lo + (n * band) / NB, rb = lo + (n * (band + 1)) / NB;
-  if (rb <= ra) return;
-  auto row_of = [&](int r) { return EDGE ? mirror1(y0 - T + r, H) - (y0 - T) : r; };
-  HqRow<FAST> A, B, C;
-  hq_load<RW, FAST>(A, su, sv, row_of(ra - 1), cm, c, cp);
-  hq_load<RW, FAST>(B, su, sv, ra, cm, c, cp);
-#pragma unroll 1
-  for (int r = ra; r < rb; r += 3) {
-    hq_load<RW, FAST>(C, su, sv, row_of(r + 1), cm, c, cp);
-    hq_update<FAST>(A, B, C, r * RW + c, sfx, sfy, sft, du, dv, a2);
-    if (r + 1 < rb) {
-      hq_load<RW, FAST>(A, su, sv, row_of(r + 2), cm, c, cp);
-      hq_update<FAST>(B, C, A, (r + 1) * RW + c, sfx, sfy, sft, du, dv, a2);
-    }
-    if (r + 2 < rb) {
-      hq_load<RW, FAST>(B, su, sv, row_of(r + 3), cm, c, cp);
-      hq_update<FAST>(C, A, B, (r + 2) * RW + c, sfx, sfy, sft, du, dv, a2);
-    }
-  }
-}
-
 // K consecutive rows r0 .. r0 + K - 1 of a thread's column in one basic block: rows r0 - 1
 // .. r0 + K are loaded, the K cells computed and stored, so the scheduler overlaps the
 // rows' float64 chains instead of running them one after another.
@@ -179,9 +134,12 @@ __device__ __forceinline__ void hq_rows(const float* __restrict__ sfx, const flo
   }
 }
 
-// Sweep s of the region, the cells and band partition of hq_sweep, with each band walked in
-// chunks of up to HQ_CHUNK rows (hq_rows).  A band is a whole number of warps (RW a multiple
-// of 32), so the chunk lengths are warp-uniform.  RD as in hq_cell.
+// Sweep s of the region: thread t owns column t % RW and a band of the rows the sweep computes
+// (band t / RW of NT / RW, NT the CTA's threads), walked in chunks of up to HQ_CHUNK rows
+// (hq_rows).  A band is a whole number of warps (RW a multiple of 32), so the chunk lengths are
+// warp-uniform.  The input and output buffers are distinct (ping-pong), so the pointers are
+// restrict.  On image borders the neighbour columns and the outer rows go through the 'mirror'
+// map; inside the image the mapped row is the row.  RD as in hq_cell.
 constexpr int HQ_CHUNK = 4;
 
 template <int RW, int RH, int T, bool EDGE, bool FAST, int NT, bool RD>
@@ -248,6 +206,8 @@ struct HrBlock {
   float2 g[BY][BX];    // spatial derivatives (fx, fy)
   float gt[BY][BX];    // temporal derivative
   float y[BY][BX];     // 1 / den, correctly rounded
+  static constexpr bool DEN = BX * BY <= 4;  // a small block has registers for the denominators too
+  float den[DEN ? BY : 1][DEN ? BX : 1];
   float a2;            // alpha^2
   float one;           // 1.0f, unknown to the assembler (see hr_row)
   unsigned lo;         // range of the numerators seen: smallest 2 |num| (bits) - 1
@@ -287,6 +247,7 @@ __device__ __forceinline__ bool hr_init_den(HrBlock<BX, BY>& K, float a2, float 
       const float den = hr_den(K.g[j][i], a2);
       ok = ok && den >= 1.f / HR_DEN && den <= HR_DEN && __float_as_uint(K.gt[j][i]) != 0x80000000u;
       K.y[j][i] = __frcp_rn(den);
+      if constexpr (HrBlock<BX, BY>::DEN) K.den[j][i] = den;
     }
   return ok;
 }
@@ -322,7 +283,11 @@ __device__ __forceinline__ void hr_row(HrBlock<BX, BY>& K, int j, const HrRow<BX
     const float2 m = make_float2((float)a, (float)b), g = K.g[j][i];
     const float2 gm = __fmul2_rn(g, m);
     const float num = __fadd_rn(__fadd_rn(gm.x, gm.y), K.gt[j][i]);
-    const float den = hr_den(g, K.a2);
+    float den;
+    if constexpr (HrBlock<BX, BY>::DEN)
+      den = K.den[j][i];
+    else
+      den = hr_den(g, K.a2);
     float der;
     if (DIV) {
       der = __fdiv_rn(num, den);
@@ -354,36 +319,54 @@ __device__ __forceinline__ void hr_publish(const HrBlock<BX, BY>& K, double2* bu
         buf[r0 * RW + c0 / BX + j * RW + i * G::NX] = make_double2(K.u[j][i], K.v[j][i]);
 }
 
+// Where a block finds its window in the exchange buffer.  Neighbours beyond an image border are
+// the mirror cells (-1 shows 1, n shows n - 2), which is only another index: every cell is
+// published (BX or BY is 2), and with blocks aligned to the image's first row and column
+// (T a multiple of BX and BY) a border lies between blocks, except the last row or column of an
+// image whose sides are no multiple of the block.  There the neighbour is an outside cell of
+// the block itself, and hr_sweep's RAG form takes the cell on the other side instead.
+// Neighbours beyond the region are held at its rim.  H, W >= 2.
+struct HrWin {
+  int cl, cr;  // columns beside the block, as offsets in a row
+  int rt, rb;  // row offsets above and below it
+  int jr, ir;  // RAG: the block's last row and column in the image when others follow, else -1
+};
+
+template <int RW, int RH, int BX, int BY>
+__device__ __forceinline__ HrWin hr_window(int r0, int c0, int gy0, int gx0, int H, int W) {
+  static_assert(BX == 2 || BY == 2, "every cell of a block is published");
+  using G = HrGeom<RW, RH, BX, BY>;
+  HrWin w;
+  const int l = gx0 == 0 ? c0 + 1 : (c0 > 0 ? c0 - 1 : 0);
+  const int r = gx0 + BX == W ? c0 + BX - 2 : (c0 + BX < RW ? c0 + BX : RW - 1);
+  w.cl = G::at(0, l);
+  w.cr = G::at(0, r);
+  w.rt = (gy0 == 0 ? r0 + 1 : (r0 > 0 ? r0 - 1 : 0)) * RW;
+  w.rb = (gy0 + BY == H ? r0 + BY - 2 : (r0 + BY < RH ? r0 + BY : RH - 1)) * RW;
+  w.jr = gy0 + BY > H ? H - 1 - gy0 : -1;
+  w.ir = gx0 + BX > W ? W - 1 - gx0 : -1;
+  return w;
+}
+
 // One sweep of the block from the exchange buffer `buf` (the other blocks' cells before the
-// sweep).  EDGE: the region touches the image border, where the neighbour beyond it is the
-// mirror cell: -1 shows 1 and n shows n - 2, which the window holds on the cell's other side
-// (gy0, gx0: image position of the block's first cell; H, W >= 2).  Cells outside the image
-// or on the region's rim get values that no exact cell reads.
-template <int RW, int RH, int BX, int BY, bool EDGE, bool DIV>
-__device__ __forceinline__ void hr_sweep(HrBlock<BX, BY>& K, const double2* buf, int r0, int c0, int gy0, int gx0,
-                                         int H, int W) {
+// sweep).  Cells outside the image or on the region's rim get values that no exact cell reads.
+template <int RW, int RH, int BX, int BY, bool RAG, bool DIV>
+__device__ __forceinline__ void hr_sweep(HrBlock<BX, BY>& K, const double2* buf, int r0, int c0, const HrWin& win) {
   using G = HrGeom<RW, RH, BX, BY>;
   const int cb = c0 / BX;
-  // the columns beside the block (held inside the region at its rim)
-  const int cl = c0 > 0 ? (BX - 1) * G::NX + cb - 1 : cb, cr = c0 + BX < RW ? cb + 1 : cb;
-  auto fix = [&](HrRow<BX>& R) {  // the window's columns at the image border
-    if (!EDGE) return;
-    if (gx0 == 0) {
-      R.u[0] = R.u[2];
-      R.v[0] = R.v[2];
-    }
-    if (gx0 + BX >= W) {
+  auto fix = [&](HrRow<BX>& R) {
+    if constexpr (RAG) {
 #pragma unroll
-      for (int i = 2; i < BX + 2; i++)
-        if (gx0 - 1 + i == W) {
-          R.u[i] = R.u[i - 2];
-          R.v[i] = R.v[i - 2];
-        }
+      for (int i = 0; i + 1 < BX; i++) {
+        const bool p = win.ir == i;
+        R.u[i + 2] = p ? R.u[i] : R.u[i + 2];
+        R.v[i + 2] = p ? R.v[i] : R.v[i + 2];
+      }
     }
   };
   auto ring = [&](HrRow<BX>& R, int row) {  // a row above or below the block
-    const double2* b = buf + row * RW;
-    double2 t = b[cl];
+    const double2* b = buf + row;
+    double2 t = b[win.cl];
     R.u[0] = t.x;
     R.v[0] = t.y;
 #pragma unroll
@@ -392,14 +375,14 @@ __device__ __forceinline__ void hr_sweep(HrBlock<BX, BY>& K, const double2* buf,
       R.u[i + 1] = t.x;
       R.v[i + 1] = t.y;
     }
-    t = b[cr];
+    t = b[win.cr];
     R.u[BX + 1] = t.x;
     R.v[BX + 1] = t.y;
     fix(R);
   };
   auto own = [&](HrRow<BX>& R, int j) {  // the block's row j with the cells beside it
     const double2* b = buf + (r0 + j) * RW;
-    const double2 l = b[cl], r = b[cr];
+    const double2 l = b[win.cl], r = b[win.cr];
     R.u[0] = l.x;
     R.v[0] = l.y;
 #pragma unroll
@@ -412,7 +395,7 @@ __device__ __forceinline__ void hr_sweep(HrBlock<BX, BY>& K, const double2* buf,
     fix(R);
   };
   HrRow<BX> w[3];
-  ring(w[0], r0 > 0 ? r0 - 1 : 0);
+  ring(w[0], win.rt);
   own(w[1], 0);
 #pragma unroll
   for (int j = 0; j < BY; j++) {
@@ -420,10 +403,19 @@ __device__ __forceinline__ void hr_sweep(HrBlock<BX, BY>& K, const double2* buf,
     if (j + 1 < BY)
       own(D, j + 1);
     else
-      ring(D, r0 + BY < RH ? r0 + BY : RH - 1);
-    if (EDGE && gy0 + j == 0) U = D;
-    if (EDGE && gy0 + j == H - 1) D = U;
-    hr_row<BX, BY, DIV>(K, j, U, C, D);
+      ring(D, win.rb);
+    if (RAG && j + 1 < BY) {
+      const bool p = win.jr == j;
+      HrRow<BX> M;
+#pragma unroll
+      for (int i = 0; i < BX + 2; i++) {
+        M.u[i] = p ? U.u[i] : D.u[i];
+        M.v[i] = p ? U.v[i] : D.v[i];
+      }
+      hr_row<BX, BY, DIV>(K, j, U, C, M);
+    } else {
+      hr_row<BX, BY, DIV>(K, j, U, C, D);
+    }
   }
 }
 
