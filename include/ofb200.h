@@ -55,6 +55,9 @@ int of_last_error(char* buf, size_t n);
  * calls: numpy frame -> pinned upload buffer, pinned download buffer -> numpy result).
  * Blocking; one pooled copy runs at a time; a forked child copies on its own thread. */
 int of_host_copy(void* dst, const void* src, size_t bytes);
+/* The same copy with stores that go past the CPU's caches, for a pinned buffer that the
+ * device reads next (its upload reads memory instead of other cores' dirty cache lines). */
+int of_host_stage(void* dst, const void* src, size_t bytes);
 
 /* ---------------------------------------------------------------------------------
  * A1 Gaussian prefilter — replaces gaussian_filterPx / convolveSeparableFilter

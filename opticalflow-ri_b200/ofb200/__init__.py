@@ -85,6 +85,17 @@ def par_copyto(dst: np.ndarray, src: np.ndarray) -> None:
     np.copyto(dst, src)
 
 
+def stage_copyto(dst: np.ndarray, src: np.ndarray) -> None:
+    """np.copyto(dst, src) into a pinned upload buffer: same-dtype C-contiguous arrays through
+    of_host_stage (threaded, past the CPU's caches, from which the upload would read slowly);
+    anything else through numpy."""
+    if dst.dtype == src.dtype and dst.shape == src.shape and dst.flags.c_contiguous and src.flags.c_contiguous:
+        from ._lib import call
+        call("of_host_stage", dst.ctypes.data, src.ctypes.data, dst.nbytes)
+        return
+    np.copyto(dst, src)
+
+
 def to_host_pair(a, b):
     """Two same-shape float32 CUDA planes -> two new numpy arrays: asynchronous copies into
     cached pinned buffers; the first plane leaves the pinned buffer (threaded host copy)

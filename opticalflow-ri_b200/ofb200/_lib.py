@@ -78,6 +78,7 @@ _SIGS = {
     "of_last_error": ([ctypes.c_char_p, _Z], _I),
     "of_launch_count": ([], ctypes.c_ulonglong),
     "of_host_copy": ([_P, _P, _Z], _I),
+    "of_host_stage": ([_P, _P, _Z], _I),
     "of_prefilter_f32": ([_P, _I, _P, _I, _I, _I, _P, _I, _P], _I),
     "of_prefilter_u8": ([_P, _I, _P, _I, _I, _I, _P, _I, _P], _I),
     "of_u8_to_f32": ([_P, _I, _P, _I, _I, _I, _P], _I),

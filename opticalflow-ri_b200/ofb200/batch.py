@@ -18,7 +18,7 @@ from dataclasses import dataclass, field
 
 import torch
 
-from . import _lib
+from . import _lib, stage_copyto
 from . import graph as _graph
 from . import ops
 
@@ -223,7 +223,10 @@ class HostBatch:
                 if t.is_pinned() and t.dtype == p.dtype:
                     srcs.append(t)
                 else:
-                    p.copy_(t)
+                    if t.dtype == p.dtype:
+                        stage_copyto(p.numpy(), t.detach().numpy())
+                    else:
+                        p.copy_(t)
                     srcs.append(p)
         cur, up, down = torch.cuda.current_stream(), self._up, self._down
         up.wait_event(st["done"])  # the slot's previous replay has read its inputs

@@ -15,7 +15,7 @@ import threading
 import numpy as np
 import torch
 
-from . import par_copyto
+from . import stage_copyto
 
 ENABLED = True
 
@@ -68,7 +68,7 @@ class GraphCache:
                         pinned[i] = (torch.empty(s.shape, dtype=s.dtype, pin_memory=True), torch.cuda.Event())
                     p, done = pinned[i]
                     done.synchronize()  # the previous asynchronous copy out of this buffer has finished
-                    par_copyto(p.numpy(), t)
+                    stage_copyto(p.numpy(), t)
                     s.copy_(p, non_blocking=True)
                     done.record()
                 else:
