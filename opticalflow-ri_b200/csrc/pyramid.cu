@@ -256,31 +256,25 @@ static int ksize_of(int in, int out, int bicubic) {
 }
 
 // ----------------------------------------------------------------------------- spline
-// Reciprocal pivots of the constant (1, 4, 1) tridiagonal elimination, shared by every
-// line: c[0] = 1/4, c[r] = 1/(4 - c[r-1]) until the fixed point (2 - sqrt 3) repeats in
-// double.  One thread runs the short division chain (about 20 steps); the block fills the
-// constant tail.
-__global__ void spline_recip_kernel(double* c, int m) {
-  __shared__ double tail;
-  __shared__ int rc;
+// Reciprocal pivots of the constant (1, 4, 1) tridiagonal elimination, the same for every
+// line: c[0] = 1/4, c[r] = 1/(4 - c[r-1]), which reaches its fixed point (2 - sqrt 3) in double
+// within 20 steps (each step shrinks the distance 14 times).  Every CTA of the solve computes
+// the short division chain itself; c[r] = c[NAK_PIV - 1] from there on.
+#define NAK_CH 24                // steps per chunk
+#define NAK_PIV (3 * NAK_CH)
+__device__ __forceinline__ void nak_pivots(double* c) {
   if (threadIdx.x == 0) {
+    double v = __ddiv_rn(1.0, 4.0);
     int r = 0;
-    double v = 0.0;
-    if (m > 0) {
-      v = __ddiv_rn(1.0, 4.0);
-      c[0] = v;
-      for (r = 1; r < m; r++) {
-        double nv = __ddiv_rn(1.0, __dadd_rn(4.0, -v));
-        c[r] = nv;
-        if (nv == v) break;
-        v = nv;
-      }
+    for (; r < NAK_PIV; r++) {
+      c[r] = v;
+      const double nv = __ddiv_rn(1.0, __dadd_rn(4.0, -v));
+      if (nv == v) break;
+      v = nv;
     }
-    tail = v;
-    rc = r;
+    for (; r < NAK_PIV; r++) c[r] = v;
   }
   __syncthreads();
-  for (int r = rc + 1 + threadIdx.x; r < m; r += blockDim.x) c[r] = tail;
 }
 
 // Thomas-algorithm moments of the not-a-knot spline through n >= 4 samples with unit
@@ -288,16 +282,16 @@ __global__ void spline_recip_kernel(double* c, int m) {
 // M[i*ls] and dp[i*ls] (double).  The elimination multiplies by the shared pivots, so a
 // step is one add and one multiply.
 //
-// Each line is one thread and the recurrence is serial, with few lines in flight (one warp
-// per scheduler), so every instruction on a line's thread costs close to its full latency.
-// The work of a step that does not depend on the previous step -- its right-hand side
-// 6 (y[r+3] - 2 y[r+2] + y[r+1]), with the end corrections of the first and last step --
-// is done first by a fully parallel kernel (nak_rhs, one thread per line and step) into
-// the scratch array; the serial kernel (nak_solve) then reads it back a chunk ahead and
-// does only the add, the multiply and the store of each step, overwriting the right-hand
-// side with the eliminated value.  The arithmetic is the same, in the same order.
-#define NAK_CH 32
-#define NAK_SPIV 4096  // pivots staged in shared memory (32 KB)
+// Each line is one thread and the recurrence is serial: an add and a multiply, 16.7 cycles, a
+// step each way.  The work of a step that does not depend on the previous step -- its
+// right-hand side 6 (y[r+3] - 2 y[r+2] + y[r+1]), with the end corrections of the first and
+// last step -- is done first by a fully parallel kernel (nak_rhs, one thread per line and
+// step) into the scratch array; the serial kernel (nak_solve) reads it back two chunks of
+// steps ahead and does only the add, the multiply and the store of each step, overwriting the
+// right-hand side with the eliminated value.  The loads must not branch (clamped indices, not
+// predicates) and the pivots come from one array, so that nothing but the chain stands in a
+// chunk; CTAs of one warp spread the lines over the SMs.  1024 lines of 512: 92 us with
+// conditional loads and pivots from two memories, 29 us here (512 of 256: 48 and 16.5).
 template <typename TY>
 __device__ __forceinline__ double nak_m1(const TY* __restrict__ y, size_t ys) {
   return __dadd_rn(__dadd_rn((double)y[2 * ys], -__dmul_rn(2.0, (double)y[ys])), (double)y[0]);
@@ -320,100 +314,88 @@ __device__ __forceinline__ void nak_rhs(const TY* __restrict__ y, size_t ys, dou
   dp[(size_t)r * ls] = v;
 }
 template <typename TY>
-__device__ void nak_solve(const TY* __restrict__ y, size_t ys, size_t ls, double* __restrict__ M,
-                          const double* __restrict__ cp, const double* sp, int nsp, double* __restrict__ dp, int n) {
+__device__ void nak_solve(const TY* __restrict__ y, size_t ys, size_t ls, double* __restrict__ M, const double* c,
+                          double* __restrict__ dp, int n) {
 #define MV(i) M[(size_t)(i) * ls]
-#define PIV(r) ((r) < nsp ? sp[r] : cp[r])
   const double M1 = nak_m1<TY>(y, ys), Ml = nak_ml<TY>(y, ys, n);
   MV(1) = M1;
   MV(n - 2) = Ml;
   double M2 = Ml, M3 = Ml;  // M[2], M[n-3] for the end conditions
   const int m = n - 4;
   if (m > 0) {
-    double dprev = 0.0;
-    double rb[NAK_CH];
+    double b0[NAK_CH], b1[NAK_CH], b2[NAK_CH];
+    double prev = 0.0;
+    auto load = [&](double(&b)[NAK_CH], int r0) {
 #pragma unroll
-    for (int j = 0; j < NAK_CH; j++) rb[j] = j < m ? dp[(size_t)j * ls] : 0.0;
-#pragma unroll 1
-    for (int r0 = 0; r0 < m; r0 += NAK_CH) {
-      double rn[NAK_CH], cb[NAK_CH];
+      for (int j = 0; j < NAK_CH; j++) b[j] = dp[(size_t)min(r0 + j, m - 1) * ls];
+    };
+    auto eliminate = [&](const double(&b)[NAK_CH], int r0) {  // steps r0 .. r0 + NAK_CH - 1
+      const double* cc = c + min(r0, NAK_PIV - NAK_CH);
+      double* d = dp + (size_t)r0 * ls;
+      if (r0 + NAK_CH <= m) {
 #pragma unroll
-      for (int j = 0; j < NAK_CH; j++) {
-        const int r = r0 + NAK_CH + j;
-        rn[j] = r < m ? dp[(size_t)r * ls] : 0.0;  // the next chunk, in flight during this one
-        cb[j] = r0 + j < m ? PIV(r0 + j) : 0.0;
-      }
-      if (r0 + NAK_CH <= m) {  // a whole chunk: the chain alone
-#pragma unroll
-        for (int j = 0; j < NAK_CH; j++) {
-          const double d = (r0 + j == 0) ? __dmul_rn(rb[j], cb[j]) : __dmul_rn(__dadd_rn(rb[j], -dprev), cb[j]);
-          dp[(size_t)(r0 + j) * ls] = d;
-          dprev = d;
-        }
+        for (int j = 0; j < NAK_CH; j++) d[(size_t)j * ls] = prev = __dmul_rn(__dadd_rn(b[j], -prev), cc[j]);
       } else {
 #pragma unroll
-        for (int j = 0; j < NAK_CH; j++) {
-          if (r0 + j < m) {
-            const double d = (r0 + j == 0) ? __dmul_rn(rb[j], cb[j]) : __dmul_rn(__dadd_rn(rb[j], -dprev), cb[j]);
-            dp[(size_t)(r0 + j) * ls] = d;
-            dprev = d;
-          }
-        }
+        for (int j = 0; j < NAK_CH; j++)
+          if (r0 + j < m) d[(size_t)j * ls] = prev = __dmul_rn(__dadd_rn(b[j], -prev), cc[j]);
       }
-#pragma unroll
-      for (int j = 0; j < NAK_CH; j++) rb[j] = rn[j];
-    }
-    double next = dprev;
-    MV(m + 1) = next;
-    M3 = next;  // M[n-3] = M[m+1]
-    // back substitution, r = m-2 .. 0, in chunks loaded one ahead
-    double db[NAK_CH];
-#pragma unroll
-    for (int j = 0; j < NAK_CH; j++) db[j] = m - 2 - j >= 0 ? dp[(size_t)(m - 2 - j) * ls] : 0.0;
+    };
+    load(b0, 0);
+    load(b1, NAK_CH);
 #pragma unroll 1
-    for (int r1 = m - 2; r1 >= 0; r1 -= NAK_CH) {
-      double dn[NAK_CH], cb[NAK_CH];
+    for (int r = 0; r < m; r += 3 * NAK_CH) {
+      load(b2, r + 2 * NAK_CH);
+      eliminate(b0, r);
+      if (r + NAK_CH >= m) break;
+      load(b0, r + 3 * NAK_CH);
+      eliminate(b1, r + NAK_CH);
+      if (r + 2 * NAK_CH >= m) break;
+      load(b1, r + 4 * NAK_CH);
+      eliminate(b2, r + 2 * NAK_CH);
+    }
+    MV(m + 1) = prev;
+    M3 = prev;  // M[n-3] = M[m+1]
+    // back substitution, step r = m - 2 - t for t = 0, 1, ...
+    auto load_back = [&](double(&b)[NAK_CH], int t0) {
 #pragma unroll
-      for (int j = 0; j < NAK_CH; j++) {
-        const int r = r1 - NAK_CH - j;
-        dn[j] = r >= 0 ? dp[(size_t)r * ls] : 0.0;
-        cb[j] = r1 - j >= 0 ? PIV(r1 - j) : 0.0;
-      }
-      if (r1 - NAK_CH + 1 >= 0) {
+      for (int j = 0; j < NAK_CH; j++) b[j] = dp[(size_t)max(m - 2 - t0 - j, 0) * ls];
+    };
+    auto substitute = [&](const double(&b)[NAK_CH], int t0) {
+      const int lo = m - 1 - t0 - NAK_CH;  // the chunk's last step
+      double* o = M + (ptrdiff_t)(lo + 2) * (ptrdiff_t)ls;
+      if (lo >= 0) {
+        const double* cc = c + min(lo, NAK_PIV - NAK_CH);
 #pragma unroll
-        for (int j = 0; j < NAK_CH; j++) {
-          next = __dadd_rn(db[j], -__dmul_rn(cb[j], next));
-          MV(r1 - j + 2) = next;
-        }
+        for (int j = NAK_CH - 1; j >= 0; j--)
+          o[(size_t)j * ls] = prev = __dadd_rn(b[NAK_CH - 1 - j], -__dmul_rn(cc[j], prev));
       } else {
 #pragma unroll
-        for (int j = 0; j < NAK_CH; j++) {
-          if (r1 - j >= 0) {
-            next = __dadd_rn(db[j], -__dmul_rn(cb[j], next));
-            MV(r1 - j + 2) = next;
-          }
-        }
+        for (int j = NAK_CH - 1; j >= 0; j--)
+          if (lo + j >= 0) o[(size_t)j * ls] = prev = __dadd_rn(b[NAK_CH - 1 - j], -__dmul_rn(c[lo + j], prev));
       }
-#pragma unroll
-      for (int j = 0; j < NAK_CH; j++) db[j] = dn[j];
+    };
+    load_back(b0, 0);
+    load_back(b1, NAK_CH);
+#pragma unroll 1
+    for (int t = 0; t < m - 1; t += 3 * NAK_CH) {
+      load_back(b2, t + 2 * NAK_CH);
+      substitute(b0, t);
+      if (t + NAK_CH >= m - 1) break;
+      load_back(b0, t + 3 * NAK_CH);
+      substitute(b1, t + NAK_CH);
+      if (t + 2 * NAK_CH >= m - 1) break;
+      load_back(b1, t + 4 * NAK_CH);
+      substitute(b2, t + 2 * NAK_CH);
     }
-    M2 = next;  // M[2]
+    M2 = prev;  // M[2]
   } else {
     M2 = Ml;  // n == 4: M[2] = M[n-2], M[n-3] = M[1]
     M3 = M1;
   }
   MV(0) = __dadd_rn(__dmul_rn(2.0, M1), -M2);
   MV(n - 1) = __dadd_rn(__dmul_rn(2.0, Ml), -M3);
-#undef PIV
 #undef MV
-}
-
-// The first min(m, NAK_SPIV) pivots into shared memory (before any thread leaves).
-__device__ __forceinline__ int nak_stage_pivots(double* sp, const double* __restrict__ cp, int m) {
-  const int nsp = m < NAK_SPIV ? (m > 0 ? m : 0) : NAK_SPIV;
-  for (int i = threadIdx.x; i < nsp; i += blockDim.x) sp[i] = cp[i];
-  __syncthreads();
-  return nsp;
 }
 
 __device__ __forceinline__ double nak_eval(double yi, double yi1, double Mi, double Mi1, double t) {
@@ -436,7 +418,7 @@ __device__ __forceinline__ void fine_index(int j, int N, int n, int* i, double* 
 }
 
 // One or two planes (blockIdx of the plane dimension) upsampled by the same launches; plane
-// p's workspace arrays sit `pstride` doubles after plane 0's, and both use plane 0's pivots.
+// p's workspace arrays sit `pstride` doubles after plane 0's.
 struct SplinePlanes {
   const float* src[2];
   float* dst[2];
@@ -453,15 +435,14 @@ __global__ void __launch_bounds__(128) spline_ry_kernel(SplinePlanes P, int sp, 
 }
 
 // moments along y for each coarse column x, read straight from the float field (pitch sp)
-__global__ void __launch_bounds__(128) spline_my_kernel(SplinePlanes P, int sp, int h, int w, double* M, double* S,
-                                                        const double* __restrict__ cp) {
-  extern __shared__ double s_piv[];
-  const int nsp = nak_stage_pivots(s_piv, cp, h - 4);
+__global__ void __launch_bounds__(32) spline_my_kernel(SplinePlanes P, int sp, int h, int w, double* M, double* S) {
+  __shared__ double c[NAK_PIV];
+  nak_pivots(c);
   int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= w) return;
   const int q = blockIdx.y;
   // moments and scratch are laid out [i][x] with stride w
-  nak_solve<float>((q ? P.src[1] : P.src[0]) + x, (size_t)sp, (size_t)w, M + q * P.pstride + x, cp, s_piv, nsp,
+  nak_solve<float>((q ? P.src[1] : P.src[0]) + x, (size_t)sp, (size_t)w, M + q * P.pstride + x, c,
                    S + q * P.pstride + x, h);
 }
 
@@ -502,14 +483,14 @@ __global__ void __launch_bounds__(128) spline_rx_kernel(const double* __restrict
   nak_rhs<double>(Tt + o + Y, (size_t)H, dp + o + Y, (size_t)H, r, w);
 }
 
-__global__ void __launch_bounds__(128) spline_mx_kernel(const double* __restrict__ Tt, int w, int H, double* M,
-                                                        const double* __restrict__ cp, double* dp, size_t pstride) {
-  extern __shared__ double s_piv[];
-  const int nsp = nak_stage_pivots(s_piv, cp, w - 4);
+__global__ void __launch_bounds__(32) spline_mx_kernel(const double* __restrict__ Tt, int w, int H, double* M, double* dp,
+                                                       size_t pstride) {
+  __shared__ double c[NAK_PIV];
+  nak_pivots(c);
   int Y = blockIdx.x * blockDim.x + threadIdx.x;
   if (Y >= H) return;
   const size_t o = blockIdx.y * pstride;
-  nak_solve<double>(Tt + o + Y, (size_t)H, (size_t)H, M + o + Y, cp, s_piv, nsp, dp + o + Y, w);
+  nak_solve<double>(Tt + o + Y, (size_t)H, (size_t)H, M + o + Y, c, dp + o + Y, w);
 }
 
 // dst[Y][X] = row spline of fine row Y at fine column X (times scale).  The coarse
@@ -811,7 +792,6 @@ extern "C" size_t of_spline_workspace_size(int h, int w, int H, int W) {
   size_t a = (size_t)h * w, b = (size_t)H * w;
   s.take<double>(a);      // moments along y
   s.take<double>(a);      // Thomas scratch along y
-  s.take<double>((size_t)(h > w ? h : w));  // shared reciprocal pivots
   s.take<double>(b);      // column splines at the fine rows, layout [x][Y]
   s.take<double>(b);      // moments along x
   s.take<double>(b);      // Thomas scratch along x
@@ -825,21 +805,18 @@ static int spline_run(const SplinePlanes& P0, int np, int h, int w, int src_pitc
   Carver c(workspace, single);
   double* My = c.take<double>(a);
   double* Sy = c.take<double>(a);
-  double* piv = c.take<double>((size_t)(h > w ? h : w));
   double* Tt = c.take<double>(b);
   double* Mx = c.take<double>(b);
   double* Sx = c.take<double>(b);
   SplinePlanes P = P0;
   P.pstride = single / sizeof(double);
-  spline_recip_kernel<<<1, 256, 0, st>>>(piv, (h > w ? h : w) - 4);
-  auto piv_smem = [](int m) { return sizeof(double) * (size_t)(m < NAK_SPIV ? (m > 0 ? m : 0) : NAK_SPIV); };
   if (h > 4) spline_ry_kernel<<<dim3((w + 127) / 128, h - 4, np), 128, 0, st>>>(P, src_pitch, h, w, Sy);
-  spline_my_kernel<<<dim3((w + 127) / 128, np), 128, piv_smem(h - 4), st>>>(P, src_pitch, h, w, My, Sy, piv);
+  spline_my_kernel<<<dim3((w + 31) / 32, np), 32, 0, st>>>(P, src_pitch, h, w, My, Sy);
   spline_ey_kernel<<<dim3((w + 31) / 32, (H + 31) / 32, np), dim3(32, 8), 0, st>>>(P, src_pitch, My, Tt, h, w, H);
   if (w > 4) spline_rx_kernel<<<dim3((H + 127) / 128, w - 4, np), 128, 0, st>>>(Tt, w, H, Sx, P.pstride);
-  spline_mx_kernel<<<dim3((H + 127) / 128, np), 128, piv_smem(w - 4), st>>>(Tt, w, H, Mx, piv, Sx, P.pstride);
+  spline_mx_kernel<<<dim3((H + 31) / 32, np), 32, 0, st>>>(Tt, w, H, Mx, Sx, P.pstride);
   spline_ex_kernel<<<dim3((W + 31) / 32, (H + 31) / 32, np), dim3(32, 8), 0, st>>>(Tt, Mx, P, dst_pitch, w, H, W);
-  return check_launch("of_spline_upsample", 5 + (h > 4) + (w > 4));
+  return check_launch("of_spline_upsample", 4 + (h > 4) + (w > 4));
 }
 
 extern "C" int of_spline_upsample(const float* src, int h, int w, int src_pitch, float* dst, int H, int W,
