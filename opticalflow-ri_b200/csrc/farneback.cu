@@ -175,6 +175,12 @@ __global__ void __launch_bounds__(FBP_T) fb_polyexp_kernel(const float* __restri
 // outputs of one row with a register window along the row.  The arithmetic of every
 // output is the row kernel's, in the same order.  The moment rows are padded by one float
 // per 8 columns, so the 8-column segments of a warp's lanes fall in distinct banks.
+// What bounds it: the issue slots (240 instructions per pixel, three quarters of them adds
+// and multiply-adds) with few warps to hide the loads in front of them.  Moments 0 and 1 are
+// stored as pairs, whose sums along the row take the same taps in packed instructions (7 for 11
+// per tap), and 80 registers a thread let three CTAs share an SM.  Blurred / plain, us:
+// 1024 x 1024 22.8 / 15.5 -> 19.2 / 12.6, 2048 x 2048 57.7 / 43.3 -> 47.0 / 35.0; two CTAs per
+// SM 20.8 / 14.3 and 54.7 / 38.9.
 //
 // BLUR = true fuses the level's 3-tap frame blur in front (gaussianBlur with kh = 1 and
 // reflect-101 borders, :160-253, then the expansion of the blurred frame, as at the
@@ -187,7 +193,7 @@ __global__ void __launch_bounds__(FBP_T) fb_polyexp_kernel(const float* __restri
 constexpr int FBQ_OW = 240, FBQ_R = 8, FBQ_SEG = 8;
 __device__ __forceinline__ int fbq_col(int c) { return c + (c >> 3); }
 template <int N, bool BLUR>
-__global__ void __launch_bounds__(256) fb_polyexp_tile_kernel(const float* __restrict__ src, float* __restrict__ dst,
+__global__ void __launch_bounds__(256, 3) fb_polyexp_tile_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                                               int H, int W, int pitch, FbPoly P, int vec, float bg0,
                                                               float bg1) {
   constexpr int CW = FBQ_OW + 2 * N;          // columns that get vertical moments
@@ -195,13 +201,15 @@ __global__ void __launch_bounds__(256) fb_polyexp_tile_kernel(const float* __res
   constexpr int WIN = FBQ_SEG + 2 * N;
   constexpr int NR = FBQ_R + 2 * N;           // rows of the vertical window
   static_assert(CW + 2 <= 256 && NR * 256 <= 3 * FBQ_R * CWP, "blur rows must fit the moment storage");
-  __shared__ float mom[3][FBQ_R][CWP];
+  __shared__ __align__(16) float store[3 * FBQ_R * CWP];
+  float2 (*mom01)[CWP] = reinterpret_cast<float2 (*)[CWP]>(store);           // moments 0 and 1
+  float (*mom2)[CWP] = reinterpret_cast<float (*)[CWP]>(store + 2 * FBQ_R * CWP);
   const int x0 = blockIdx.x * FBQ_OW, y0 = blockIdx.y * FBQ_R, tx = threadIdx.x;
   float c[NR];
   if (BLUR) {
     // V(y, x) = g1 (src[y-1] + src[y+1]) + g0 src[y] at the window's clamped rows y, for
     // the columns clamp(x0 - N - 1 + j), j <= CW + 1
-    float (*vs)[256] = reinterpret_cast<float (*)[256]>(&mom[0][0][0]);
+    float (*vs)[256] = reinterpret_cast<float (*)[256]>(store);
     if (tx < CW + 2) {
       const float* col = src + clampi(x0 - N - 1 + tx, 0, W - 1);
       if (y0 - N - 1 >= 0 && y0 + FBQ_R + N < H) {  // rows y0-N-1 .. y0+R+N, all inside
@@ -248,64 +256,92 @@ __global__ void __launch_bounds__(256) fb_polyexp_tile_kernel(const float* __res
         r1 = __fmaf_rn(P.xg[k], __fsub_rn(t1, t0), r1);
         r2 = __fmaf_rn(P.xxg[k], __fadd_rn(t0, t1), r2);
       }
-      mom[0][r][fbq_col(tx)] = r0;
-      mom[1][r][fbq_col(tx)] = r1;
-      mom[2][r][fbq_col(tx)] = r2;
+      mom01[r][fbq_col(tx)] = make_float2(r0, r1);
+      mom2[r][fbq_col(tx)] = r2;
     }
   }
   __syncthreads();
   constexpr int NSEG = FBQ_OW / FBQ_SEG;
-  if (tx >= FBQ_R * NSEG) return;
   const int r = tx / NSEG, sg = tx - r * NSEG;
   const int y = y0 + r, xs = x0 + sg * FBQ_SEG;
-  if (y >= H || xs >= W) return;
-  // output column xs + i is moment column sg*8 + i + N; its window is sg*8 .. sg*8 + 7 + 2N
-  float a0[WIN], a1[WIN], a2[WIN];
-#pragma unroll
-  for (int q = 0; q < WIN; q++) {
-    const int cc = sg * (FBQ_SEG + 1) + q + (q >> 3);  // fbq_col(sg * 8 + q)
-    a0[q] = mom[0][r][cc];
-    a1[q] = mom[1][r][cc];
-    a2[q] = mom[2][r][cc];
-  }
+  const bool act = tx < FBQ_R * NSEG && y < H && xs < W;
   const size_t pl = (size_t)H * pitch;
   float o[5][FBQ_SEG];
+  if (act) {
+    // output column xs + i is moment column sg*8 + i + N; its window is sg*8 .. sg*8 + 7 + 2N
+    float2 a01[WIN];
+    float a2[WIN];
 #pragma unroll
-  for (int i = 0; i < FBQ_SEG; i++) {
-    const int t = i + N;
-    float b1 = __fmul_rn(P.g[0], a0[t]), b3 = __fmul_rn(P.g[0], a1[t]), b5 = __fmul_rn(P.g[0], a2[t]);
-    float b2 = 0.f, b4 = 0.f, b6 = 0.f;
-#pragma unroll
-    for (int k = 1; k <= N; k++) {
-      const float sp = __fadd_rn(a0[t + k], a0[t - k]), sm_ = __fsub_rn(a0[t + k], a0[t - k]);
-      b1 = __fmaf_rn(sp, P.g[k], b1);
-      b4 = __fmaf_rn(sp, P.xxg[k], b4);
-      b2 = __fmaf_rn(sm_, P.xg[k], b2);
-      b3 = __fmaf_rn(__fadd_rn(a1[t + k], a1[t - k]), P.g[k], b3);
-      b6 = __fmaf_rn(__fsub_rn(a1[t + k], a1[t - k]), P.xg[k], b6);
-      b5 = __fmaf_rn(__fadd_rn(a2[t + k], a2[t - k]), P.g[k], b5);
+    for (int q = 0; q < WIN; q++) {
+      const int cc = sg * (FBQ_SEG + 1) + q + (q >> 3);  // fbq_col(sg * 8 + q)
+      a01[q] = mom01[r][cc];
+      a2[q] = mom2[r][cc];
     }
-    o[0][i] = __fmul_rn(b3, P.ig[0]);
-    o[1][i] = __fmul_rn(b2, P.ig[0]);
-    o[2][i] = __fmaf_rn(b1, P.ig[1], __fmul_rn(b5, P.ig[2]));
-    o[3][i] = __fmaf_rn(b1, P.ig[1], __fmul_rn(b4, P.ig[2]));
-    o[4][i] = __fmul_rn(b6, P.ig[3]);
-  }
-  const size_t i0 = (size_t)y * pitch + xs;
-  if (vec && xs + FBQ_SEG <= W) {
 #pragma unroll
-    for (int p = 0; p < 5; p++) {
-      float4* d = reinterpret_cast<float4*>(dst + p * pl + i0);
-      d[0] = make_float4(o[p][0], o[p][1], o[p][2], o[p][3]);
-      d[1] = make_float4(o[p][4], o[p][5], o[p][6], o[p][7]);
-    }
-  } else {
+    for (int i = 0; i < FBQ_SEG; i++) {
+      const int t = i + N;
+      float2 b13 = __fmul2_rn(make_float2(P.g[0], P.g[0]), a01[t]), b26 = make_float2(0.f, 0.f);
+      float b5 = __fmul_rn(P.g[0], a2[t]), b4 = 0.f;
 #pragma unroll
-    for (int i = 0; i < FBQ_SEG; i++)
-      if (xs + i < W) {
-#pragma unroll
-        for (int p = 0; p < 5; p++) dst[p * pl + i0 + i] = o[p][i];
+      for (int k = 1; k <= N; k++) {
+        // sums and differences of moments 0 and 1; the product with -1 is exact
+        const float2 sp = __fadd2_rn(a01[t + k], a01[t - k]);
+        const float2 sm = __ffma2_rn(a01[t - k], make_float2(-1.f, -1.f), a01[t + k]);
+        b13 = __ffma2_rn(sp, make_float2(P.g[k], P.g[k]), b13);
+        b26 = __ffma2_rn(sm, make_float2(P.xg[k], P.xg[k]), b26);
+        b4 = __fmaf_rn(sp.x, P.xxg[k], b4);
+        b5 = __fmaf_rn(__fadd_rn(a2[t + k], a2[t - k]), P.g[k], b5);
       }
+      o[0][i] = __fmul_rn(b13.y, P.ig[0]);
+      o[1][i] = __fmul_rn(b26.x, P.ig[0]);
+      o[2][i] = __fmaf_rn(b13.x, P.ig[1], __fmul_rn(b5, P.ig[2]));
+      o[3][i] = __fmaf_rn(b13.x, P.ig[1], __fmul_rn(b4, P.ig[2]));
+      o[4][i] = __fmul_rn(b26.y, P.ig[3]);
+    }
+  }
+  if (vec) {  // 16-byte aligned rows
+    if (!act) return;
+    const size_t i0 = (size_t)y * pitch + xs;
+    if (xs + FBQ_SEG <= W) {
+#pragma unroll
+      for (int p = 0; p < 5; p++) {
+        float4* d = reinterpret_cast<float4*>(dst + p * pl + i0);
+        d[0] = make_float4(o[p][0], o[p][1], o[p][2], o[p][3]);
+        d[1] = make_float4(o[p][4], o[p][5], o[p][6], o[p][7]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < FBQ_SEG; i++)
+        if (xs + i < W) {
+#pragma unroll
+          for (int p = 0; p < 5; p++) dst[p * pl + i0 + i] = o[p][i];
+        }
+    }
+    return;
+  }
+  // Any other rows: through shared memory, so that a warp stores consecutive words (8 apart they
+  // cost a sector each: 719 x 1013, blurred, 31.0 us against 18.7).
+  static_assert(3 * FBQ_R * FBQ_OW <= 3 * FBQ_R * CWP, "three planes of the tile fit");
+#pragma unroll
+  for (int p0 = 0; p0 < 5; p0 += 3) {
+    __syncthreads();
+    if (act) {
+#pragma unroll
+      for (int p = p0; p < p0 + 3 && p < 5; p++) {
+        float4* d = reinterpret_cast<float4*>(store + ((p - p0) * FBQ_R + r) * FBQ_OW + sg * FBQ_SEG);
+        d[0] = make_float4(o[p][0], o[p][1], o[p][2], o[p][3]);
+        d[1] = make_float4(o[p][4], o[p][5], o[p][6], o[p][7]);
+      }
+    }
+    __syncthreads();
+    if (tx < FBQ_OW && x0 + tx < W) {
+#pragma unroll
+      for (int p = p0; p < p0 + 3 && p < 5; p++)
+#pragma unroll
+        for (int rr = 0; rr < FBQ_R; rr++)
+          if (y0 + rr < H)
+            dst[p * pl + (size_t)(y0 + rr) * pitch + x0 + tx] = store[((p - p0) * FBQ_R + rr) * FBQ_OW + tx];
+    }
   }
 }
 
