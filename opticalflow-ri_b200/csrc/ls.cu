@@ -319,10 +319,12 @@ constexpr int LB_PL = LB_RW * LB_CH;                         // floats per coeff
 constexpr int LB_COEF_BYTES = 8 * LB_CPLANE;
 // (u, v) ping-pong between two buffers.
 constexpr size_t LB_SMEM = LB_COEF_BYTES + 4 * LB_PLANE + 128 + 128;
-#ifndef OF_LS_PASS_WARPS
-#define OF_LS_PASS_WARPS 6
-#endif
-constexpr int LB_WARPS = OF_LS_PASS_WARPS;  // warps per CTA, each a band of the region's rows
+// Warps per CTA, each a band of the region's rows: 8 fill the 128 registers that two CTAs per SM
+// leave a thread (60 sweeps with 6, 8, 10: 2048 x 2048 2.47, 2.38, 2.81 ms; 719 x 1013 0.570,
+// 0.546, 0.649; 517 x 389 0.332, 0.335, 0.391).  Two rows of a band in one basic block are no
+// faster (0.346 at 517 x 389): a pass of a small image waits for its launch, its first copies and
+// the stop rule's sums.
+constexpr int LB_WARPS = 8;
 
 typedef float LbPlane[LB_RW];
 
