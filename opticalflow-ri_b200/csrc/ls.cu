@@ -92,10 +92,9 @@ struct Nb3 {
 #pragma unroll
       for (int c = 0; c < 3; c++) p[r][c] = P[(size_t)ys[r] * pitch + xs[c]];
   }
-  __device__ __forceinline__ float dy() const { return (float)dacc(dacc(0.0, p[0][1], -0.5), p[2][1], 0.5); }
-  __device__ __forceinline__ float dx() const { return (float)dacc(dacc(0.0, p[1][0], -0.5), p[1][2], 0.5); }
-  __device__ __forceinline__ float fy() const { return (float)dadd(dadd(0.0, p[0][1]), p[2][1]); }
-  __device__ __forceinline__ float fx() const { return (float)dadd(dadd(0.0, p[1][0]), p[1][2]); }
+  // two terms in float32: one rounding of the exact value, as the double sum's (see the sweep)
+  __device__ __forceinline__ float dy() const { return __fmaf_rn(p[2][1], 0.5f, __fmaf_rn(p[0][1], -0.5f, 0.0f)); }
+  __device__ __forceinline__ float dx() const { return __fmaf_rn(p[1][2], 0.5f, __fmaf_rn(p[1][0], -0.5f, 0.0f)); }
   __device__ __forceinline__ float m() const {
     return (float)dacc(dacc(dacc(dacc(0.0, p[0][0], 0.25), p[0][2], -0.25), p[2][0], -0.25), p[2][2], 0.25);
   }
@@ -122,18 +121,36 @@ __device__ __forceinline__ float hsum(const float* __restrict__ P, int y, int x,
   return (float)a;
 }
 
+// A divisor and its correctly rounded reciprocal; `ok`: in [2^-40, 2^40] either sign.
+struct LsDiv {
+  float d, y;
+  bool ok;
+};
+__device__ __forceinline__ LsDiv ls_divisor(float den) {
+  return {den, __frcp_rn(den), fabsf(den) >= 9.094947e-13f && fabsf(den) <= 1.0995116e12f};
+}
+
+// num / D.d, correctly rounded: two residual corrections of num * y (P. Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Develop. 34(1),
+// 1990), whose residuals are exact for |num| in [2^-60, 2^60]; a zero takes num * y.  The compiler's
+// divide calls a subroutine for a zero numerator, and black pixels are what particle images
+// mostly consist of.
+__device__ __forceinline__ float ls_div(float num, const LsDiv& D) {
+  const float q0 = __fmul_rn(num, D.y), a = fabsf(num);
+  float q = __fmaf_rn(__fmaf_rn(-q0, D.d, num), D.y, q0);
+  q = __fmaf_rn(__fmaf_rn(-q, D.d, num), D.y, q);
+  if (num == 0.0f) q = q0;
+  if (!(D.ok && (num == 0.0f || (a >= 8.6736174e-19f && a <= 1.1529215e18f)))) q = __fdiv_rn(num, D.d);
+  return q;
+}
+
 // Coefficient planes of pixel (y, x) (pitch-`pitch` index i) from its 3x3 neighbourhoods
 // of the normalised frame (n) and the temporal difference (e).
 __device__ __forceinline__ void ls_coef_at(const Nb3& n, const Nb3& e, int y, int x, int H, int W, float h,
                                            float* __restrict__ coef, size_t plane, size_t i) {
   float I = n.p[1][1];
-  int cnt = 0;
-#pragma unroll
-  for (int dy = -1; dy <= 1; dy++)
-#pragma unroll
-    for (int dx = -1; dx <= 1; dx++)
-      if (dy || dx) cnt += (y + dy >= 0 && y + dy < H && x + dx >= 0 && x + dx < W);
-  float cm = (float)cnt;
+  // neighbours inside the image
+  const float cm = (float)((1 + (y > 0) + (y < H - 1)) * (1 + (x > 0) + (x < W - 1)) - 1);
   coef[i] = __fmul_rn(I, n.dy());                 // IIx
   coef[plane + i] = __fmul_rn(I, n.dx());         // IIy
   coef[2 * plane + i] = __fmul_rn(I, I);          // II
@@ -145,9 +162,10 @@ __device__ __forceinline__ void ls_coef_at(const Nb3& n, const Nb3& e, int y, in
   float A22 = __fsub_rn(__fmul_rn(I, __fsub_rn(n.d2x(), twoI)), hc);
   float A12 = __fmul_rn(I, n.m());
   float det = __fsub_rn(__fmul_rn(A11, A22), __fmul_rn(A12, A12));
-  coef[5 * plane + i] = __fdiv_rn(A22, det);
-  coef[6 * plane + i] = __fdiv_rn(-A12, det);
-  coef[7 * plane + i] = __fdiv_rn(A11, det);
+  const LsDiv D = ls_divisor(det);
+  coef[5 * plane + i] = ls_div(A22, D);
+  coef[6 * plane + i] = ls_div(-A12, D);
+  coef[7 * plane + i] = ls_div(A11, D);
 }
 
 __global__ void ls_coef_kernel(const float* __restrict__ I1, const float* __restrict__ Et, float* __restrict__ coef,
@@ -160,43 +178,68 @@ __global__ void ls_coef_kernel(const float* __restrict__ I1, const float* __rest
   ls_coef_at(n, e, y, x, H, W, h, coef, plane, (size_t)y * pitch + x);
 }
 
-// The whole set-up of a solve after the frame maxima, in one pass: a 32 x 8 tile of the
+// The whole set-up of a solve after the frame maxima, in one pass: a 32 x 8 R tile of the
 // normalised frame I1 = im1 / max1 and of Et = im2 / max2 - I1 is formed in shared memory
 // with a 1-pixel halo of clamped ('nearest') coordinates -- exactly the neighbourhoods
 // Nb3::load reads -- then each pixel's coefficient planes are computed as in
 // ls_coef_kernel, and the initial field (V, U) is copied into ping-pong buffer 0.  The
 // normalised planes never reach global memory.
+// What bounds it: the latency of a tile's loads, hidden only by other CTAs, so a thread takes R
+// rows with their loads in flight together; then instructions (the divides, LsDiv).  R = 4 from
+// two CTAs per SM on, else 1, so that a small image still covers the chip: 1024 x 1024 14.8 -> 12.2
+// us, 2048 x 2048 74 -> 45.5 us (64.6 with one row; 34 at the bandwidth of a copy).
+template <int R>
 __global__ void __launch_bounds__(256) ls_prep_kernel(const float* __restrict__ a, const float* __restrict__ b,
                                                       int sp, const unsigned int* __restrict__ keys,
                                                       const float* __restrict__ V, const float* __restrict__ U,
                                                       float* __restrict__ coef, size_t plane, float* __restrict__ u0,
                                                       float* __restrict__ v0, int H, int W, int P, float h) {
-  __shared__ float t1[10][35], te[10][35];
-  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 8;
-  const float ma = key2f(keys[0]), mb = key2f(keys[1]);
-  for (int k = threadIdx.x; k < 10 * 34; k += 256) {
-    const int ly = k / 34, lx = k - ly * 34;
+  constexpr int TH = 8 * R, N = (TH + 2) * 34, NK = (N + 255) / 256;
+  __shared__ float t1[TH + 2][35], te[TH + 2][35];
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * TH;
+  const LsDiv ma = ls_divisor(key2f(keys[0])), mb = ls_divisor(key2f(keys[1]));
+  float va[NK], vb[NK];
+#pragma unroll
+  for (int j = 0; j < NK; j++) {
+    const int k = min((int)threadIdx.x + 256 * j, N - 1), ly = k / 34, lx = k - ly * 34;
     const size_t g = (size_t)clampi(y0 - 1 + ly, 0, H - 1) * sp + clampi(x0 - 1 + lx, 0, W - 1);
-    const float i1 = __fdiv_rn(a[g], ma), i2 = __fdiv_rn(b[g], mb);
+    va[j] = a[g];
+    vb[j] = b[g];
+  }
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, x = x0 + tx;
+  float fu[R], fv[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const size_t si = (size_t)min(y0 + ty + 8 * r, H - 1) * sp + min(x, W - 1);
+    fu[r] = U[si];
+    fv[r] = V[si];
+  }
+#pragma unroll
+  for (int j = 0; j < NK; j++) {
+    const int k = min((int)threadIdx.x + 256 * j, N - 1), ly = k / 34, lx = k - ly * 34;
+    const float i1 = ls_div(va[j], ma), i2 = ls_div(vb[j], mb);
     t1[ly][lx] = i1;
     te[ly][lx] = __fsub_rn(i2, i1);
   }
   __syncthreads();
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int x = x0 + tx, y = y0 + ty;
-  if (x >= W || y >= H) return;
-  Nb3 n, e;
+  if (x >= W) return;
 #pragma unroll
-  for (int r = 0; r < 3; r++)
+  for (int r = 0; r < R; r++) {
+    const int ly = ty + 8 * r, y = y0 + ly;
+    if (y >= H) return;
+    Nb3 n, e;
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      n.p[r][c] = t1[ty + r][tx + c];
-      e.p[r][c] = te[ty + r][tx + c];
-    }
-  const size_t i = (size_t)y * P + x, si = (size_t)y * sp + x;
-  ls_coef_at(n, e, y, x, H, W, h, coef, plane, i);
-  u0[i] = V[si];
-  v0[i] = U[si];
+    for (int rr = 0; rr < 3; rr++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        n.p[rr][c] = t1[ly + rr][tx + c];
+        e.p[rr][c] = te[ly + rr][tx + c];
+      }
+    const size_t i = (size_t)y * P + x;
+    ls_coef_at(n, e, y, x, H, W, h, coef, plane, i);
+    u0[i] = fv[r];
+    v0[i] = fu[r];
+  }
 }
 
 __device__ __forceinline__ double ls_err(const double* ss, int k, double inv_n) {
@@ -1138,8 +1181,12 @@ extern "C" int of_ls_solve_mode(const float* I0, const float* I1, float* U, floa
     ls_max_kernel<<<H < 4 * 148 ? H : 4 * 148, 256, 0, st>>>(I0, I1, H, W, pitch, vec, ctrl->maxkey);
   }
   dim3 rg((W + 255) / 256, H);
-  ls_prep_kernel<<<dim3((W + 31) / 32, (H + 7) / 8), 256, 0, st>>>(I0, I1, pitch, ctrl->maxkey, V, U, coef, N,
-                                                                 ub[0], vb[0], H, W, P, h);
+  if ((long long)((W + 31) / 32) * ((H + 31) / 32) >= 2 * kNumSMs)
+    ls_prep_kernel<4><<<dim3((W + 31) / 32, (H + 31) / 32), 256, 0, st>>>(I0, I1, pitch, ctrl->maxkey, V, U, coef, N,
+                                                                         ub[0], vb[0], H, W, P, h);
+  else
+    ls_prep_kernel<1><<<dim3((W + 31) / 32, (H + 7) / 8), 256, 0, st>>>(I0, I1, pitch, ctrl->maxkey, V, U, coef, N,
+                                                                       ub[0], vb[0], H, W, P, h);
   double inv_n = 1.0 / ((double)H * (double)W);
   dim3 pgrd((W + LB_TW - 1) / LB_TW, (H + LB_TH - 1) / LB_TH);
   const int tiles = (int)(pgrd.x * pgrd.y);
