@@ -50,3 +50,27 @@ def test_persistent_against_oracle(cuda_ok, h, w, pad, alpha):
     with np.errstate(all="ignore"):
         Uo, Vo, _ = O.hs_solve(*x, alpha, 19)
     assert same(U, Uo) and same(V, Vo)
+
+
+@pytest.mark.parametrize("h,w", [(256, 256), (300, 290), (401, 389)])
+def test_beside_other_work(cuda_ok, h, w):
+    """Another kernel holds all but 20 SMs for a few milliseconds when the solve starts: its CTAs do not
+    all run, so they take the work queue (or, if the holder is gone by then, their resident stages);
+    the result is the same."""
+    import torch
+    from ofb200 import ops
+    from test_gpu_hs_batch import _occupy
+    x = [torch.from_numpy(y).cuda() for y in frames(h, w, h)]
+    ref = ops.hs_solve(x[0], x[1], x[2].clone(), x[3].clone(), 21.0, 41, persistent=False)
+    side, main = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(main):  # sizes the stream's scratch
+        ops.hs_solve(x[0], x[1], x[2].clone(), x[3].clone(), 21.0, 41, persistent=True)
+        uv = x[2].clone(), x[3].clone()
+    torch.cuda.synchronize()
+    held = _occupy(torch, side, torch.cuda.get_device_properties(0).multi_processor_count - 20, 200 * 1024, 5_000_000)
+    with torch.cuda.stream(main):
+        U, V, err = ops.hs_solve(x[0], x[1], *uv, 21.0, 41, persistent=True)
+    torch.cuda.synchronize()
+    del held
+    assert torch.equal(U, ref[0]) and torch.equal(V, ref[1])
+    assert float(err) == pytest.approx(float(ref[2]), rel=1e-12)
