@@ -93,7 +93,7 @@ __device__ bool cv_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort
 // the compiler, and moving them to uniform registers costs more than a small MMA takes
 // (128 x 16 x 16 from shared memory: 171 cycles with index divisions, 53 unrolled, 39 converged).
 // In a training step of 16 crops of 128 x 128: the convolutions 564 -> 505 us, the weight
-// gradients 407 -> 355 us; both are now bound by the boxes they load, nine per pixel.
+// gradients 407 -> 355 us (before whole waves of splits, of_cnn_conv3x3_wgrad_tc); both are now bound by the boxes they load, nine per pixel.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t e;
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
 // CTAs split the pixel range; each adds its sums into dW with atomics, four input channels at
 // a time where the lanes run over output channels (scalar ones touch a sector each there).
 // The 12 layers of a training step of 16 crops of 128 x 128: 634 us with one tap per CTA and
-// scalar atomics, 355 us here.
+// scalar atomics, about 370 us here.
 constexpr int WT_KP = 64;  // pixels per K chunk
 constexpr int WT_STAGES = 4;
 
@@ -1395,11 +1395,19 @@ extern "C" int of_cnn_conv3x3_wgrad_tc(const void* x, int x_ctot, int x_coff, co
   size_t smem = 1024 + (size_t)p.stages * p.stage_bytes;
   size_t floor_smem = (size_t)p.tmem_cols * 448;  // resident CTAs never exceed 512 TMEM columns
   if (smem < floor_smem) smem = floor_smem;
-  // split the pixel chunks over one wave of resident CTAs
+  // split the pixel chunks over whole waves of resident CTAs
   const long long resident = 228 * 1024 / (long long)(smem + 2048);
   const long long tiles = 9LL / p.tg * tiles_mn;
   const int least = p.tg > 1 ? 4 : 8;
   long long ks = kNumSMs * (resident > 1 ? resident : 1) / tiles;
+  if (ks < 1) ks = 1;
+  // The tensor core truncates its running sums, so a sum's error grows with the chunks one CTA
+  // adds: whole waves until there are as many splits as four CTAs per SM with a tap each would
+  // make, eight chunks at least (16 x 256 x 256, 192 -> 64 channels: 500 accumulations in a chain
+  // there, 683 in one wave, 342 in two).
+  long long splits = (4LL * kNumSMs + 9 * tiles_mn - 1) / (9 * tiles_mn);
+  if (splits > p.nchunk / 8) splits = p.nchunk / 8;
+  if (ks < splits) ks *= (splits + ks - 1) / ks;
   if (ks > p.nchunk / least) ks = p.nchunk / least;
   if (ks < 1) ks = 1;
   p.chunks_per_cta = (int)((p.nchunk + ks - 1) / ks);
