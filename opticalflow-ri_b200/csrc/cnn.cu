@@ -93,7 +93,8 @@ __device__ bool cv_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort
 // the compiler, and moving them to uniform registers costs more than a small MMA takes
 // (128 x 16 x 16 from shared memory: 171 cycles with index divisions, 53 unrolled, 39 converged).
 // In a training step of 16 crops of 128 x 128: the convolutions 564 -> 505 us, the weight
-// gradients 407 -> 355 us (before whole waves of splits, of_cnn_conv3x3_wgrad_tc); both are now bound by the boxes they load, nine per pixel.
+// gradients 407 -> 355 us with one wave of splits (of_cnn_conv3x3_wgrad_tc takes whole waves); both
+// are now bound by the boxes they load, nine per pixel.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t e;
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
