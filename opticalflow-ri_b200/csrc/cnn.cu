@@ -66,20 +66,10 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 
-// Waits for phase `parity`; gives up after CV_WAIT_NS or when *abort becomes nonzero.
-__device__ bool cv_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
-  if (mbar_try(bar, parity)) return true;  // the clock is read only when there is something to wait for
-  unsigned long long t0 = globaltimer_ns();
-  while (!mbar_try(bar, parity)) {
-    if (abort && *abort) return false;
-    if (globaltimer_ns() - t0 > CV_WAIT_NS) return false;
-  }
-  return true;
-}
-
-// The same wait by a whole warp, with one result for all its lanes.
+// Waits for phase `parity`, a whole warp at once with one result for all its lanes; gives up
+// after CV_WAIT_NS or when *abort becomes nonzero.
 __device__ bool cv_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort) {
-  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;  // the clock is read only to wait
   unsigned long long t0 = globaltimer_ns();
   while (!__all_sync(0xffffffffu, mbar_try(bar, parity))) {
     const bool stop = (abort && *abort) || globaltimer_ns() - t0 > CV_WAIT_NS;
@@ -132,7 +122,10 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// 16 accumulator columns of the warp's 32 TMEM lanes.  Called by all 32 lanes; they converge here,
+// as both instructions demand.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
       "%15}, [%16];"
@@ -298,10 +291,12 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
     const int m = q * 32 + lane;
     const int mi = m / (p.bh * p.bw), mr = m - mi * (p.bh * p.bw);
     const int img = img0 + mi, py = y0 + mr / p.bw, px = x0 + mr % p.bw;
-    const bool ok = cv_wait(&accf, 0u, nullptr);
+    const bool ok = cv_wait_warp(&accf, 0u, nullptr);
     if (!ok) atomicOr(p.err, 8u);
     tc_fence_after();
-    if (ok && !abort_flag) cv_epilogue(p, tmem + ((uint32_t)(q * 32) << 16), ((size_t)img * p.H + py) * p.W + px, n0);
+    // one decision for the warp: cv_epilogue reads TMEM
+    if (__all_sync(0xffffffffu, ok && !abort_flag))
+      cv_epilogue(p, tmem + ((uint32_t)(q * 32) << 16), ((size_t)img * p.H + py) * p.W + px, n0);
   }
   tc_fence_before();
   __syncthreads();
@@ -457,33 +452,34 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
   } else {
     const int q = warp & 3;
     const int m = q * 32 + lane;
-    const bool ok = cv_wait(&accf, 0u, nullptr);
+    const bool ok = cv_wait_warp(&accf, 0u, nullptr);
     if (!ok) atomicOr(p.err, 8u);
     tc_fence_after();
     const int am = m0 + m;  // this thread's A-side channel
-    if (ok && !abort_flag && kiters > 0) {
+    // one decision for the warp, and no lane leaves a round early: the loads from TMEM are warp-wide
+    if (__all_sync(0xffffffffu, ok && !abort_flag && kiters > 0)) {
       const bool vec = p.a_is_dy && (p.cin & 3) == 0 && (reinterpret_cast<uintptr_t>(p.dw) & 15) == 0;
       for (int t = 0; t < p.tg; t++)
         for (int c = 0; c < p.nmma; c += 16) {
           uint32_t r[16];
           tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(t * p.cstride + c), r);
-          if (am >= p.a_ch) continue;
           float* dw = p.dw + (size_t)(tap0 + t) * p.cout * p.cin;
-          if (vec) {
+          if (am < p.a_ch) {
+            if (vec) {
 #pragma unroll
-            for (int j = 0; j < 16; j += 4)
-              if (n0 + c + j < p.b_ch)
-                atomicAdd(reinterpret_cast<float4*>(dw + (size_t)am * p.cin + n0 + c + j),
-                          make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                                      __uint_as_float(r[j + 3])));
-            continue;
-          }
+              for (int j = 0; j < 16; j += 4)
+                if (n0 + c + j < p.b_ch)
+                  atomicAdd(reinterpret_cast<float4*>(dw + (size_t)am * p.cin + n0 + c + j),
+                            make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
+                                        __uint_as_float(r[j + 3])));
+            } else {
 #pragma unroll
-          for (int j = 0; j < 16; j++) {
-            const int bn = n0 + c + j;
-            if (bn >= p.b_ch) break;
-            const int co = p.a_is_dy ? am : bn, ci = p.a_is_dy ? bn : am;
-            atomicAdd(&dw[(size_t)co * p.cin + ci], __uint_as_float(r[j]));
+              for (int j = 0; j < 16; j++) {
+                const int bn = n0 + c + j;
+                const int co = p.a_is_dy ? am : bn, ci = p.a_is_dy ? bn : am;
+                if (bn < p.b_ch) atomicAdd(&dw[(size_t)co * p.cin + ci], __uint_as_float(r[j]));
+              }
+            }
           }
         }
     }

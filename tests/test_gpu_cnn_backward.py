@@ -155,3 +155,25 @@ def test_weight_gradient_taps_per_cta(torch, n, H, W, cin, cout, coff):
     assert int(err.item()) == 0
     want = O.conv3x3_wgrad(_f(x)[..., coff:coff + cin], _f(dy)[..., :cout])
     assert np.max(np.abs(dw.cpu().numpy() - want)) <= 1e-4 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("n,H,W,cin,cout", [(10, 64, 64, 8, 40), (10, 64, 64, 6, 41), (10, 64, 64, 40, 8), (2, 64, 64, 72, 137),
+                                            (8, 16, 16, 129, 24), (2, 8, 8, 33, 33)])
+def test_weight_gradient_sides_ending_inside_a_warp(torch, n, H, W, cin, cout):
+    """Wider sides that no multiple of 32 channels makes: some lanes of a warp have no channel to add while
+    the warp goes on reading accumulators together.  Nothing outside dw is written; the tolerance is the
+    one above."""
+    import cnn_oracle as O
+    from ofb200._lib import call
+    rng = np.random.default_rng(cin + cout)
+    xct, dct = max(16, (cin + 7) // 8 * 8), max(16, (cout + 7) // 8 * 8)
+    x, dy = _bf(torch, rng, n, H, W, xct), _bf(torch, rng, n, H, W, dct)
+    size = 9 * cout * cin
+    buf = torch.zeros(size + 64, dtype=torch.float32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    call("of_cnn_conv3x3_wgrad_tc", _P(x), xct, 0, _P(dy), dct, 0, n, H, W, cin, cout, _P(buf), _P(err), _sp())
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0 and not buf[size:].any()
+    want = O.conv3x3_wgrad(_f(x)[..., :cin], _f(dy)[..., :cout])
+    got = buf[:size].cpu().numpy().reshape(9, cout, cin)
+    assert np.max(np.abs(got - want)) <= 1e-4 * np.max(np.abs(want))
