@@ -77,8 +77,8 @@ __global__ void hs_sweep_kernel(const float* __restrict__ fx, const float* __res
 //
 // What bounds it: the issue slots (65 instructions per cell update, 16 of them float64
 // multiply-adds) at 50 % busy, and the latency of the pass's loads and barriers behind two
-// CTAs per SM (128 registers a thread).  600 sweeps, one pair alone: 256 x 256 2.75 -> 1.19 ms,
-// 512 x 512 3.3 -> 1.25 ms; 100 sweeps of 2048 x 2048 3.96 -> 2.27 ms (106 -> 185 G cell updates
+// CTAs per SM (128 registers a thread).  600 sweeps, one pair alone: 256 x 256 2.75 -> 1.21 ms,
+// 512 x 512 3.1 -> 1.27 ms; 100 sweeps of 2048 x 2048 3.96 -> 2.26 ms (106 -> 186 G cell updates
 // per second) against the column walk with one cell per thread and row it replaces.  4 x 4
 // blocks spill at 12 warps per SM (113 G/s), a 64 x 64 region in one CTA of 512 threads does
 // less halo work but leaves its loads exposed (164 G/s).
@@ -127,7 +127,10 @@ struct HbPass {
 
 using HbBlock = HrBlock<HB_BX, HB_BY>;
 
-__device__ __forceinline__ void hb_load_uv(HbBlock& K, const HbPass& P, int gy0, int gx0, bool inside) {
+// Loads the block's cells.  Returns whether those of two corners are so small (and not zero) that
+// numerators made of such may leave the refined quotient's range: a guess, from 4 of 16 values, since
+// the flow that diffuses into a region is of one size over a block.
+__device__ __forceinline__ bool hb_load_uv(HbBlock& K, const HbPass& P, int gy0, int gx0, bool inside) {
   float2 u[HB_BY], v[HB_BY];
   hb_load(u, P.U, gy0, gx0, P.H, P.W, P.pitch, inside);
   hb_load(v, P.V, gy0, gx0, P.H, P.W, P.pitch, inside);
@@ -136,76 +139,137 @@ __device__ __forceinline__ void hb_load_uv(HbBlock& K, const HbPass& P, int gy0,
     K.u[j][0] = u[j].x; K.u[j][1] = u[j].y;
     K.v[j][0] = v[j].x; K.v[j][1] = v[j].y;
   }
+  auto key = [](float x) { return 2u * __float_as_uint(x) - 1u; };
+  return min(min(key(u[0].x), key(v[0].x)), min(key(u[HB_BY - 1].y), key(v[HB_BY - 1].y))) < HR_LO;
 }
 
-// The sweeps of a pass; on return the CTA's last sweep is in the blocks only.
-template <bool RAG, bool DIV>
+// The sweeps of a pass from the cells that the CTA's blocks have published in the first buffer; on
+// return the last sweep's are in the blocks only.
+template <bool RAG, int Q>
 __device__ __forceinline__ void hb_sweeps(HbBlock& K, const HbPass& P, double2* sm, bool in, int r0, int c0,
                                           const HrWin& win) {
-  if (in) hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, sm, r0, c0);
-  __syncthreads();
   // a warp whose rows no later sweep reads (the outermost, in the last sweep) sits out
   auto needed = [&](int k) { return in && r0 + HB_BY > 1 + k && r0 < HB_RH - 1 - k; };
 #pragma unroll 1
   for (int s = 0; s < P.nsw; s += 2) {
     double2* const b0 = sm;
     double2* const b1 = sm + HB_RW * HB_RH;
-    if (needed(s)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, RAG, DIV>(K, b0, r0, c0, win);
+    if (needed(s)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, RAG, Q>(K, b0, r0, c0, win);
     if (s + 1 >= P.nsw) break;
     if (needed(s)) hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, b1, r0, c0);
     __syncthreads();
-    if (needed(s + 1)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, RAG, DIV>(K, b1, r0, c0, win);
+    if (needed(s + 1)) hr_sweep<HB_RW, HB_RH, HB_BX, HB_BY, RAG, Q>(K, b1, r0, c0, win);
     if (s + 2 >= P.nsw) break;
     if (needed(s + 1)) hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, b0, r0, c0);
     __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(HbGeom::NT, 2) hs_pass_kernel(const HbPass P) {
+// The CTA's region and the thread's block in it.
+struct HbPos {
+  int x0, y0;    // image position of region cell (0, 0)
+  int c0, r0;    // the block's first region cell
+  int gx0, gy0;  // its image position
+  bool in;       // the block has cells in the image
+  bool inside;   // the whole region is in the image, with 8-byte aligned rows
+};
+
+__device__ __forceinline__ HbPos hb_pos(const HbPass& P) {
+  HbPos p;
+  p.x0 = blockIdx.x * HB_TW - HB_T;
+  p.y0 = blockIdx.y * HB_TH - HB_T;
+  p.c0 = ((int)threadIdx.x % HbGeom::NX) * HB_BX;
+  p.r0 = ((int)threadIdx.x / HbGeom::NX) * HB_BY;
+  p.gx0 = p.x0 + p.c0;
+  p.gy0 = p.y0 + p.r0;
+  p.in = p.gx0 + HB_BX > 0 && p.gy0 + HB_BY > 0 && p.gx0 < P.W && p.gy0 < P.H;
+  p.inside = !(p.x0 < 0 || p.y0 < 0 || p.x0 + HB_RW > P.W || p.y0 + HB_RH > P.H) && P.vec;
+  return p;
+}
+
+// Loads the block's derivatives; the result is hr_init_den's.
+__device__ __forceinline__ bool hb_load_g(HbBlock& K, const HbPass& P, const HbPos& p) {
+  float2 a[HB_BY], b[HB_BY], c[HB_BY];
+  hb_load(a, P.fx, p.gy0, p.gx0, P.H, P.W, P.pitch, p.inside);
+  hb_load(b, P.fy, p.gy0, p.gx0, P.H, P.W, P.pitch, p.inside);
+  hb_load(c, P.ft, p.gy0, p.gx0, P.H, P.W, P.pitch, p.inside);
+#pragma unroll
+  for (int j = 0; j < HB_BY; j++) {
+    K.g[j][0] = make_float2(a[j].x, b[j].x);
+    K.g[j][1] = make_float2(a[j].y, b[j].y);
+    K.gt[j][0] = c[j].x; K.gt[j][1] = c[j].y;
+  }
+  return hr_init_den(K, P.a2, P.one);
+}
+
+__device__ __forceinline__ void hb_store(const HbBlock& K, const HbPass& P, const HbPos& p) {
+  if (p.in && p.c0 >= HB_T && p.c0 < HB_T + HB_TW && p.r0 >= HB_T && p.r0 < HB_T + HB_TH) {
+#pragma unroll
+    for (int j = 0; j < HB_BY; j++) {
+      hb_store2(P.Un, K.u[j], p.gy0 + j, p.gx0, P.H, P.W, P.pitch, P.vec);
+      hb_store2(P.Vn, K.v[j], p.gy0 + j, p.gx0, P.H, P.W, P.pitch, P.vec);
+    }
+  }
+}
+
+extern __shared__ __align__(16) double2 hb_sm[];
+
+// The CTA's pass with the wide quotient, or with the divide where that one's range fails too.  A
+// function of its own that starts from the image: in the kernel its registers cost every pass 1 to
+// 2 % from 1024 x 1024 on.  512 x 512, 600 sweeps, one half the same texture in both frames: 1.93 ms
+// (4.50 where such passes were run again with the divide, 1.27 without tiny numerators).
+__device__ __noinline__ void hb_pass_wide(const HbPass& P) {
+  const HbPos p = hb_pos(P);
+  const HrWin win = hr_window<HB_RW, HB_RH, HB_BX, HB_BY>(p.r0, p.c0, p.gy0, p.gx0, P.H, P.W);
+  HbBlock K;
+  bool ok = true;
+  if (p.in) {
+    ok = hb_load_g(K, P, p);
+    hb_load_uv(K, P, p.gy0, p.gx0, p.inside);
+    hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, hb_sm, p.r0, p.c0);
+  }
+  bool bad = __syncthreads_or(p.in && !ok);
+  if (!bad) {
+    hb_sweeps<true, HR_WIDE>(K, P, hb_sm, p.in, p.r0, p.c0, win);
+    bad = __syncthreads_or(p.in && !hr_in_range(K, HR_WIDE));
+    if (bad) {
+      if (p.in) {
+        hb_load_uv(K, P, p.gy0, p.gx0, p.inside);
+        hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, hb_sm, p.r0, p.c0);
+      }
+      __syncthreads();
+    }
+  }
+  if (bad) hb_sweeps<true, HR_DIVIDE>(K, P, hb_sm, p.in, p.r0, p.c0, win);
+  hb_store(K, P, p);
+}
+
+__global__ void __launch_bounds__(HbGeom::NT, 2) hs_pass_kernel(const __grid_constant__ HbPass P) {
   // passes after the first are programmatic dependents of the pass before them: they take the
   // SM slots its tail frees and load the derivatives, which do not change during a solve
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  extern __shared__ __align__(16) double2 hb_sm[];
-  const int x0 = blockIdx.x * HB_TW - HB_T, y0 = blockIdx.y * HB_TH - HB_T;  // image position of region cell (0, 0)
-  const int c0 = ((int)threadIdx.x % HbGeom::NX) * HB_BX, r0 = ((int)threadIdx.x / HbGeom::NX) * HB_BY;
-  const int gx0 = x0 + c0, gy0 = y0 + r0;
-  const bool in = gx0 + HB_BX > 0 && gy0 + HB_BY > 0 && gx0 < P.W && gy0 < P.H;  // the block has cells in the image
+  const HbPos p = hb_pos(P);
   HbBlock K;
-  const bool edge = x0 < 0 || y0 < 0 || x0 + HB_RW > P.W || y0 + HB_RH > P.H, inside = !edge && P.vec;
-  bool ok = true;
-  if (in) {
-    float2 a[HB_BY], b[HB_BY], c[HB_BY];
-    hb_load(a, P.fx, gy0, gx0, P.H, P.W, P.pitch, inside);
-    hb_load(b, P.fy, gy0, gx0, P.H, P.W, P.pitch, inside);
-    hb_load(c, P.ft, gy0, gx0, P.H, P.W, P.pitch, inside);
-#pragma unroll
-    for (int j = 0; j < HB_BY; j++) {
-      K.g[j][0] = make_float2(a[j].x, b[j].x);
-      K.g[j][1] = make_float2(a[j].y, b[j].y);
-      K.gt[j][0] = c[j].x; K.gt[j][1] = c[j].y;
-    }
-    ok = hr_init_den(K, P.a2, P.one);
-  }
+  bool wide = p.in && !hb_load_g(K, P, p);
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (in) hb_load_uv(K, P, gy0, gx0, inside);
-  const HrWin win = hr_window<HB_RW, HB_RH, HB_BX, HB_BY>(r0, c0, gy0, gx0, P.H, P.W);
-  // the region holds blocks that the image ends inside of
-  const bool rag = (P.W % HB_BX && x0 + HB_RW > P.W) || (P.H % HB_BY && y0 + HB_RH > P.H);
-  if (rag)
-    hb_sweeps<true, false>(K, P, hb_sm, in, r0, c0, win);
-  else
-    hb_sweeps<false, false>(K, P, hb_sm, in, r0, c0, win);
-  if (__syncthreads_or(in && !(ok && hr_in_range(K)))) {  // rare: see hr_row
-    if (in) hb_load_uv(K, P, gy0, gx0, inside);
-    hb_sweeps<true, true>(K, P, hb_sm, in, r0, c0, win);
+  if (p.in) {
+    wide = hb_load_uv(K, P, p.gy0, p.gx0, p.inside) || wide;
+    hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, hb_sm, p.r0, p.c0);
   }
-  if (in && c0 >= HB_T && c0 < HB_T + HB_TW && r0 >= HB_T && r0 < HB_T + HB_TH) {
-#pragma unroll
-    for (int j = 0; j < HB_BY; j++) {
-      hb_store2(P.Un, K.u[j], gy0 + j, gx0, P.H, P.W, P.pitch, P.vec);
-      hb_store2(P.Vn, K.v[j], gy0 + j, gx0, P.H, P.W, P.pitch, P.vec);
+  if (!__syncthreads_or(wide)) {
+    const HrWin win = hr_window<HB_RW, HB_RH, HB_BX, HB_BY>(p.r0, p.c0, p.gy0, p.gx0, P.H, P.W);
+    // the region holds blocks that the image ends inside of
+    const bool rag = (P.W % HB_BX && p.x0 + HB_RW > P.W) || (P.H % HB_BY && p.y0 + HB_RH > P.H);
+    if (rag)
+      hb_sweeps<true, HR_REFINED>(K, P, hb_sm, p.in, p.r0, p.c0, win);
+    else
+      hb_sweeps<false, HR_REFINED>(K, P, hb_sm, p.in, p.r0, p.c0, win);
+    if (!__syncthreads_or(p.in && !hr_in_range(K, HR_REFINED))) {
+      hb_store(K, P, p);
+      return;
     }
   }
+  hb_pass_wide(P);
 }
 
 __global__ void copy2_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ ao,

@@ -541,7 +541,8 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2)
 // 600 sweeps, square images, before (counters, or their work queue) and now, ms:
 //   48 x 32  to 148 tiles of 32 x 16:  96 0.65 -> 0.51, 192 0.65 -> 0.53, 256 0.80 -> 0.56
 //   64 x 32  to 148 tiles of 48 x 16:  304 1.2 -> 0.66
-//   64 x 48  to 148 tiles of 48 x 32:  384 1.70 -> 0.99, 448 2.30 -> 1.02
+//   64 x 48  to 148 tiles of 48 x 32:  384 1.70 -> 0.99, 448 2.30 -> 0.95
+// With one half the same texture in both frames (hr_row's HR_WIDE): 96 0.56, 256 0.60, 448 1.10.
 // Larger images: one launch per pass (hs.cu), 512 2.98 -> 1.23.
 template <int RW_, int RH_, int T_, int BX_, int BY_>
 struct HrShape {
@@ -580,7 +581,7 @@ __device__ __forceinline__ HrCell hr_get(const HrCell* p) {
 }
 
 // nsw sweeps from the blocks' cells; the last one's results are in the blocks only.
-template <class S, bool RAG, bool DIV>
+template <class S, bool RAG, int Q>
 __device__ __forceinline__ void hr_stage(typename S::K& K, double2* sm, bool in, int r0, int c0, const HrWin& win,
                                          int nsw) {
   // a block whose rows no later sweep reads sits out
@@ -591,11 +592,11 @@ __device__ __forceinline__ void hr_stage(typename S::K& K, double2* sm, bool in,
     double2* const b1 = sm + S::RW * S::RH;
     if (s == 0 ? in : needed(s - 1)) hr_publish<S::RW, S::RH, S::BX, S::BY>(K, b0, r0, c0);
     __syncthreads();
-    if (needed(s)) hr_sweep<S::RW, S::RH, S::BX, S::BY, RAG, DIV>(K, b0, r0, c0, win);
+    if (needed(s)) hr_sweep<S::RW, S::RH, S::BX, S::BY, RAG, Q>(K, b0, r0, c0, win);
     if (s + 1 >= nsw) break;
     if (needed(s)) hr_publish<S::RW, S::RH, S::BX, S::BY>(K, b1, r0, c0);
     __syncthreads();
-    if (needed(s + 1)) hr_sweep<S::RW, S::RH, S::BX, S::BY, RAG, DIV>(K, b1, r0, c0, win);
+    if (needed(s + 1)) hr_sweep<S::RW, S::RH, S::BX, S::BY, RAG, Q>(K, b1, r0, c0, win);
   }
 }
 
@@ -616,7 +617,7 @@ __device__ __forceinline__ void hrb_body(const HsqPair& P, HrCell* __restrict__ 
   float2* const start = reinterpret_cast<float2*>(hr_sm + 2 * S::RW * S::RH) + threadIdx.x;
   typename S::K K;
   unsigned int own = 0, ring = 0;  // the block's cells in the image, owned by this CTA or by others (bit j * BX + i)
-  bool fin = true, ok = true;
+  bool fin = true;
 #pragma unroll
   for (int j = 0; j < S::BY; j++)
 #pragma unroll
@@ -642,8 +643,8 @@ __device__ __forceinline__ void hrb_body(const HsqPair& P, HrCell* __restrict__ 
       }
     }
   if (__syncthreads_or(!fin) && threadIdx.x == 0) atomicOr(status, OF_ST_NONFINITE_INPUT);
-  ok = hr_init_den(K, P.a2, one) || !in;
-  const bool den_ok = ok;
+  const bool den_bad = __syncthreads_or(!hr_init_den(K, P.a2, one) && in);
+  int quot = den_bad ? HR_DIVIDE : HR_REFINED;  // the quotient that the next stage begins with (hr_row)
   const int np = (niter + S::T - 1) / S::T;
   bool gave_up = false;
   for (int p = 0; p < np; p++) {
@@ -671,26 +672,37 @@ __device__ __forceinline__ void hrb_body(const HsqPair& P, HrCell* __restrict__ 
         }
       }
     }
-    // the stage's first values, for a repeat with DIV
+    const int nsw = min(S::T, niter - p * S::T);
+    // the stage's first values, for a repeat
 #pragma unroll
     for (int b = 0; b < S::BX * S::BY; b++)
       start[b * S::NT] = make_float2((float)K.u[b / S::BX][b % S::BX], (float)K.v[b / S::BX][b % S::BX]);
-    const int nsw = min(S::T, niter - p * S::T);
-    if (rag)
-      hr_stage<S, true, false>(K, hr_sm, in, r0, c0, win, nsw);
-    else
-      hr_stage<S, false, false>(K, hr_sm, in, r0, c0, win, nsw);
-    if (__syncthreads_or(in && !(den_ok && hr_in_range(K)))) {  // rare: see hr_row
+    while (true) {
+      if (quot == HR_DIVIDE) {
+        hr_stage<S, true, HR_DIVIDE>(K, hr_sm, in, r0, c0, win, nsw);
+        break;
+      }
+      if (quot == HR_WIDE)
+        hr_stage<S, true, HR_WIDE>(K, hr_sm, in, r0, c0, win, nsw);
+      else if (rag)
+        hr_stage<S, true, HR_REFINED>(K, hr_sm, in, r0, c0, win, nsw);
+      else
+        hr_stage<S, false, HR_REFINED>(K, hr_sm, in, r0, c0, win, nsw);
+      if (!__syncthreads_or(in && !hr_in_range(K, quot))) break;
+      quot = __syncthreads_or(in && !hr_in_range(K, HR_WIDE)) ? HR_DIVIDE : HR_WIDE;
 #pragma unroll
       for (int b = 0; b < S::BX * S::BY; b++) {
         const float2 s = start[b * S::NT];
         K.u[b / S::BX][b % S::BX] = (double)s.x;
         K.v[b / S::BX][b % S::BX] = (double)s.y;
       }
-      hr_stage<S, true, true>(K, hr_sm, in, r0, c0, win, nsw);
-      K.lo = 0xffffffffu;
-      K.hi = 0.f;
-      __syncthreads();
+      hr_reset_range(K);
+    }
+    if (quot != HR_REFINED) {  // the next stage begins with what this one's numerators allow
+      const bool wide = __syncthreads_or(in && !hr_in_range(K, HR_REFINED));
+      const bool divide = __syncthreads_or(in && !hr_in_range(K, HR_WIDE)) || den_bad;
+      quot = divide ? HR_DIVIDE : wide ? HR_WIDE : HR_REFINED;
+      hr_reset_range(K);
     }
     HrCell* dst = halo + (size_t)(p & 1) * cells;
     fin = true;

@@ -214,12 +214,12 @@ struct HrBlock {
   float hi;            // and largest |num|
 };
 
-// Where the quotient by refinement (hr_row) is the correctly rounded one: for den in [2^-40,
-// 2^40] and |num| in [2^-60, 2^60] no intermediate leaves the normal range and the residuals
-// are exact (multiples of 2^-46 |num|; the quotients are at least 2^-100); and for num = +0,
+// Where the quotient by refinement (hr_div) is the correctly rounded one: for den in [2^-40,
+// 2^40] and |num| in [2^-80, 2^60] no intermediate leaves the normal range and the residuals
+// are exact (multiples of 2^-47 |num|; the quotients are at least 2^-120); and for num = +0,
 // which is what a zero numerator is unless gt is -0.
-constexpr float HR_DEN = 1.0995116e12f, HR_NUM = 1.1529215e18f;
-constexpr unsigned HR_LO = 2u * 0x21800000u - 1u;  // 2^-60
+constexpr float HR_DEN = 0x1p40f, HR_NUM = 0x1p60f;
+constexpr unsigned HR_LO = 2u * 0x17800000u - 1u;  // 2^-80
 
 __device__ __forceinline__ float hr_max_nan(float a, float b) {  // NaN if either is
   float r;
@@ -232,13 +232,20 @@ __device__ __forceinline__ float hr_den(float2 g, float a2) {
   return __fadd_rn(__fadd_rn(a2, q.x), q.y);
 }
 
+enum HrQuot { HR_REFINED, HR_WIDE, HR_DIVIDE };  // see hr_row
+
+template <int BX, int BY>
+__device__ __forceinline__ void hr_reset_range(HrBlock<BX, BY>& K) {
+  K.lo = 0xffffffffu;
+  K.hi = 0.f;
+}
+
 // The block's reciprocals; false when a denominator or gt is outside the ranges above.
 template <int BX, int BY>
 __device__ __forceinline__ bool hr_init_den(HrBlock<BX, BY>& K, float a2, float one) {
   K.a2 = a2;
   K.one = one;
-  K.lo = 0xffffffffu;
-  K.hi = 0.f;
+  hr_reset_range(K);
   bool ok = true;
 #pragma unroll
   for (int j = 0; j < BY; j++)
@@ -252,20 +259,48 @@ __device__ __forceinline__ bool hr_init_den(HrBlock<BX, BY>& K, float a2, float 
   return ok;
 }
 
-// Whether every quotient since hr_init_den was in range.
+// Whether every numerator since the last reset was in the range of quotient q (HR_REFINED or HR_WIDE).
 template <int BX, int BY>
-__device__ __forceinline__ bool hr_in_range(const HrBlock<BX, BY>& K) {
-  return K.lo >= HR_LO && K.hi <= HR_NUM;
+__device__ __forceinline__ bool hr_in_range(const HrBlock<BX, BY>& K, int q) {
+  return (K.lo >= HR_LO || q == HR_WIDE) && K.hi <= HR_NUM;
+}
+
+// num / den by two residual corrections of num * y, y = 1 / den correctly rounded; the last is
+// correctly rounded (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Develop. 34(1), 1990) for operands in the ranges above.
+__device__ __forceinline__ float hr_div(float num, float den, float y) {
+  float q = __fmul_rn(num, y);
+  q = __fmaf_rn(__fmaf_rn(-q, den, num), y, q);
+  return __fmaf_rn(__fmaf_rn(-q, den, num), y, q);
+}
+
+// The same for |num| down to the smallest subnormal.  A numerator below 2^-60 is divided at 2^64
+// times its size, which is exact.  So is the way back unless the quotient is subnormal: there it is a
+// second rounding, wrong where the first one's result lies midway between two subnormal numbers and
+// its residual points to the other one.  No branch, and no divide, which is slow for such operands.
+__device__ __forceinline__ float hr_div_wide(float num, float den, float y) {
+  const bool tiny = fabsf(num) < 0x1p-60f;
+  const float up = tiny ? 0x1p64f : 1.f, down = tiny ? 0x1p-64f : 1.f;
+  const float n = __fmul_rn(num, up), q = hr_div(n, den, y), der = __fmul_rn(q, down);
+  const float e = __fmaf_rn(der, up, -q), r = __fmaf_rn(-q, den, n);  // exact; e: what the way back added
+  const float fix = e == 0x1p-86f && r < 0.f ? -0x1p-149f : e == -0x1p-86f && r > 0.f ? 0x1p-149f : 0.f;
+  return fix != 0.f ? __fadd_rn(der, fix) : der;
 }
 
 // The update of a block's row j from the old window rows U (above), C, D (below):
 // hs_sweep_kernel's arithmetic, the 8 neighbours summed in its order; the results replace the
-// block's cells.  DIV: the quotient by __fdiv_rn; else by two residual corrections of num * y,
-// y the correctly rounded reciprocal, the last of which is correctly rounded (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Develop. 34(1), 1990) for numerators in range.  The range is only recorded here: one
-// check per pass, and a CTA that fails it repeats the pass with DIV.
-template <int BX, int BY, bool DIV>
+// block's cells.  The quotient by Q; the range of the numerators is only recorded here, for one check
+// per pass, and a CTA that fails it repeats the pass with the next Q:
+//   HR_REFINED  hr_div
+//   HR_WIDE     hr_div_wide.  Tiny numerators are common where both frames show the same texture:
+//               the flow that diffuses in shrinks by a factor of 6 to 12 a cell, down to the
+//               subnormal numbers.  So a CTA that has reason to expect them (its last pass, or the
+//               flow it starts from) begins with this one.  256 x 256, 600 sweeps, one half the
+//               same texture in both frames: 0.60 ms (0.54 where no numerator is tiny); every such
+//               pass run again with the divide 1.99, with this one's scaling but the divide for
+//               subnormal quotients 1.76, in float64 0.60 but 5 % on every pass of hs.cu in spills.
+//   HR_DIVIDE   __fdiv_rn, for all operands.
+template <int BX, int BY, int Q>
 __device__ __forceinline__ void hr_row(HrBlock<BX, BY>& K, int j, const HrRow<BX>& U, const HrRow<BX>& C,
                                        const HrRow<BX>& D) {
   const double wc = (double)(1.0f / 12.0f), we = (double)(1.0f / 6.0f);
@@ -288,17 +323,11 @@ __device__ __forceinline__ void hr_row(HrBlock<BX, BY>& K, int j, const HrRow<BX
       den = K.den[j][i];
     else
       den = hr_den(g, K.a2);
-    float der;
-    if (DIV) {
-      der = __fdiv_rn(num, den);
-    } else {
-      const float y = K.y[j][i];
-      float q = __fmul_rn(num, y);
-      q = __fmaf_rn(__fmaf_rn(-q, den, num), y, q);
-      der = __fmaf_rn(__fmaf_rn(-q, den, num), y, q);
-      K.lo = min(K.lo, 2u * __float_as_uint(num) - 1u);
-      K.hi = hr_max_nan(K.hi, fabsf(num));
-    }
+    const float der = Q == HR_REFINED ? hr_div(num, den, K.y[j][i])
+                      : Q == HR_WIDE  ? hr_div_wide(num, den, K.y[j][i])
+                                      : __fdiv_rn(num, den);
+    K.lo = min(K.lo, 2u * __float_as_uint(num) - 1u);
+    K.hi = hr_max_nan(K.hi, fabsf(num));
     // m - g der with two roundings: the assembler would fuse a packed product into a packed
     // sum, so the product goes through a multiply-add by minus one that it cannot see
     const float2 r = __ffma2_rn(__fmul2_rn(g, make_float2(der, der)), make_float2(-K.one, -K.one), m);
@@ -350,7 +379,7 @@ __device__ __forceinline__ HrWin hr_window(int r0, int c0, int gy0, int gx0, int
 
 // One sweep of the block from the exchange buffer `buf` (the other blocks' cells before the
 // sweep).  Cells outside the image or on the region's rim get values that no exact cell reads.
-template <int RW, int RH, int BX, int BY, bool RAG, bool DIV>
+template <int RW, int RH, int BX, int BY, bool RAG, int Q>
 __device__ __forceinline__ void hr_sweep(HrBlock<BX, BY>& K, const double2* buf, int r0, int c0, const HrWin& win) {
   using G = HrGeom<RW, RH, BX, BY>;
   const int cb = c0 / BX;
@@ -412,9 +441,9 @@ __device__ __forceinline__ void hr_sweep(HrBlock<BX, BY>& K, const double2* buf,
         M.u[i] = p ? U.u[i] : D.u[i];
         M.v[i] = p ? U.v[i] : D.v[i];
       }
-      hr_row<BX, BY, DIV>(K, j, U, C, M);
+      hr_row<BX, BY, Q>(K, j, U, C, M);
     } else {
-      hr_row<BX, BY, DIV>(K, j, U, C, D);
+      hr_row<BX, BY, Q>(K, j, U, C, D);
     }
   }
 }
