@@ -45,15 +45,22 @@ __device__ __forceinline__ void hq_load(HqRow<FAST>& R, const HqVal<FAST>* __res
 // The float32 quotient num / den, correctly rounded, from rd = 1 / (double)den rounded to
 // float64: RN32(RN64(num * rd)).  RN64(num * rd) lies within 2^-52 (relative) of num / den.
 // A quotient of two float32 values is never that close to a midpoint m = M 2^e (M odd, 25
-// bits) of two float32 neighbours unless it equals it, which it cannot: den * m would need
-// 25 significant bits for num to have 24, and a non-zero num - den * m is a multiple of
-// 2^e ulp(den), i.e. at least 2^-49 of m relative; the same bound holds for the midpoints of
-// the subnormal range.  So the last rounding falls on the side of num / den (the
-// innocuous-double-rounding argument of S. Figueroa, "When is double rounding innocuous?",
-// SIGNUM Newsletter 30(3), 1995).  Zeros, infinities and NaNs give IEEE's answers (rd = inf
-// for den = 0, 0 for den = inf), and float64's range holds every product.  No branch: the
-// rows of a sweep are one basic block the scheduler interleaves.
-__device__ __forceinline__ float hq_div(float num, double rd) { return __double2float_rn(__dmul_rn((double)num, rd)); }
+// bits) of two normal float32 neighbours unless it equals it, which it cannot: den * m would
+// need 25 significant bits for num to have 24, and a non-zero num - den * m is a multiple of
+// 2^e ulp(den), i.e. at least 2^-49 of m relative.  So the last rounding falls on the side of
+// num / den (the innocuous-double-rounding argument of S. Figueroa, "When is double rounding
+// innocuous?", SIGNUM Newsletter 30(3), 1995).  A midpoint of the subnormal range has fewer bits,
+// and the quotient may equal it: there the product is first rounded to a multiple of 2^-177, which
+// makes a quotient on a midpoint exact (its product is within 2^-179) and keeps any other, at
+// least 2^-174 away, on its side.  Zeros, infinities and NaNs give IEEE's answers (rd = inf for
+// den = 0, 0 for den = inf), and float64's range holds every product.  No branch: the rows of a
+// sweep are one basic block the scheduler interleaves.
+__device__ __forceinline__ float hq_div(float num, double rd) {
+  const double q = __dmul_rn((double)num, rd), c = 0x1.8p-125, s = __dadd_rn(__dadd_rn(q, c), -c);
+  // 2^-151 <= |q| < 2^-126, by the exponent
+  const unsigned e = (unsigned)__double2hiint(q) & 0x7ff00000u;
+  return __double2float_rn(e - ((1023u - 151u) << 20) < (25u << 20) ? s : q);
+}
 
 // The update of region cell i from its window rows U (above), C and D (below):
 // hs_sweep_kernel's arithmetic, the 8 neighbours summed in its order.  RD: the quotient

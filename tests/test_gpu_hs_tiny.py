@@ -63,3 +63,36 @@ def test_static_half_is_not_slow(cuda_ok, persistent, s):
             t.append(e0.elapsed_time(e1))
         best.append(min(t))
     assert best[1] < 2 * best[0], best
+
+
+def particles(s):
+    """Moving particles on black beside the same texture in both frames."""
+    a = np.round(np.random.default_rng(0).uniform(20, 230, (s, s)))
+    b = a.copy()
+    rng = np.random.default_rng(1)
+    p = np.zeros((s, s), np.float32)
+    yy, xx = np.mgrid[-3:4, -3:4]
+    for _ in range(s * s // 60):
+        y, x = rng.uniform(4, s - 5, 2)
+        i, j = int(y), int(x)
+        p[i - 3:i + 4, j - 3:j + 4] += 200 * np.exp(-((yy + i - y) ** 2 + (xx + j - x) ** 2) / 2)
+    p = np.clip(np.round(p), 0, 255)
+    a[:, :s // 2], b[:, :s // 2] = p[:, :s // 2], np.roll(p, 1, 1)[:, :s // 2]
+    return a.astype(np.float32), b.astype(np.float32)
+
+
+@pytest.mark.parametrize("schedule,shape", [("queue", 0), ("queue", 1), ("queue", 3), ("resident", 3), ("resident", 1),
+                                            ("cluster", 0)])
+def test_batch_schedules_against_oracle(cuda_ok, schedule, shape):
+    """Subnormal quotients that lie on rounding midpoints, in the kernels that divide by a float64 reciprocal."""
+    import torch
+    from ofb200 import ops
+    a, b = particles(256)
+    I0, I1 = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    U, V = torch.zeros_like(I0), torch.zeros_like(I0)
+    st = ops.hs_batch([(I0, I1, U, V, 21.0, 200)], tile_shape=shape, schedule=schedule)
+    z = np.zeros_like(a)
+    Uo, Vo, _ = O.hs_solve(a, b, z, z, 21.0, 200)
+    assert int(st.item()) == 0
+    assert np.array_equal(U.cpu().numpy().view(np.uint32), Uo.view(np.uint32))
+    assert np.array_equal(V.cpu().numpy().view(np.uint32), Vo.view(np.uint32))

@@ -97,3 +97,28 @@ def test_wide_quotient_on_subnormal_midpoints():
         num = ((tie + np.ldexp(float(k), -149)) * rng.choice([-1.0, 1.0], n)).astype(F)
         ok = num != 0
         check(hr_div_wide, num[ok], den[ok])
+
+
+def hq_div(num, den):
+    """hq_div: the product with the float64 reciprocal, rounded to a multiple of 2^-177 where it is subnormal."""
+    q = num.astype(np.float64) * (1.0 / den.astype(np.float64))
+    c = 1.5 * 2.0 ** -125
+    s = (q + c) - c
+    return np.where((np.abs(q) >= 2.0 ** -151) & (np.abs(q) < 2.0 ** -126), s, q).astype(F)
+
+
+def test_float64_quotient_of_subnormal_results():
+    """Quotients on and next to the midpoints of the subnormal numbers, random ones, and all the short
+    numerators a diffusing flow ends in."""
+    rng = np.random.default_rng(4)
+    n = 1 << 19
+    f = lambda num, den, y: hq_div(num, den)  # noqa: E731
+    for den in ((2.0 * rng.integers(1, 1 << 10, n)).astype(F), (441 + rng.integers(0, 1 << 16, n) / 16).astype(F),
+                np.abs(mantissas(rng, n, -30, 60)).astype(F)):
+        m = 2 * rng.integers(0, 1 << 12, n) + 1
+        tie = np.ldexp(den.astype(np.float64) * m, -150)
+        for k in (-1, 0, 1):
+            check(f, ((tie + np.ldexp(float(k), -149)) * rng.choice([-1.0, 1.0], n)).astype(F), den)
+        check(f, np.ldexp(rng.integers(-4096, 4097, n).astype(float), -149).astype(F), den)
+        check(f, mantissas(rng, n, -149, -90).astype(F), den)
+        check(f, mantissas(rng, n, -60, 60).astype(F), den)
