@@ -19,11 +19,14 @@
 // change between the steps of a pixel, so each lane keeps its samples' 84 values in
 // registers (the reason for 128-thread CTAs at 168 registers, 3 per SM).  The footprints of
 // a lane's samples lie at fixed steps of 8 texels unless a position rounds across a texel,
-// which the step's fractions show; so all addresses are one base plus constants.  A
-// warp with such a position, or one outside the region, takes the per-sample path.
-// One 512x512 level from a smooth field (4.5 steps per pixel): 1.14 -> 0.92 ms (shared-memory
-// pipe 72 %, FMA pipe 60 %, issue 67 % busy); a 301x413 level with a 19 x 19 window, status
-// and error: 1.16 -> 0.52 ms.
+// which the step's fractions show; so all addresses are one base plus constants.  A warp with
+// such a position (where a flow is close to a whole number of pixels, a third of them) reads
+// each tile's texels from their own place, 32 bits at a time; one with footprints outside the
+// region tests every sample.  The error takes the same two ways.
+// One 512x512 level from a smooth field (4.5 steps per pixel): 1.10 -> 0.93 ms (shared-memory
+// pipe 72 %, FMA pipe 60 %, issue 67 % busy), with status and error 2.63 -> 1.44; from within
+// 1e-5 of the frames' 2-pixel shift 0.44 -> 0.41 and 1.30 -> 0.84; a 301x413 level with a
+// 19 x 19 window, status and error: 1.23 -> 0.46 ms.
 #include <float.h>
 
 #include "common.cuh"
@@ -46,9 +49,12 @@ static_assert(LK_JP % 16 == 8, "J pair stride");
 // dynamic shared memory of the kernel: sJ2 pairs, sD2 pairs, sI
 constexpr size_t LK_SMEM = (size_t)LK_JR * LK_JP * 8 + (size_t)LK_G * LK_GP * 8 + (size_t)LK_I * LK_IP * 4;
 
-// Threads and CTAs per SM of the kernel for NT window tiles per axis: 3 values per sample are
-// held in registers, 2 NT^2 samples per lane (the default window: 28).
-constexpr int lk_threads(int nt) { return nt == 4 ? 128 : 256; }
+// Whether a lane holds its window samples in registers, 3 values each, 2 NT^2 samples (28 of the
+// default window): not the 32 of the other windows above 24, with which 8 warps fit an SM (a 31 x 31
+// window on the smooth field above: 1.53 ms, 1.31 with the samples read again in every step).
+constexpr bool lk_hold(int nt, bool def) { return nt < 4 || def; }
+// Threads and CTAs per SM of the kernel.
+constexpr int lk_threads(int nt, bool def) { return nt == 4 && def ? 128 : 256; }
 constexpr int lk_ctas(int nt, bool def) { return nt == 4 && def ? 3 : 2; }
 
 struct LkParams {
@@ -79,36 +85,43 @@ __device__ __forceinline__ void lk_weights(int id, int ws, int lo, int hi, float
 // every image (H, W < 2^21), so that the index arithmetic that follows cannot overflow.
 __device__ __forceinline__ int lk_texel(float f) { return (int)fminf(fmaxf(f, -4194304.f), 4194304.f); }
 
-// A bilinear sample (clamp to edge) from the staged region when its 2 x 2 footprint lies inside it
-// (rx, ry: footprint origin relative to the region), else from global memory.
-__device__ __forceinline__ float lk_bilinear_s(const float2* __restrict__ sJ, const float* __restrict__ J, int H, int W,
-                                               int pitch, float x, float y, int ox, int oy) {
-  float xs = __fsub_rn(x, 0.5f), ys = __fsub_rn(y, 0.5f);
-  float fx0 = floorf(xs), fy0 = floorf(ys);
-  float a = __fsub_rn(xs, fx0), b = __fsub_rn(ys, fy0);
-  const int i0 = lk_texel(fx0), j0 = lk_texel(fy0);
-  const int rx = i0 - ox, ry = j0 - oy;
-  float t00, t10, t01, t11;
+// The texels (clamp to edge) of the 2 x 2 footprint at (rx, ry) relative to the region: from it when
+// they lie inside, else from global memory.
+__device__ __forceinline__ void lk_texels(const float2* __restrict__ sJ, const float* __restrict__ J, int H, int W,
+                                          int pitch, int rx, int ry, int ox, int oy, float (&t)[4]) {
   if ((unsigned)rx <= (unsigned)(LK_JR - 2) && (unsigned)ry <= (unsigned)(LK_JR - 2)) {
     const float2* q = sJ + ry * LK_JP + rx;
-    t00 = q[0].x;
-    t10 = q[1].x;
-    t01 = q[LK_JP].x;
-    t11 = q[LK_JP + 1].x;
+    t[0] = q[0].x;
+    t[1] = q[1].x;
+    t[2] = q[LK_JP].x;
+    t[3] = q[LK_JP + 1].x;
   } else {
-    int xa = clampi(i0, 0, W - 1), xb = clampi(i0 + 1, 0, W - 1);
-    int ya = clampi(j0, 0, H - 1), yb = clampi(j0 + 1, 0, H - 1);
-    t00 = __ldg(J + (size_t)ya * pitch + xa);
-    t10 = __ldg(J + (size_t)ya * pitch + xb);
-    t01 = __ldg(J + (size_t)yb * pitch + xa);
-    t11 = __ldg(J + (size_t)yb * pitch + xb);
+    const int i0 = rx + ox, j0 = ry + oy;
+    const int xa = clampi(i0, 0, W - 1), xb = clampi(i0 + 1, 0, W - 1);
+    const int ya = clampi(j0, 0, H - 1), yb = clampi(j0 + 1, 0, H - 1);
+    t[0] = __ldg(J + (size_t)ya * pitch + xa);
+    t[1] = __ldg(J + (size_t)ya * pitch + xb);
+    t[2] = __ldg(J + (size_t)yb * pitch + xa);
+    t[3] = __ldg(J + (size_t)yb * pitch + xb);
   }
-  float oa = __fsub_rn(1.f, a), ob = __fsub_rn(1.f, b);
-  float r = __fmul_rn(__fmul_rn(oa, ob), t00);
-  r = __fmaf_rn(__fmul_rn(a, ob), t10, r);
-  r = __fmaf_rn(__fmul_rn(oa, b), t01, r);
-  r = __fmaf_rn(__fmul_rn(a, b), t11, r);
-  return r;
+}
+
+__device__ __forceinline__ float lk_blend(float a, float oa, float b, float ob, const float (&t)[4]) {
+  float r = __fmul_rn(__fmul_rn(oa, ob), t[0]);
+  r = __fmaf_rn(__fmul_rn(a, ob), t[1], r);
+  r = __fmaf_rn(__fmul_rn(oa, b), t[2], r);
+  return __fmaf_rn(__fmul_rn(a, b), t[3], r);
+}
+
+// A bilinear sample at any position.
+__device__ __forceinline__ float lk_bilinear_s(const float2* __restrict__ sJ, const float* __restrict__ J, int H, int W,
+                                               int pitch, float x, float y, int ox, int oy) {
+  const float xs = __fsub_rn(x, 0.5f), ys = __fsub_rn(y, 0.5f);
+  const float fx0 = floorf(xs), fy0 = floorf(ys);
+  const float a = __fsub_rn(xs, fx0), b = __fsub_rn(ys, fy0);
+  float t[4];
+  lk_texels(sJ, J, H, W, pitch, lk_texel(fx0) - ox, lk_texel(fy0) - oy, ox, oy, t);
+  return lk_blend(a, __fsub_rn(1.f, a), b, __fsub_rn(1.f, b), t);
 }
 
 // floor(x) for |x| < 2^22, as a float and as an int, on the FMA pipe: x + 1.5 * 2^23 rounded
@@ -116,7 +129,7 @@ __device__ __forceinline__ float lk_bilinear_s(const float2* __restrict__ sJ, co
 // hold the integer.
 __device__ __forceinline__ float lk_floor(float x, int& i) {
   const float t = __fadd_rd(x, 12582912.0f);
-  i = __float_as_int(t) - 0x4B400000;
+  i = (int)(__float_as_uint(t) - 0x4B400000u);
   return __fsub_rn(t, 12582912.0f);
 }
 
@@ -158,10 +171,11 @@ __device__ __forceinline__ bool lk_on(unsigned act, int v, int ty, int tx, int x
 // time: lane (xid, yid)'s 4th column tile is used when xid < 3, its 4th row tile of the first
 // half when yid < 3, the 4th row tile of the second half never.
 template <int NT, bool DEF>
-__global__ void __launch_bounds__(lk_threads(NT), lk_ctas(NT, DEF)) lk_dense_kernel(
+__global__ void __launch_bounds__(lk_threads(NT, DEF), lk_ctas(NT, DEF)) lk_dense_kernel(
     const float* __restrict__ I, const float* __restrict__ J, float* __restrict__ U, float* __restrict__ V, int H, int W,
     int pitch, LkParams p, uint8_t* __restrict__ status, float* __restrict__ err) {
-  constexpr int LK_THREADS = lk_threads(NT);
+  constexpr int LK_THREADS = lk_threads(NT, DEF);
+  constexpr bool HOLD = lk_hold(NT, DEF);
   extern __shared__ float4 lk_dyn[];
   float2* const sJ = reinterpret_cast<float2*>(lk_dyn);  // (J[y][x], J[y + 4][x]) pairs
   float2* const sD = sJ + LK_JR * LK_JP;                 // (dx, dy) pairs
@@ -213,6 +227,11 @@ __global__ void __launch_bounds__(lk_threads(NT), lk_ctas(NT, DEF)) lk_dense_ker
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int xid = lane & 7, yid = lane >> 3;
+  // A single texel (y, x) as a float index from sJ's pair (y, x): its first part, or for the lanes of
+  // rows 2 and 3 the second part of the pair 4 rows up, so that a warp's reads fall in distinct banks.
+  const unsigned row_lo = yid >= 2 ? 4 : 0;
+  const int row_part = yid >= 2 ? 1 - 8 * LK_JP : 0;
+  const float* const texel = reinterpret_cast<const float*>(sJ) + row_part;
   unsigned act = 0;  // bit 16 v + 4 ty + tx: the sample's tile weight is not 0
   unsigned any = 0;  // the same bit set when it is for some lane of the warp
   if (!DEF) {
@@ -248,37 +267,60 @@ __global__ void __launch_bounds__(lk_threads(NT), lk_ctas(NT, DEF)) lk_dense_ker
       const int gxb = c;  // (gyb, gxb): gradient-tile origin of this pixel's window
       const float* const pI = sI + (gyb + yid + 1) * LK_IP + gxb + xid + 1;
       const float2* const pD = sD + (gyb + yid) * LK_GP + gxb + xid;
-      // The window's intensities (negated) and gradients, as pairs over the two row halves:
-      // they stay in registers for every Newton step.  Samples without weight hold 0.
-      float2 nI[NT][NT], Dx[NT][NT], Dy[NT][NT];
-      float a11[2] = {0.f, 0.f}, a12[2] = {0.f, 0.f}, a22[2] = {0.f, 0.f};
+      // A window sample's intensities (negated) and gradients, as pairs over the two row halves.
+      // Samples without weight hold 0.
+      struct Sample {
+        float2 nI, Dx, Dy;
+      };
+      auto window = [&](int ty, int tx) {
+        float iv[2], dx[2], dy[2];
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+          iv[v] = dx[v] = dy[v] = 0.f;
+          if (LK_SKIP(v, ty, tx)) continue;
+          iv[v] = -pI[(ty * 8 + 4 * v) * LK_IP + tx * 8];
+          const float2 d = pD[(ty * 8 + 4 * v) * LK_GP + tx * 8];
+          const bool on = lk_on<DEF>(act, v, ty, tx, xid, yid);
+          dx[v] = on ? d.x : 0.f;
+          dy[v] = on ? d.y : 0.f;
+        }
+        return Sample{make_float2(iv[0], iv[1]), make_float2(dx[0], dx[1]), make_float2(dy[0], dy[1])};
+      };
+      Sample held[HOLD ? NT : 1][HOLD ? NT : 1] = {};  // stay in registers for every Newton step
+      auto sample = [&](int ty, int tx) {
+        if constexpr (HOLD)
+          return held[ty][tx];
+        else
+          return window(ty, tx);
+      };
+      float2 a11 = make_float2(0.f, 0.f), a12 = a11, a22 = a11;
 #pragma unroll
       for (int ty = 0; ty < NT; ty++)
 #pragma unroll
         for (int tx = 0; tx < NT; tx++) {
-          float iv[2], dx[2], dy[2];
-#pragma unroll
-          for (int v = 0; v < 2; v++) {
-            iv[v] = dx[v] = dy[v] = 0.f;
-            if (LK_SKIP(v, ty, tx)) continue;
-            iv[v] = -pI[(ty * 8 + 4 * v) * LK_IP + tx * 8];
-            const float2 d = pD[(ty * 8 + 4 * v) * LK_GP + tx * 8];
-            const bool on = lk_on<DEF>(act, v, ty, tx, xid, yid);
-            dx[v] = on ? d.x : 0.f;
-            dy[v] = on ? d.y : 0.f;
-            // w is 1 here (the tile weights are products of 0 / 1 values), so the reference's
-            // multiplications by w are exact identities; + 0 * 0 changes no sum
-            a11[v] = __fmaf_rn(dx[v], dx[v], a11[v]);
-            a12[v] = __fmaf_rn(dx[v], dy[v], a12[v]);
-            a22[v] = __fmaf_rn(dy[v], dy[v], a22[v]);
+          if (!HOLD && LK_SKIP2(ty, tx)) continue;
+          const Sample w = window(ty, tx);
+          // the tile weights are products of 0 / 1 values, so the reference's multiplications by
+          // them are exact identities; + 0 * 0 changes no sum
+          if (DEF) {
+            if (ty < NT - 1) {
+              a11.y = __fmaf_rn(w.Dx.y, w.Dx.y, a11.y);
+              a12.y = __fmaf_rn(w.Dx.y, w.Dy.y, a12.y);
+              a22.y = __fmaf_rn(w.Dy.y, w.Dy.y, a22.y);
+            }
+            a11.x = __fmaf_rn(w.Dx.x, w.Dx.x, a11.x);
+            a12.x = __fmaf_rn(w.Dx.x, w.Dy.x, a12.x);
+            a22.x = __fmaf_rn(w.Dy.x, w.Dy.x, a22.x);
+          } else {
+            a11 = __ffma2_rn(w.Dx, w.Dx, a11);
+            a12 = __ffma2_rn(w.Dx, w.Dy, a12);
+            a22 = __ffma2_rn(w.Dy, w.Dy, a22);
           }
-          nI[ty][tx] = make_float2(iv[0], iv[1]);
-          Dx[ty][tx] = make_float2(dx[0], dx[1]);
-          Dy[ty][tx] = make_float2(dy[0], dy[1]);
+          if constexpr (HOLD) held[ty][tx] = w;
         }
       float A11, A12, A22;
-      lk_tree2(make_float2(a11[0], a11[1]), make_float2(a12[0], a12[1]), A11, A12);
-      A22 = lk_tree(a22[0], a22[1]);
+      lk_tree2(a11, a12, A11, A12);
+      A22 = lk_tree(a22.x, a22.y);
       const size_t gid = (size_t)i * pitch + j;
       float D = __fmaf_rn(A11, A22, -__fmul_rn(A12, A12));
       if (D < 1.192092896e-07f) {
@@ -305,6 +347,28 @@ __global__ void __launch_bounds__(lk_threads(NT), lk_ctas(NT, DEF)) lk_dense_ker
         ly[t].x = __fadd_rn(ly[t - 1].x, 8.0f);
         ly[t].y = __fadd_rn(ly[t - 1].y, 8.0f);
       }
+      // The fractions of every tile's position and the texels of their footprints relative to the
+      // region; whether those of the whole warp lie in it.  Of use for positions below 2^22.
+      auto footprints = [&](float2(&xa)[NT], float2(&xo)[NT], float2(&yb)[NT], float2(&yo)[NT], int(&xi)[NT],
+                            int(&yi)[2][NT]) {
+        unsigned xout = 0, yout = 0;
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+          const float xs = __fsub_rn(lx[t], 0.5f), y0 = __fsub_rn(ly[t].x, 0.5f), y1 = __fsub_rn(ly[t].y, 0.5f);
+          const float a = __fsub_rn(xs, lk_floor(xs, xi[t])), oa = __fsub_rn(1.f, a);
+          xa[t] = make_float2(a, a);
+          xo[t] = make_float2(oa, oa);
+          yb[t] = make_float2(__fsub_rn(y0, lk_floor(y0, yi[0][t])), __fsub_rn(y1, lk_floor(y1, yi[1][t])));
+          yo[t] = __ffma2_rn(yb[t], m1, make_float2(1.f, 1.f));
+          // unsigned: the texels of a position that is out of reach may wrap, but not overflow
+          xi[t] = (int)((unsigned)xi[t] - (unsigned)jox);
+          yi[0][t] = (int)((unsigned)yi[0][t] - (unsigned)joy);
+          yi[1][t] = (int)((unsigned)yi[1][t] - (unsigned)joy);
+          xout = max(xout, (unsigned)xi[t]);
+          yout = max(yout, max((unsigned)yi[0][t] - row_lo, (unsigned)yi[1][t] - row_lo));
+        }
+        return __all_sync(0xffffffffu, xout <= LK_JR - 2 && yout <= LK_JR - 2 - row_lo) != 0;
+      };
       uint8_t st = 1;
 #pragma unroll 1
       for (int k = 0; k < p.niter; k++) {
@@ -336,6 +400,35 @@ __global__ void __launch_bounds__(lk_threads(NT), lk_ctas(NT, DEF)) lk_dense_ker
         const bool regular = worst < 0x3f800000u && (unsigned)rx <= (unsigned)(LK_JR - 2 - 8 * (NT - 1)) &&
                              (unsigned)ry <= (unsigned)(LK_JR - 2 - 8 * (NT - 1) - 4);
         float2 b1 = make_float2(0.f, 0.f), b2 = b1;
+        // sample (ty, tx) of both row halves from the texels of its footprint
+        auto add = [&](int ty, int tx, float2 t00, float2 t10, float2 t01, float2 t11) {
+          const float2 w00 = __fmul2_rn(xo[tx], yo[ty]), w10 = __fmul2_rn(xa[tx], yo[ty]);
+          const float2 w01 = __fmul2_rn(xo[tx], yb[ty]), w11 = __fmul2_rn(xa[tx], yb[ty]);
+          float2 Jv = __fmul2_rn(w00, t00);
+          Jv = __ffma2_rn(w10, t10, Jv);
+          Jv = __ffma2_rn(w01, t01, Jv);
+          Jv = __ffma2_rn(w11, t11, Jv);
+          const Sample w = sample(ty, tx);
+          float2 d = __fadd2_rn(Jv, w.nI);  // (Jv - Iv) * w with w == 1
+          if (!DEF || tx == NT - 1) {
+            if (!lk_on<DEF>(act, 0, ty, tx, xid, yid)) d.x = 0.f;
+            if (!lk_on<DEF>(act, 1, ty, tx, xid, yid)) d.y = 0.f;
+          }
+          b1 = __ffma2_rn(d, w.Dx, b1);
+          b2 = __ffma2_rn(d, w.Dy, b2);
+        };
+        // the same for the first half alone
+        auto add0 = [&](int ty, int tx, float t00, float t10, float t01, float t11) {
+          float Jv = __fmul_rn(__fmul_rn(xo[tx].x, yo[ty].x), t00);
+          Jv = __fmaf_rn(__fmul_rn(xa[tx].x, yo[ty].x), t10, Jv);
+          Jv = __fmaf_rn(__fmul_rn(xo[tx].x, yb[ty].x), t01, Jv);
+          Jv = __fmaf_rn(__fmul_rn(xa[tx].x, yb[ty].x), t11, Jv);
+          const Sample w = sample(ty, tx);
+          float d = __fadd_rn(Jv, w.nI.x);
+          if (!lk_on<DEF>(act, 0, ty, tx, xid, yid)) d = 0.f;
+          b1.x = __fmaf_rn(d, w.Dx.x, b1.x);
+          b2.x = __fmaf_rn(d, w.Dy.x, b2.x);
+        };
         if (__all_sync(0xffffffffu, regular)) {
           const float2* const q = sJ + ry * LK_JP + rx;
 #pragma unroll
@@ -344,46 +437,51 @@ __global__ void __launch_bounds__(lk_threads(NT), lk_ctas(NT, DEF)) lk_dense_ker
             for (int tx = 0; tx < NT; tx++) {
               if (LK_SKIP2(ty, tx)) continue;
               const float2* const s = q + (8 * ty) * LK_JP + 8 * tx;
-              if (DEF && ty == NT - 1) {  // the first half alone: 32-bit reads, scalar arithmetic
-                float Jv = __fmul_rn(__fmul_rn(xo[tx].x, yo[ty].x), s[0].x);
-                Jv = __fmaf_rn(__fmul_rn(xa[tx].x, yo[ty].x), s[1].x, Jv);
-                Jv = __fmaf_rn(__fmul_rn(xo[tx].x, yb[ty].x), s[LK_JP].x, Jv);
-                Jv = __fmaf_rn(__fmul_rn(xa[tx].x, yb[ty].x), s[LK_JP + 1].x, Jv);
-                float d = __fadd_rn(Jv, nI[ty][tx].x);
-                if (!lk_on<DEF>(act, 0, ty, tx, xid, yid)) d = 0.f;
-                b1.x = __fmaf_rn(d, Dx[ty][tx].x, b1.x);
-                b2.x = __fmaf_rn(d, Dy[ty][tx].x, b2.x);
-                continue;
-              }
-              const float2 w00 = __fmul2_rn(xo[tx], yo[ty]), w10 = __fmul2_rn(xa[tx], yo[ty]);
-              const float2 w01 = __fmul2_rn(xo[tx], yb[ty]), w11 = __fmul2_rn(xa[tx], yb[ty]);
-              float2 Jv = __fmul2_rn(w00, s[0]);
-              Jv = __ffma2_rn(w10, s[1], Jv);
-              Jv = __ffma2_rn(w01, s[LK_JP], Jv);
-              Jv = __ffma2_rn(w11, s[LK_JP + 1], Jv);
-              float2 d = __fadd2_rn(Jv, nI[ty][tx]);  // (Jv - Iv) * w with w == 1
-              if (!DEF || tx == NT - 1) {
-                if (!lk_on<DEF>(act, 0, ty, tx, xid, yid)) d.x = 0.f;
-                if (!lk_on<DEF>(act, 1, ty, tx, xid, yid)) d.y = 0.f;
-              }
-              b1 = __ffma2_rn(d, Dx[ty][tx], b1);
-              b2 = __ffma2_rn(d, Dy[ty][tx], b2);
+              if (DEF && ty == NT - 1)  // 32-bit reads, scalar arithmetic
+                add0(ty, tx, s[0].x, s[1].x, s[LK_JP].x, s[LK_JP + 1].x);
+              else
+                add(ty, tx, s[0], s[1], s[LK_JP], s[LK_JP + 1]);
             }
-        } else {  // some footprint leaves the staged region or rounds to another texel
-          auto half = [&](int v, float& s1, float& s2) {
+        } else {
+          // some footprint rounds to another texel or leaves the region: each tile's own
+          int xi[NT], yi[2][NT];
+          if (footprints(xa, xo, yb, yo, xi, yi)) {
 #pragma unroll
             for (int ty = 0; ty < NT; ty++)
 #pragma unroll
               for (int tx = 0; tx < NT; tx++) {
-                if (LK_SKIP(v, ty, tx) || !lk_on<DEF>(act, v, ty, tx, xid, yid)) continue;
-                const float Jv = lk_bilinear_s(sJ, J, H, W, pitch, lx[tx], v ? ly[ty].y : ly[ty].x, jox, joy);
-                const float d = __fadd_rn(Jv, v ? nI[ty][tx].y : nI[ty][tx].x);
-                s1 = __fmaf_rn(d, v ? Dx[ty][tx].y : Dx[ty][tx].x, s1);
-                s2 = __fmaf_rn(d, v ? Dy[ty][tx].y : Dy[ty][tx].x, s2);
+                if (LK_SKIP2(ty, tx)) continue;
+                const float* const s = texel + 2 * (yi[0][ty] * LK_JP + xi[tx]);
+                if (DEF && ty == NT - 1) {
+                  add0(ty, tx, s[0], s[2], s[2 * LK_JP], s[2 * LK_JP + 2]);
+                } else {
+                  const float* const r = texel + 2 * (yi[1][ty] * LK_JP + xi[tx]);
+                  add(ty, tx, make_float2(s[0], r[0]), make_float2(s[2], r[2]),
+                      make_float2(s[2 * LK_JP], r[2 * LK_JP]), make_float2(s[2 * LK_JP + 2], r[2 * LK_JP + 2]));
+                }
               }
-          };
-          half(0, b1.x, b2.x);
-          half(1, b1.y, b2.y);
+          } else {
+            auto half = [&](int v, float& s1, float& s2) {
+#pragma unroll
+              for (int ty = 0; ty < NT; ty++)
+#pragma unroll
+                for (int tx = 0; tx < NT; tx++) {
+                  if (LK_SKIP(v, ty, tx) || !lk_on<DEF>(act, v, ty, tx, xid, yid)) continue;
+                  float t[4];
+                  int y;
+                  const float ys = __fsub_rn(v ? ly[ty].y : ly[ty].x, 0.5f), b = __fsub_rn(ys, lk_floor(ys, y));
+                  const float ob = __fsub_rn(1.f, b);
+                  lk_texels(sJ, J, H, W, pitch, xi[tx], y - joy, jox, joy, t);
+                  const float Jv = lk_blend(xa[tx].x, xo[tx].x, b, ob, t);
+                  const Sample w = sample(ty, tx);
+                  const float d = __fadd_rn(Jv, v ? w.nI.y : w.nI.x);
+                  s1 = __fmaf_rn(d, v ? w.Dx.y : w.Dx.x, s1);
+                  s2 = __fmaf_rn(d, v ? w.Dy.y : w.Dy.x, s2);
+                }
+            };
+            half(0, b1.x, b2.x);
+            half(1, b1.y, b2.y);
+          }
         }
         float B1, B2;
         lk_tree2(b1, b2, B1, B2);
@@ -407,31 +505,42 @@ __global__ void __launch_bounds__(lk_threads(NT), lk_ctas(NT, DEF)) lk_dense_ker
         lk_weights(xid, p.ws, p.aL, p.aR, wx, bx);
         lk_weights(yid, p.ws, p.aT, p.aB, wy0, by0);
         lk_weights(yid + 4, p.ws, p.aT, p.aB, wy1, by1);
-        float e[2] = {0.f, 0.f};
+        float2 xa[NT], xo[NT], yb[NT], yo[NT];
+        int xi[NT], yi[2][NT];
+        // the positions of an infinite or huge flow are beyond footprints' reach
+        const bool inside = footprints(xa, xo, yb, yo, xi, yi) &
+                            (__all_sync(0xffffffffu, fabsf(lx[0]) < 2097152.f && fabsf(ly[0].x) < 2097152.f) != 0);
+        float e0 = 0.f, e1 = 0.f;
 #pragma unroll
-        for (int v = 0; v < 2; v++) {
-          const float* wy = v ? wy1 : wy0;
-          const int* by = v ? by1 : by0;
-#pragma unroll
-          for (int o = 0; o < 16; o++) {
-            int ty = ord[o] >> 8, tx = (ord[o] >> 4) & 15, gb = ord[o] & 15;
-            if ((gb & 1) && !(bx[0] < p.ws)) continue;
-            if ((gb & 2) && !(by[0] < p.ws)) continue;
-            if ((gb & 4) && !(bx[1] < p.ws)) continue;
-            if ((gb & 8) && !(by[1] < p.ws)) continue;
-            float w = __fmul_rn(wx[tx], wy[ty]);
-            float Iv = pI[(ty * 8 + 4 * v) * LK_IP + tx * 8];
-            // positions past the window's last tile continue the same additions of 8
-            float x = lx[tx < NT ? tx : NT - 1], y = v ? ly[ty < NT ? ty : NT - 1].y : ly[ty < NT ? ty : NT - 1].x;
-            float Jv = lk_bilinear_s(sJ, J, H, W, pitch, x, y, jox, joy);
-            // the reference's divisions by 512 are exact scalings
-            float d = __fmul_rn(__fsub_rn(__fmul_rn(__fmaf_rn(Jv, 16384.f, 256.f), 1.f / 512.f),
-                                          __fmul_rn(__fmaf_rn(Iv, 16384.f, 256.f), 1.f / 512.f)),
-                                w);
-            e[v] = __fadd_rn(e[v], fabsf(d));
+        for (int o = 0; o < 16; o++) {
+          const int ty = ord[o] >> 8, tx = (ord[o] >> 4) & 15, gb = ord[o] & 15;
+          if (ty >= NT || tx >= NT) continue;  // beyond the window: their guards are false
+          if ((gb & 1) && !(bx[0] < p.ws)) continue;
+          if ((gb & 4) && !(bx[1] < p.ws)) continue;
+          const bool on0 = (!(gb & 2) || by0[0] < p.ws) && (!(gb & 8) || by0[1] < p.ws);
+          const bool on1 = (!(gb & 2) || by1[0] < p.ws) && (!(gb & 8) || by1[1] < p.ws);
+          float2 Jv;
+          if (inside) {
+            const float* const s = texel + 2 * (yi[0][ty] * LK_JP + xi[tx]);
+            const float* const r = texel + 2 * (yi[1][ty] * LK_JP + xi[tx]);
+            Jv = __fmul2_rn(__fmul2_rn(xo[tx], yo[ty]), make_float2(s[0], r[0]));
+            Jv = __ffma2_rn(__fmul2_rn(xa[tx], yo[ty]), make_float2(s[2], r[2]), Jv);
+            Jv = __ffma2_rn(__fmul2_rn(xo[tx], yb[ty]), make_float2(s[2 * LK_JP], r[2 * LK_JP]), Jv);
+            Jv = __ffma2_rn(__fmul2_rn(xa[tx], yb[ty]), make_float2(s[2 * LK_JP + 2], r[2 * LK_JP + 2]), Jv);
+          } else {
+            Jv.x = lk_bilinear_s(sJ, J, H, W, pitch, lx[tx], ly[ty].x, jox, joy);
+            Jv.y = lk_bilinear_s(sJ, J, H, W, pitch, lx[tx], ly[ty].y, jox, joy);
           }
+          const float2 Iv = make_float2(pI[ty * 8 * LK_IP + tx * 8], pI[(ty * 8 + 4) * LK_IP + tx * 8]);
+          // the reference's divisions by 512 are exact scalings
+          const float2 big = make_float2(16384.f, 16384.f), half = make_float2(256.f, 256.f);
+          const float2 inv = make_float2(1.f / 512.f, 1.f / 512.f);
+          float2 d = __ffma2_rn(__fmul2_rn(__ffma2_rn(Iv, big, half), inv), m1, __fmul2_rn(__ffma2_rn(Jv, big, half), inv));
+          d = __fmul2_rn(d, make_float2(__fmul_rn(wx[tx], wy0[ty]), __fmul_rn(wx[tx], wy1[ty])));
+          if (on0) e0 = __fadd_rn(e0, fabsf(d.x));
+          if (on1) e1 = __fadd_rn(e1, fabsf(d.y));
         }
-        float E = lk_tree(e[0], e[1]);
+        float E = lk_tree(e0, e1);
         if (lane == 0) err[gid] = __fdiv_rn(E, (float)(32 * p.ws * p.ws));
       }
       if (lane == 0) {
@@ -476,7 +585,7 @@ extern "C" int of_lk_dense(const float* I, const float* J, float* U, float* V, i
     return check_launch("of_lk_dense");
   };
 #define LK_RUN(NT, DEF) \
-  run(lk_dense_kernel<NT, DEF>, lk_threads(NT), OF_SMEM_OPT_IN((lk_dense_kernel<NT, DEF>), LK_SMEM))
+  run(lk_dense_kernel<NT, DEF>, lk_threads(NT, DEF), OF_SMEM_OPT_IN((lk_dense_kernel<NT, DEF>), LK_SMEM))
   if (def) return LK_RUN(4, true);
   if (nt == 4) return LK_RUN(4, false);
   return nt == 3 ? LK_RUN(3, false) : LK_RUN(2, false);

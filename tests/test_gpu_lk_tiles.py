@@ -70,3 +70,33 @@ def test_lk_infinite_flow(cuda_ok, hw):
     for x, y in zip(got, want):
         assert np.array_equal(x[~odd], y[~odd])
     assert not got[2][odd].any()
+
+
+@pytest.mark.parametrize("hw", [13, 15])
+def test_lk_near_whole_pixels_is_not_slow(cuda_ok, hw):
+    """A flow within 1e-5 of a whole number of pixels, whose positions round across texels, against the
+    whole number itself: at most 1.3 times the time (1.03 and 1.07 as measured; 1.5 when every sample
+    of such a warp was placed by itself)."""
+    import torch
+    from ofb200 import ops
+    h = w = 512
+    rng = np.random.default_rng(2)
+    a = torch.from_numpy(frames(h, w, 5)[0]).cuda()
+    b = torch.roll(a, (1, 2), (0, 1)).contiguous()
+    noise = torch.from_numpy(rng.normal(0, 1e-5, (h, w)).astype(np.float32)).cuda()
+    st = torch.empty((h, w), dtype=torch.uint8, device="cuda")
+    er = torch.empty((h, w), dtype=torch.float32, device="cuda")
+    best = []
+    for off in (torch.zeros_like(noise), noise):
+        t = []
+        for _ in range(8):
+            U, V = 2 + off, 1 - off
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            e0.record()
+            ops.lk_dense(a, b, U, V, hw, 5, (0, 0, 0, 0), st, er)
+            e1.record()
+            e1.synchronize()
+            t.append(e0.elapsed_time(e1))
+        best.append(min(t))
+    assert best[1] < 1.3 * best[0], best
