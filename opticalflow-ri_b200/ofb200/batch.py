@@ -161,6 +161,16 @@ class PairBatch:
         return e
 
 
+def _stage(p, t):
+    """p.copy_(t) into a pinned upload buffer: plain CPU memory of p's type goes past the CPU's caches
+    (stage_copyto); a cast, a strided or negated view and a CUDA tensor through torch."""
+    if (t.dtype == p.dtype and t.shape == p.shape and t.device.type == "cpu" and t.is_contiguous()
+            and not t.is_neg()):
+        stage_copyto(p.numpy(), t.detach().numpy())
+    else:
+        p.copy_(t.detach())
+
+
 class HostBatch:
     """Frame pairs from host memory to flow fields in host memory, `depth` batches in flight.
 
@@ -223,10 +233,7 @@ class HostBatch:
                 if t.is_pinned() and t.dtype == p.dtype:
                     srcs.append(t)
                 else:
-                    if t.dtype == p.dtype:
-                        stage_copyto(p.numpy(), t.detach().numpy())
-                    else:
-                        p.copy_(t)
+                    _stage(p, t)
                     srcs.append(p)
         cur, up, down = torch.cuda.current_stream(), self._up, self._down
         up.wait_event(st["done"])  # the slot's previous replay has read its inputs

@@ -204,3 +204,16 @@ def test_host_batch_in_flight(torch_cuda):
             assert np.array_equal(Ug, Uw) and np.array_equal(Vg, Vw)
     with pytest.raises(ValueError):
         hb.submit(batches[0][:2])
+
+
+def test_host_batch_takes_strided_and_device_frames(torch_cuda):
+    """Frames given as a crop of a larger array or as CUDA tensors give what contiguous host arrays do."""
+    torch = torch_cuda
+    from ofb200.batch import HostBatch
+    rng = np.random.default_rng(8)
+    big = [rng.integers(0, 256, (70, 100)).astype(np.float32) for _ in range(2)]
+    hb = HostBatch(_specs()[0][:1], streams=1, depth=1)
+    want = [x.copy() for x in hb.run([tuple(np.ascontiguousarray(b[3:67, 5:85]) for b in big)])[0]]
+    for frames in (tuple(b[3:67, 5:85] for b in big), tuple(torch.from_numpy(b).cuda()[3:67, 5:85] for b in big)):
+        got = hb.run([frames])[0]
+        assert all(np.array_equal(x, y) for x, y in zip(got, want))

@@ -26,3 +26,16 @@ def test_host_stage_refuses_overlap_and_converts_through_numpy():
         out = np.zeros_like(a)
         stage_copyto(out, src)
         assert np.array_equal(out, src.astype(np.float32))
+
+
+def test_batch_staging_takes_what_copy_takes():
+    """HostBatch's staging copy: plain memory, strided and negated views, other types."""
+    import torch
+    from ofb200.batch import _stage
+    a = torch.from_numpy(np.random.default_rng(2).random((300, 1030), dtype=np.float32))
+    neg = torch.conj(torch.complex(a, a)).imag  # a lazily negated view: it has no numpy form
+    assert neg.is_neg()
+    for t in (a[:, :1024].contiguous(), a[:, 3:1027], a[:, :1024].double(), neg[:, :1024], a[:, :1024].clone().requires_grad_()):
+        p = torch.zeros(300, 1024)
+        _stage(p, t)
+        assert torch.equal(p, t.detach().float()) and not p.requires_grad
