@@ -338,6 +338,11 @@ static size_t hs_persistent_ws(int H, int W, int pitch) {
   return of_hs_batch_workspace_size(&q, 1);
 }
 
+// Whether of_hs_solve_persistent runs a size in one launch.  Images with more tiles than SMs: a
+// launch per pass, whose tiles all SMs share, beats the persistent queue (600 sweeps of 512 x 512:
+// 1.27 ms against 2.98).
+static bool hs_one_launch(int H, int W) { return hs_halo_bytes(H, W) != 0 || H < 16 || W < 16; }
+
 // Covers both of_hs_solve and of_hs_solve_persistent.
 extern "C" size_t of_hs_workspace_size(int H, int W, int pitch) {
   size_t N = (size_t)H * pitch;
@@ -434,17 +439,25 @@ extern "C" int of_hs_solve(const float* I0, const float* I1, float* U, float* V,
 extern "C" int of_hs_solve_persistent(const float* I0, const float* I1, float* U, float* V, int H, int W, int pitch,
                                       float alpha, int niter, double* err_out, void* workspace, size_t workspace_bytes,
                                       void* stream) {
+  return of_hs_solve_persistent_limit(I0, I1, U, V, H, W, pitch, alpha, niter, err_out, 1ll << 20, nullptr, workspace,
+                                      workspace_bytes, stream);
+}
+
+extern "C" int of_hs_solve_persistent_limit(const float* I0, const float* I1, float* U, float* V, int H, int W, int pitch,
+                                            float alpha, int niter, double* err_out, long long wait_limit,
+                                            int* schedule, void* workspace, size_t workspace_bytes, void* stream) {
   OF_REQUIRE(!bad_plane(I0, H, W, pitch) && I1 && U && V, "of_hs_solve_persistent: bad plane");
   OF_REQUIRE(niter >= 0, "of_hs_solve_persistent: niter < 0");
   if (!workspace || workspace_bytes < of_hs_workspace_size(H, W, pitch))
     return set_error(OF_ERR_WORKSPACE, "of_hs_solve_persistent: workspace too small (%zu < %zu)", workspace_bytes,
                      of_hs_workspace_size(H, W, pitch));
-  const size_t hbs = hs_halo_bytes(H, W);
-  // Images with more tiles than SMs: a launch per pass, whose tiles all SMs share, beats the
-  // persistent queue (600 sweeps of 512 x 512: 1.23 ms against 2.98).
-  if (!hbs && H >= 16 && W >= 16)
-    return of_hs_solve(I0, I1, U, V, H, W, pitch, alpha, niter, err_out, workspace, workspace_bytes, stream);
+  OF_REQUIRE(wait_limit > 0, "of_hs_solve_persistent: wait_limit must be positive");
   cudaStream_t st = as_stream(stream);
+  cudaError_t e = schedule ? cudaMemsetAsync(schedule, 0, sizeof(int), st) : cudaSuccess;
+  if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_hs_solve_persistent: %s", cudaGetErrorString(e));
+  if (!hs_one_launch(H, W))
+    return of_hs_solve(I0, I1, U, V, H, W, pitch, alpha, niter, err_out, workspace, workspace_bytes, stream);
+  const size_t hbs = hs_halo_bytes(H, W);
   const size_t N = (size_t)H * pitch;
   Carver c(workspace, workspace_bytes);
   float* U0 = c.take<float>(2 * N);
@@ -459,12 +472,16 @@ extern "C" int of_hs_solve_persistent(const float* I0, const float* I1, float* U
     copy2_kernel<<<dim3((W + 255) / 256, H), 256, 0, st>>>(U, V, U0, V0, W, pitch);
     n++;
   }
-  cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), st);
+  e = cudaMemsetAsync(status, 0, sizeof(int), st);
   if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_hs_solve_persistent: %s", cudaGetErrorString(e));
   OfHsBatchPair q = {I0, I1, U, V, H, W, pitch, alpha, niter};
   OfTuning tun = {kHsSolveShape, 0, OF_HS_EXACT, OF_HS_SCHED_AUTO};
-  const int rc = hs_batch(&q, 1, &tun, status, 1ll << 20, bw, bws, halo, stream);
+  const int rc = hs_batch(&q, 1, &tun, status, wait_limit, bw, bws, halo, stream);
   if (rc != OF_OK) return rc;
+  if (schedule) {
+    e = cudaMemcpyAsync(schedule, hs_batch_mode(&q, 1, bw, bws), sizeof(int), cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return set_error(OF_ERR_CUDA, "of_hs_solve_persistent: %s", cudaGetErrorString(e));
+  }
   if (err_out) {
     cudaMemsetAsync(acc, 0, 2 * sizeof(double), st);
     dim3 g2((W + 255) / 256 < 4 ? (W + 255) / 256 : 4, H < 256 ? H : 256);

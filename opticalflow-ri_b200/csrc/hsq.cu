@@ -1127,6 +1127,11 @@ static HsqControl hsq_carve_control(Carver& c, const OfHsBatchPair* pairs, int n
   return k;
 }
 
+const int* ofb::hs_batch_mode(const OfHsBatchPair* pairs, int n, void* workspace, size_t workspace_bytes) {
+  Carver c(workspace, workspace_bytes);
+  return hsq_carve_control(c, pairs, n).mode;
+}
+
 extern "C" int of_hs_batch_schedule(const OfHsBatchPair* pairs, int n, const void* workspace, size_t workspace_bytes,
                                     int* schedule, void* stream) {
   OF_REQUIRE(pairs && n > 0 && n <= (1 << 20) && schedule, "of_hs_batch_schedule: bad arguments");

@@ -16,6 +16,8 @@ constexpr int HQ_THREADS = 256;  // threads per CTA of the region sweeps
 int hs_batch(const OfHsBatchPair* pairs, int n, const OfTuning* tuning, int* status, long long wait_limit,
              void* workspace, size_t workspace_bytes, void* halo, void* stream);
 size_t hs_halo_bytes(int H, int W);
+// The device word in the workspace that says which schedule the last such launch ran.
+const int* hs_batch_mode(const OfHsBatchPair* pairs, int n, void* workspace, size_t workspace_bytes);
 
 // (u, v) as held in shared memory: float64 copies of the float32 values for the bit-exact
 // arithmetic (the reference's float64 stencil sums then need no conversion per

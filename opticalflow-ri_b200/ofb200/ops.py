@@ -268,9 +268,9 @@ def in_concurrent_streams() -> bool:
 
 def hs_solve(I0, I1, U, V, alpha: float, niter: int, err: torch.Tensor | None = None, persistent=None):
     """Horn-Schunck in place on U, V.  Returns (U, V, err) with err a device float64 scalar.
-    persistent: all sweeps in one launch (of_hs_solve_persistent) or one launch per pass of
-    4 sweeps (of_hs_solve); None picks the persistent form except inside
-    concurrent_streams().  Both give the same results bit for bit."""
+    persistent: all sweeps in one launch where every tile gets an SM (of_hs_solve_persistent)
+    or one launch per pass of 4 sweeps (of_hs_solve); None picks the persistent form except
+    inside concurrent_streams().  Both give the same results bit for bit."""
     p = _same_pitch(I0, I1, U, V)
     H, W = I0.shape
     if persistent is None:
