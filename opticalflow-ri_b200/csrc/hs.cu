@@ -349,6 +349,7 @@ extern "C" size_t of_hs_workspace_size(int H, int W, int pitch) {
   Sizer s;  // of_hs_solve
   for (int i = 0; i < 7; i++) s.take<float>(N);
   s.take<double>(2);
+  if (!hs_one_launch(H, W)) return s.off;
   Sizer q;  // of_hs_solve_persistent: initial flow (for the error), sums, status, batch workspace
   q.take<float>(2 * N);
   q.take<double>(2);

@@ -1,5 +1,5 @@
 """The one-launch Horn-Schunck solve: its waits that run out, its work queue when not all of its CTAs
-start at once, and the sizes it hands over."""
+start at once, and the scratch of the sizes it hands over."""
 import ctypes
 
 import numpy as np
@@ -68,3 +68,10 @@ def test_beyond_one_launch_against_oracle(cuda_ok, h, w):
     U, V, _, sched = solve(x, 9)
     Uo, Vo, _ = O.hs_solve(*x, 21.0, 9)
     assert int(sched) == 0 and same(U.cpu().numpy(), Uo) and same(V.cpu().numpy(), Vo)
+
+
+def test_scratch_beyond_one_launch_is_the_pass_form_s():
+    """Seven planes (derivatives, the two ping-pong fields, the initial one) and two sums."""
+    from ofb200._lib import lib
+    for h, w in ((2048, 2048), (1185, 192), (512, 512)):
+        assert lib().of_hs_workspace_size(h, w, w) <= 7 * 4 * h * w + 4096
