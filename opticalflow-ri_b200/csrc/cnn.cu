@@ -83,8 +83,7 @@ __device__ bool cv_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort
 // the compiler, and moving them to uniform registers costs more than a small MMA takes
 // (128 x 16 x 16 from shared memory: 171 cycles with index divisions, 53 unrolled, 39 converged).
 // In a training step of 16 crops of 128 x 128: the convolutions 564 -> 505 us, the weight
-// gradients 407 -> 355 us with one wave of splits (of_cnn_conv3x3_wgrad_tc takes whole waves); both
-// are now bound by the boxes they load, nine per pixel.
+// gradients 407 -> 383 us; both are now bound by the boxes they load, nine per pixel.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t e;
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
@@ -319,7 +318,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
 // CTAs split the pixel range; each adds its sums into dW with atomics, four input channels at
 // a time where the lanes run over output channels (scalar ones touch a sector each there).
 // The 12 layers of a training step of 16 crops of 128 x 128: 634 us with one tap per CTA and
-// scalar atomics, about 370 us here.
+// scalar atomics, 383 us here.
 constexpr int WT_KP = 64;  // pixels per K chunk
 constexpr int WT_STAGES = 4;
 
@@ -476,8 +475,9 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
 #pragma unroll
               for (int j = 0; j < 16; j++) {
                 const int bn = n0 + c + j;
+                if (bn >= p.b_ch) break;
                 const int co = p.a_is_dy ? am : bn, ci = p.a_is_dy ? bn : am;
-                if (bn < p.b_ch) atomicAdd(&dw[(size_t)co * p.cin + ci], __uint_as_float(r[j]));
+                atomicAdd(&dw[(size_t)co * p.cin + ci], __uint_as_float(r[j]));
               }
             }
           }
@@ -911,8 +911,7 @@ __global__ void relu_bwd_kernel(bf16* __restrict__ g, int gct, int gco, const bf
   if (!(__bfloat162float(y[p * yct + yco + c]) > 0.f)) g[p * gct + gco + c] = __float2bfloat16_rn(0.f);
 }
 
-// mean squared flow error: loss += sum (pred - label)^2 / (2 P);  dpred = (pred - label) / P
-// (bf16, padded to gct channels, the padding zeroed)
+// The same, 8 channels per thread.
 __global__ void relu_bwd_v8_kernel(bf16* __restrict__ g, int gct, int gco, const bf16* __restrict__ y, int yct, int yco,
                                    long long P, int C) {
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -924,10 +923,13 @@ __global__ void relu_bwd_v8_kernel(bf16* __restrict__ g, int gct, int gco, const
   *o = relu_mask8(*o, *reinterpret_cast<const uint4*>(y + p * yct + yco + c));
 }
 
-// One pixel per thread; the CTA adds its warps' sums in double and issues one atomic (one per
-// warp serialised on the loss's address: 16 x 128 x 128 pixels 25.4 us, 4.8 us here).
-__global__ void __launch_bounds__(256) flow_mse_kernel(const float* __restrict__ pred, const float* __restrict__ label, long long P,
-                                bf16* __restrict__ dpred, int gct, double* __restrict__ loss) {
+// mean squared flow error: loss += sum (pred - label)^2 / (2 P);  dpred = (pred - label) / P
+// (bf16, padded to gct channels, the padding zeroed).  One pixel per thread; the CTA adds its warps'
+// sums in double and issues one atomic (one per warp serialised on the loss's address: 16 x 128 x 128
+// pixels 25.4 us, 4.8 us here).
+__global__ void __launch_bounds__(256) flow_mse_kernel(const float* __restrict__ pred, const float* __restrict__ label,
+                                                       long long P, bf16* __restrict__ dpred, int gct,
+                                                       double* __restrict__ loss) {
   long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   float l = 0.f;
   if (p < P) {
