@@ -191,8 +191,8 @@ __device__ __forceinline__ void hq_sweep2(const float* __restrict__ sfx, const f
 // ---- Register-blocked sweep (bit-exact arithmetic) ---------------------------------------
 // A thread owns a BX x BY block of region cells and keeps their (u, v), as float64 copies of
 // the float32 values, and their derivatives in registers through all sweeps of a pass; a sweep
-// exchanges only the blocks' boundary cells through shared memory.  A cell update then costs
-// 20 bytes of reads and 12 of writes at 4 x 4 where a column walk reads 72 and writes 16.
+// exchanges the cells through shared memory (all of them: one side of a block is 2).  A cell update
+// then writes 16 bytes and reads 48 at 2 x 2, 32 at 2 x 4, where a column walk writes 16 and reads 72.
 // The exchange buffer holds region cell (r, c) as a double2 (u, v) at [r][c % BX][c / BX], so
 // that the threads of a row, BX cells apart, access consecutive 16-byte words.
 template <int RW, int RH, int BX, int BY>

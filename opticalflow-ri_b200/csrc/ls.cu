@@ -132,9 +132,8 @@ __device__ __forceinline__ LsDiv ls_divisor(float den) {
 
 // num / D.d, correctly rounded: two residual corrections of num * y (P. Markstein, "Computation
 // of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Develop. 34(1),
-// 1990), whose residuals are exact for |num| in [2^-60, 2^60]; a zero takes num * y.  The compiler's
-// divide calls a subroutine for a zero numerator, and black pixels are what particle images
-// mostly consist of.
+// 1990), whose residuals are exact for |num| in [2^-60, 2^60]; a zero takes num * y.  The
+// set-up of a 2048 x 2048 particle image, a third of it black: 45.5 us, 51.9 with __fdiv_rn for all.
 __device__ __forceinline__ float ls_div(float num, const LsDiv& D) {
   const float q0 = __fmul_rn(num, D.y), a = fabsf(num);
   float q = __fmaf_rn(__fmaf_rn(-q0, D.d, num), D.y, q0);
@@ -734,9 +733,7 @@ __device__ __forceinline__ void lf_fill(LfBlock& K, const float* st, const LfGeo
 
 // What a pass needs of the solve (both arithmetics).
 struct LsPassArgs {
-  const float* coef;   // 8 planes
   float *ub0, *vb0, *ub1, *vb1;
-  size_t plane;
   int H, W, pitch;
   float h;
   LsCtrl* ctrl;
@@ -1197,7 +1194,7 @@ extern "C" int of_ls_solve_mode(const float* I0, const float* I1, float* U, floa
   cudaLaunchAttribute pdl[1];
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl[0].val.programmaticStreamSerializationAllowed = 1;
-  const LsPassArgs A{coef, ub[0], vb[0], ub[1], vb[1], N, H, W, P, h, ctrl, ss, run, done, redo, inv_n, tol};
+  const LsPassArgs A{ub[0], vb[0], ub[1], vb[1], H, W, P, h, ctrl, ss, run, done, redo, inv_n, tol};
   auto launch_pass = [&](LbPass PP, bool dependent) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = fast ? dim3(tiles < 2 * kNumSMs ? tiles : 2 * kNumSMs) : pgrd;
