@@ -77,8 +77,8 @@ __global__ void hs_sweep_kernel(const float* __restrict__ fx, const float* __res
 //
 // What bounds it: the issue slots (65 instructions per cell update, 16 of them float64
 // multiply-adds) at 50 % busy, and the latency of the pass's loads and barriers behind two
-// CTAs per SM (128 registers a thread).  600 sweeps, one pair alone: 256 x 256 2.75 -> 1.21 ms,
-// 512 x 512 3.1 -> 1.27 ms; 100 sweeps of 2048 x 2048 3.96 -> 2.26 ms (106 -> 186 G cell updates
+// CTAs per SM (128 registers a thread).  600 sweeps, one pair alone: 256 x 256 2.75 -> 1.14 ms,
+// 512 x 512 3.1 -> 1.22 ms; 100 sweeps of 2048 x 2048 3.96 -> 2.20 ms (106 -> 191 G cell updates
 // per second) against the column walk with one cell per thread and row it replaces.  4 x 4
 // blocks spill at 12 warps per SM (113 G/s), a 64 x 64 region in one CTA of 512 threads does
 // less halo work but leaves its loads exposed (164 G/s).
@@ -217,7 +217,7 @@ extern __shared__ __align__(16) double2 hb_sm[];
 // The CTA's pass with the wide quotient, or with the divide where that one's range fails too.  A
 // function of its own that starts from the image: in the kernel its registers cost every pass 1 to
 // 2 % from 1024 x 1024 on.  512 x 512, 600 sweeps, one half the same texture in both frames: 1.93 ms
-// (4.50 where such passes were run again with the divide, 1.27 without tiny numerators).
+// (4.50 where such passes were run again with the divide, 1.22 without tiny numerators).
 __device__ __noinline__ void hb_pass_wide(const HbPass& P) {
   const HbPos p = hb_pos(P);
   const HrWin win = hr_window<HB_RW, HB_RH, HB_BX, HB_BY>(p.r0, p.c0, p.gy0, p.gx0, P.H, P.W);
@@ -256,10 +256,13 @@ __global__ void __launch_bounds__(HbGeom::NT, 2) hs_pass_kernel(const __grid_con
     wide = hb_load_uv(K, P, p.gy0, p.gx0, p.inside) || wide;
     hr_publish<HB_RW, HB_RH, HB_BX, HB_BY>(K, hb_sm, p.r0, p.c0);
   }
+  // formed here, while the loads are on their way: behind the barrier it would stand in front of the
+  // first sweep (600 sweeps of 256 x 256 1.21 -> 1.14 ms)
+  HrWin win = hr_window<HB_RW, HB_RH, HB_BX, HB_BY>(p.r0, p.c0, p.gy0, p.gx0, P.H, P.W);
+  // the region holds blocks that the image ends inside of
+  const bool rag = (P.W % HB_BX && p.x0 + HB_RW > P.W) || (P.H % HB_BY && p.y0 + HB_RH > P.H);
+  asm volatile("" : "+r"(win.cl), "+r"(win.cr), "+r"(win.rt), "+r"(win.rb));
   if (!__syncthreads_or(wide)) {
-    const HrWin win = hr_window<HB_RW, HB_RH, HB_BX, HB_BY>(p.r0, p.c0, p.gy0, p.gx0, P.H, P.W);
-    // the region holds blocks that the image ends inside of
-    const bool rag = (P.W % HB_BX && p.x0 + HB_RW > P.W) || (P.H % HB_BY && p.y0 + HB_RH > P.H);
     if (rag)
       hb_sweeps<true, HR_REFINED>(K, P, hb_sm, p.in, p.r0, p.c0, win);
     else
@@ -340,7 +343,7 @@ static size_t hs_persistent_ws(int H, int W, int pitch) {
 
 // Whether of_hs_solve_persistent runs a size in one launch.  Images with more tiles than SMs: a
 // launch per pass, whose tiles all SMs share, beats the persistent queue (600 sweeps of 512 x 512:
-// 1.27 ms against 2.98).
+// 1.22 ms against 2.98).
 static bool hs_one_launch(int H, int W) { return hs_halo_bytes(H, W) != 0 || H < 16 || W < 16; }
 
 // Covers both of_hs_solve and of_hs_solve_persistent.

@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2)
 //   64 x 32  to 148 tiles of 48 x 16:  304 1.2 -> 0.66
 //   64 x 48  to 148 tiles of 48 x 32:  384 1.70 -> 0.99, 448 2.30 -> 0.95
 // With one half the same texture in both frames (hr_row's HR_WIDE): 96 0.56, 256 0.60, 448 1.10.
-// Larger images: one launch per pass (hs.cu), 512 2.98 -> 1.23.
+// Larger images: one launch per pass (hs.cu), 512 2.98 -> 1.22.
 template <int RW_, int RH_, int T_, int BX_, int BY_>
 struct HrShape {
   static constexpr int RW = RW_, RH = RH_, T = T_, BX = BX_, BY = BY_, TW = RW - 2 * T, TH = RH - 2 * T;
