@@ -52,7 +52,7 @@ REF_BUDGET_S = 90.0
 # DRAM bytes (read + write) of one 60-sweep Liu-Shen solve at 1024^2, summed over its
 # launches from one ncu capture per arithmetic (profiles/ls_solve_traffic_1024.txt; cold cache
 # per launch)
-NCU_LS_TRAFFIC = {("exact", 1024): 663.48e6, ("fast", 1024): 663.93e6}
+NCU_LS_TRAFFIC = {("exact", 1024): 663.52e6, ("fast", 1024): 663.93e6}
 
 
 def parse():
